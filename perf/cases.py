@@ -261,9 +261,9 @@ def _pass(s):
     if kind == "tables":
         which = int(np.argmax(s.table_sizes))
         d = tables.run(s.g, s.table_sizes, s.table_seed, s.case["batched"], dump_table=which)
-        keys, vals = d["dump"]
-        order = np.argsort(keys)
-        return {"keys": keys[order].view(np.int64), "values": vals[order].view(np.int64),
+        keys, vals = (torch.from_numpy(x.view(np.int64)).cuda() for x in d["dump"])
+        keys, order = keys.sort()  # the largest table's pairs, in whatever order its chains held them
+        return {"keys": keys, "values": vals[order],
                 "inserted": int(d["inserted"]), "deleted": int(d["deleted"]), "violations": int(d["violations"]),
                 "nodes_left": int(d["nodes_allocated"] - d["nodes_freed"] - d["spare_nodes_freed"])}
     d = s.server.run(s.jobs, realtime=False)
