@@ -60,7 +60,7 @@ __global__ void k_init_words(gal::state st, uint64_t nblocks) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t b = i; b < nblocks; b += stride) *gal::mword_ptr(&st, (uint32_t)b) = 4097ull;
-  for (uint64_t g = i; g < st.num_segments; g += stride) st.act[g] = gal::act_word(0, -1);
+  for (uint64_t g = i; g < st.num_segments; g += stride) st.act[g] = gal::act_word(0, gal::ACT_FREE, -1);
   for (uint32_t l = 0; l < sh.layers; l++) {
     uint64_t items = sh.items[l];
     for (uint64_t w = i; w < sh.nwords[l]; w += stride) {
@@ -699,8 +699,9 @@ int gal_import_state(gal_handle *h, const gal_state_view *v) {
   CUDA_TRY(cudaMemcpy(st.sub_trees, v->sub_tree_words, T * W * 8, H2D));
   CUDA_TRY(cudaMemcpy(st.tree_ids, v->tree_ids, S * 2, H2D));
   {
-    std::vector<unsigned long long> act(S);  // generation 0, the view's counts
-    for (uint64_t i = 0; i < S; i++) act[i] = gal::act_word(0, v->active_counts[i]);
+    std::vector<unsigned long long> act(S);  // generation 0, the view's classes and counts
+    for (uint64_t i = 0; i < S; i++)
+      act[i] = gal::act_word(0, v->tree_ids[i] < T ? v->tree_ids[i] : gal::ACT_FREE, v->active_counts[i]);
     CUDA_TRY(cudaMemcpy(st.act, act.data(), S * 8, H2D));
   }
   CUDA_TRY(cudaMemcpy(st.qc, v->queue_counters, S * 4, H2D));

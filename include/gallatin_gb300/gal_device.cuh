@@ -18,9 +18,9 @@
 //     sector per block, gal_config.block_layout), so the pinned blocks that
 //     different SMs claim from never share a sector; the dense layout (all
 //     malloc words, then all free counters) remains selectable;
-//   * each segment's count of blocks left carries a set-up generation, so a
-//     reservation checks the segment's class before it subtracts and never
-//     has to give back into a later owner's count;
+//   * each segment's count of blocks left carries the segment's class and a
+//     set-up generation, so one word tells a reservation whose segment it is
+//     and it never has to give back into a later owner's count;
 //   * every class lock sits in a 32-byte sector of its own;
 //   * every spin-wait is bounded by state::spin_limit and reports through the
 //     error word instead of trapping (the reference traps, gallatin.cuh:87);
@@ -96,7 +96,7 @@ struct state {
   uint32_t *qc;                  // [S] hand-out position
   uint32_t *qfc;                 // [S] return position
   uint32_t *fqfc;                // [S] finalised return position
-  unsigned long long *act;       // [S] (generation << 32) | (blocks left - 1 + ACT_BIAS)
+  unsigned long long *act;       // [S] generation, class and blocks left (see act_word)
   unsigned long long *mwords;    // per block (tree << 32) | count, every mstride-th word
   uint32_t *fctr;                // per block frees counted, every fstride-th word
   uint32_t mstride;              // 4 with fstride 8: one 32-byte record per block
@@ -118,16 +118,20 @@ GAL_DEVICE_INLINE __host__ unsigned long long *mword_ptr(const state *s, uint32_
 GAL_DEVICE_INLINE __host__ uint32_t *fctr_ptr(const state *s, uint32_t blk) {
   return s->fctr + (uint64_t)blk * s->fstride;
 }
-// A segment's count word: generation in the high half, the reference's
-// active count (blocks left to hand out minus one; -1 when none is left or the
-// segment is free) plus ACT_BIAS in the low half, so adding or subtracting one
-// never carries into the generation.
+// A segment's count word: in the low half the reference's active count (blocks
+// left to hand out minus one; -1 when none is left or the segment is free) plus
+// ACT_BIAS, so adding or subtracting one never carries into the high half,
+// which holds the class that owns the segment (ACT_FREE: none) in its low byte
+// and the set-up generation in the rest.  The atomic that reserves a block
+// thus also says whose segment it was taken from, with no second word to read.
 static constexpr uint32_t ACT_BIAS = 0x80000000u;
+static constexpr uint32_t ACT_FREE = 0xFFu;
 GAL_DEVICE_INLINE __host__ int32_t act_unbias(uint32_t low) { return (int32_t)(low - ACT_BIAS); }
 GAL_DEVICE_INLINE __host__ int32_t act_count(unsigned long long w) { return act_unbias((uint32_t)w); }
-GAL_DEVICE_INLINE __host__ uint32_t act_gen(unsigned long long w) { return (uint32_t)(w >> 32); }
-GAL_DEVICE_INLINE __host__ unsigned long long act_word(uint32_t gen, int32_t count) {
-  return ((unsigned long long)gen << 32) | (uint32_t)((uint32_t)count + ACT_BIAS);
+GAL_DEVICE_INLINE __host__ uint32_t act_class(unsigned long long w) { return (uint32_t)(w >> 32) & 0xFFu; }
+GAL_DEVICE_INLINE __host__ uint32_t act_gen(unsigned long long w) { return (uint32_t)(w >> 40); }
+GAL_DEVICE_INLINE __host__ unsigned long long act_word(uint32_t gen, uint32_t cls, int32_t count) {
+  return ((unsigned long long)((gen << 8) | cls) << 32) | (uint32_t)((uint32_t)count + ACT_BIAS);
 }
 
 // ------------------------------------------------------------------ helpers
@@ -191,6 +195,18 @@ GAL_DEVICE_INLINE uint64_t amo_or(uint64_t *p, uint64_t v) {
 }
 GAL_DEVICE_INLINE uint64_t amo_and(uint64_t *p, uint64_t v) {
   return atomicAnd((unsigned long long *)p, (unsigned long long)v);
+}
+// atomicAdd whose later accesses by this thread stay after it
+GAL_DEVICE_INLINE unsigned long long add_acquire(unsigned long long *p, unsigned long long v) {
+  unsigned long long r;
+  asm volatile("atom.acquire.gpu.global.add.u64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(v) : "memory");
+  return r;
+}
+GAL_DEVICE_INLINE void st_rlx(unsigned long long *p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+GAL_DEVICE_INLINE void st_rlx(uint32_t *p, uint32_t v) {
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 GAL_DEVICE_INLINE uint16_t cas16(uint16_t *p, uint16_t cmp, uint16_t val) {
   return (uint16_t)atomicCAS((unsigned short *)p, (unsigned short)cmp, (unsigned short)val);
@@ -279,11 +295,13 @@ GAL_DEVICE_INLINE bool veb_query(const veb_ref &v, uint64_t x) {
 // the refilled word.  Without them a clear could land after the insert's set
 // while the re-read still saw the empty word, leaving a non-empty word behind
 // a clear summary bit, where top-down searches never find its items.
-GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x) {
+// `left` receives the other items the bottom word held.
+GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x, uint64_t &left) {
   int layer = (int)v.sh->layers - 1;
   uint64_t high = x >> 6;
   int low = (int)(x & 63);
   uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
+  left = old & ~(1ULL << low);
   if (!(old & (1ULL << low))) return false;
   while (__popcll(old) == 1 && layer > 0) {
     uint64_t *child = v.word(layer, high);
@@ -299,6 +317,11 @@ GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x) {
     }
   }
   return true;
+}
+
+GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x) {
+  uint64_t left;
+  return veb_remove(v, x, left);
 }
 
 // veb_tree::insert_force_update (veb.cuh:775-798); the fence orders each
@@ -357,40 +380,113 @@ GAL_DEVICE_INLINE uint64_t veb_lock_offset(const veb_ref &v, uint64_t start) {
   }
 }
 
-// veb_tree::malloc_first (veb.cuh:979-991)
+// Trees of up to 64 bottom words (4,096 segments) are searched top-down from
+// the one summary word above them, held in a register: `top` has the bottom
+// words that are not empty (a one-layer tree is its only bottom word).  Each
+// search below
+// then costs two or three dependent loads, where climbing from a start word
+// and coming down again for every start tried cost eight to ten (a block
+// request spent 6 of its 13 us there).
+GAL_DEVICE_INLINE bool veb_shallow(const veb_ref &v) { return v.sh->nwords[v.sh->layers - 1] <= 64; }
+GAL_DEVICE_INLINE uint64_t veb_top(const veb_ref &v) {
+  return v.sh->layers > 1 ? ld_rlx(v.w + v.sh->off[v.sh->layers - 2]) : 1ull;
+}
+GAL_DEVICE_INLINE uint64_t *veb_bottom(const veb_ref &v) { return v.w + v.sh->off[v.sh->layers - 1]; }
+
+// veb_tree::malloc_first (veb.cuh:979-991): takes the smallest item.  Threads
+// that lose it to one another would all go for the next smallest together, one
+// winner per round trip; each loser goes on from the word as its own attempt
+// left it, at a place of its own, so k contenders are served in a few round
+// trips.  One thread alone never loses and always gets the smallest.
 GAL_DEVICE_COLD uint64_t veb_malloc_first(const veb_ref &v) {
+  if (!veb_shallow(v)) {
+    for (int a = 0; a < VEB_ATTEMPTS; a++) {
+      uint64_t o = veb_lock_offset(v, 0);
+      if (o != FAIL) return o;
+    }
+    return FAIL;
+  }
+  uint64_t *bottom = veb_bottom(v);
+  const uint32_t spread = (uint32_t)(thread_linear_id() * 0x9E3779B1u) >> 26;
   for (int a = 0; a < VEB_ATTEMPTS; a++) {
-    uint64_t o = veb_lock_offset(v, 0);
-    if (o != FAIL) return o;
+    for (uint64_t top = veb_top(v); top; top &= top - 1ull) {
+      const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
+      uint64_t word = ld_rlx(bottom + high);
+      for (uint32_t turn = 0; word; turn = spread) {
+        const uint64_t turned = (word >> turn) | (turn ? word << (64u - turn) : 0ull);
+        const uint64_t low = ((uint64_t)(__ffsll((long long)turned) - 1) + turn) & 63u;
+        if (veb_remove(v, (high << 6) + low, word)) return (high << 6) + low;
+      }
+    }
   }
   return FAIL;
 }
 
-// veb_tree::find_random_valid_index (veb.cuh:946-977)
-// A search that came back empty from `start` shows that no item lies in
-// [start, U); later attempts starting at or above the lowest such start are
-// answered from that without touching the tree (the result is the one the
-// reference's repeated searches give when nothing is inserted meanwhile, and
-// one of the outcomes its relaxed reads allow when something is).  A sparse
-// tree whose items sit at low ids otherwise costs all 15 attempts.
+// The smallest listed item at or above `start`, which must not exceed an item
+// last seen listed in bottom word `last` (its content then: `last_word`).
+GAL_DEVICE_INLINE uint64_t veb_at_or_above(const uint64_t *bottom, uint64_t top, uint64_t start, uint64_t last,
+                                           uint64_t last_word) {
+  uint64_t high = start >> 6;
+  uint64_t word = (high == last ? last_word : ld_rlx(bottom + high)) & ~bitmask((int)(start & 63u));
+  while (!word) {  // reaches `last` at the latest, whose remembered word holds an item above start
+    const uint64_t above = top & ~bitmask((int)high + 1);
+    high = above ? (uint64_t)(__ffsll((long long)above) - 1) : last;
+    word = high >= last ? last_word : ld_rlx(bottom + high);
+  }
+  return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
+}
+
+// veb_tree::find_random_valid_index (veb.cuh:946-977): of 15 hashed starts the
+// first with a listed item at or above it gives the smallest such item; if none
+// has one, the smallest item above 0.  A start has one exactly when it does not
+// exceed the largest listed item, so that is found first (two loads) and the
+// starts are tried in registers.  A deeper tree is searched from each start;
+// one that found nothing shows that no item lies in [start, U), and later
+// starts at or above the lowest such start are skipped.
 GAL_DEVICE_COLD uint64_t veb_find_random(const veb_ref &v, uint64_t tid) {
   const uint64_t U = v.sh->items[v.sh->layers - 1];
-  uint64_t h1 = murmur64a_u64(tid, v.seed);
-  uint64_t h2 = murmur64a_u64(tid, h1);
-  uint64_t empty_from = U;  // no item in [empty_from, U)
-  for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
-    uint64_t start = (h1 + a * h2) % U;
-    if (start >= empty_from) continue;
-    if (veb_query(v, start)) return start;
-    uint64_t idx = veb_successor(v, start);
-    if (idx != FAIL) return idx;
-    empty_from = start;
+  const uint64_t h1 = murmur64a_u64(tid, v.seed);
+  const uint64_t h2 = murmur64a_u64(tid, h1);
+  if (!veb_shallow(v)) {
+    uint64_t empty_from = U;  // no item in [empty_from, U)
+    for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
+      uint64_t start = (h1 + a * h2) % U;
+      if (start >= empty_from) continue;
+      if (veb_query(v, start)) return start;
+      uint64_t idx = veb_successor(v, start);
+      if (idx != FAIL) return idx;
+      empty_from = start;
+    }
+    return veb_successor(v, 0);
   }
-  return veb_successor(v, 0);
+  const uint64_t *bottom = veb_bottom(v);
+  uint64_t top = veb_top(v), last = 0, last_word = 0;
+  while (top) {
+    last = 63u - (uint64_t)__clzll((long long)top);
+    last_word = ld_rlx(bottom + last);
+    if (last_word) break;
+    top &= ~(1ull << last);  // emptied since its summary was read
+  }
+  if (!last_word) return FAIL;
+  const uint64_t largest = (last << 6) + 63u - (uint64_t)__clzll((long long)last_word);
+  for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
+    const uint64_t start = (U & (U - 1ull)) == 0 ? (h1 + a * h2) & (U - 1ull) : (h1 + a * h2) % U;
+    if (start <= largest) return veb_at_or_above(bottom, top, start, last, last_word);
+  }
+  return largest ? veb_at_or_above(bottom, top, 1, last, last_word) : FAIL;
 }
 
 // veb_tree::find_first_valid_index (veb.cuh:940-944): smallest listed id
 GAL_DEVICE_INLINE uint64_t veb_find_first(const veb_ref &v) {
+  if (veb_shallow(v)) {
+    const uint64_t *bottom = veb_bottom(v);
+    for (uint64_t top = veb_top(v); top; top &= top - 1ull) {
+      const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
+      const uint64_t word = ld_rlx(bottom + high);
+      if (word) return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
+    }
+    return FAIL;
+  }
   if (veb_query(v, 0)) return 0;
   return veb_successor(v, 0);
 }
@@ -535,40 +631,51 @@ GAL_DEVICE_INLINE bool try_lock(const state *s, uint32_t bit) {
   return atomicExch(s->locks + bit * LOCK_STRIDE, 1u) == 0u;
 }
 GAL_DEVICE_INLINE void unlock(const state *s, uint32_t bit) {
-  __threadfence();
-  atomicExch(s->locks + bit * LOCK_STRIDE, 0u);
+  fence_acq_rel();
+  st_rlx(s->locks + bit * LOCK_STRIDE, 0u);
 }
 
 // ------------------------------------------------------------------ table
-// alloc_table::setup_segment (memory_table.cuh:746-818)
-GAL_DEVICE_COLD bool setup_segment(const state *s, uint64_t seg, uint32_t tree) {
+// alloc_table::setup_segment (memory_table.cuh:746-818).  `taken` blocks (0 or
+// 1) are handed out with the set-up itself.
+GAL_DEVICE_COLD bool setup_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t taken) {
+  // the high half of a free segment's count word changes only here
+  const uint32_t high = (uint32_t)(ld_rlx(&s->act[seg]) >> 32);
   if (cas16(&s->tree_ids[seg], FREE_TREE, (uint16_t)tree) != FREE_TREE) return false;
-  uint32_t nb = blocks_in_segment(s, tree);
+  const uint32_t nb = blocks_in_segment(s, tree);
   uint32_t *q = s->queues + (seg << s->bps_shift);
-  for (uint32_t i = 0; i < nb; i++) q[i] = NOBLK;
-  __threadfence();
-  atomicExch(&s->qc[seg], 0u);
-  atomicExch(&s->qfc[seg], 0u);
-  atomicExch(&s->fqfc[seg], 0u);
-  __threadfence();
-  // count -1 -> nb - 1 and a new generation, by addition: a reservation
-  // attempt still in flight from before the segment's release gives its one
-  // back into this count, as it took it from the count it found
-  atomicAdd(&s->act[seg], (1ull << 32) + nb);
+  if (nb >= 4) {
+    for (uint32_t i = 0; i < nb; i += 4) *(uint4 *)(q + i) = make_uint4(NOBLK, NOBLK, NOBLK, NOBLK);
+  } else {
+    for (uint32_t i = 0; i < nb; i++) q[i] = NOBLK;
+  }
+  st_rlx(&s->qc[seg], taken);
+  st_rlx(&s->qfc[seg], 0u);
+  st_rlx(&s->fqfc[seg], 0u);
+  fence_acq_rel();
+  // count -1 -> nb - 1 - taken, the class and a new generation, by addition: a
+  // reservation attempt still in flight from before the segment's release gives
+  // its one back into this count, as it took it from the count it found
+  const uint32_t next = (((high >> 8) + 1u) << 8) | tree;
+  atomicAdd(&s->act[seg], ((unsigned long long)(next - high) << 32) + nb - taken);
   return true;
 }
 
-// Gallatin::gather_new_segment (gallatin.cuh:1465-1510)
-GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree) {
+// Gallatin::gather_new_segment (gallatin.cuh:1465-1510).  With `take` the
+// segment's first block (pos 0) is the caller's: it is counted out before the
+// segment is listed, and a segment of one block is not listed at all, as it
+// would be taken off again by the same thread.
+GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool take) {
   uint64_t seg = veb_malloc_first(seg_tree(s));
   if (seg == FAIL) return -1;
-  if (!setup_segment(s, seg, tree)) {
+  if (!setup_segment(s, seg, tree, take ? 1u : 0u)) {
     set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
     return -1;
   }
-  __threadfence();
-  veb_insert(sub_tree(s, tree), seg);
-  __threadfence();
+  if (!take || blocks_in_segment(s, tree) > 1) {
+    fence_acq_rel();
+    veb_insert(sub_tree(s, tree), seg);
+  }
   return (int64_t)seg;
 }
 
@@ -578,13 +685,13 @@ GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree) {
 // Gallatin::return_block, gallatin.cuh:1663-1722, finish_freeing_block,
 // memory_table.cuh:1226-1241).
 GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
-  const unsigned long long home = act_word(gen, (int32_t)nb - 1);
-  if (atomicCAS(&s->act[seg], home, act_word(gen, -1)) != home) return;
-  __threadfence();
+  const unsigned long long home = act_word(gen, tree, (int32_t)nb - 1);
+  if (atomicCAS(&s->act[seg], home, act_word(gen, ACT_FREE, -1)) != home) return;
+  fence_acq_rel();
   veb_remove(sub_tree(s, tree), seg);
-  __threadfence();
+  fence_acq_rel();
   if (cas16(&s->tree_ids[seg], (uint16_t)tree, FREE_TREE) != (uint16_t)tree) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
-  __threadfence();
+  fence_acq_rel();
   veb_insert(seg_tree(s), seg);
 }
 
@@ -596,9 +703,8 @@ GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree
 // hand-out yet the segment is a fresh one whose gatherer takes its first
 // block next, so it stays.
 GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
-  const unsigned long long old = atomicAdd(&s->act[seg], 1ull);
-  __threadfence();
-  const uint16_t tree = ld_rlx(&s->tree_ids[seg]);
+  const unsigned long long old = add_acquire(&s->act[seg], 1ull);
+  const uint32_t tree = act_class(old);
   if (tree >= s->num_trees) return;
   const uint32_t nb = blocks_in_segment(s, tree);
   if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&s->qc[seg]) != 0)
@@ -611,29 +717,20 @@ GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
 // (memory_table.cuh:923-929, get_slot_in_segment / return_slot_to_segment).
 // An add-back that lands after the segment was released and set up again
 // raises the new owner's count above its blocks, and one that lands after the
-// segment's last return leaves it unreleased.  Here the class is checked
-// against the count's generation before the subtraction, a count already
-// negative is not touched, and the subtraction carries into a new set-up (see
-// setup_segment), so the only give-backs left are the rare ones of a race
-// between the check and the subtraction, which give_back_reservation
-// settles.
+// segment's last return leaves it unreleased.  Here the count word carries the
+// class: a word of another class or a count already negative is not touched,
+// and the subtraction carries into a new set-up (see setup_segment), so the
+// only give-backs left are the rare ones of a race between the load and the
+// subtraction, which give_back_reservation settles.  The new block's malloc
+// word is stored, not yet published: whoever installs the block fences first.
 GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, bool &last) {
   last = false;
   const unsigned long long seen = ld_rlx(&s->act[seg]);
-  if (act_count(seen) < 0) return NOBLK;  // nothing left (or a free segment)
-  __threadfence();
-  if (ld_rlx(&s->tree_ids[seg]) != (uint16_t)tree) return NOBLK;  // another class's segment
-  const unsigned long long old = atomicAdd(&s->act[seg], ~0ull);  // minus one
-  const int32_t ac = act_count(old);
-  if (ac < 0) {  // the last block went to another thread meanwhile
-    give_back_reservation(s, seg);
-    return NOBLK;
-  }
-  __threadfence();
-  if (act_gen(old) != act_gen(seen) && ld_rlx(&s->tree_ids[seg]) != (uint16_t)tree) {
-    // released and set up for another class between the check and the
-    // subtraction; the class read now is the generation's own, as the
-    // reservation keeps it from being released
+  if (act_class(seen) != tree || act_count(seen) < 0) return NOBLK;  // another class's, or nothing left
+  const unsigned long long old = add_acquire(&s->act[seg], ~0ull);  // minus one
+  if (act_count(old) < 0 || act_class(old) != tree) {
+    // the last block went to another thread meanwhile, or the segment was
+    // released and set up for another class
     give_back_reservation(s, seg);
     return NOBLK;
   }
@@ -643,7 +740,7 @@ GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, 
   if (pos < nb) {
     blk = (uint32_t)(seg << s->bps_shift) + pos;
   } else {
-    uint32_t *e = s->queues + (seg << s->bps_shift) + (pos % nb);
+    uint32_t *e = s->queues + (seg << s->bps_shift) + (pos & (nb - 1u));
     blk = atomicExch(e, NOBLK);
     for (uint32_t i = 0; blk == NOBLK && i < s->spin_limit; i++) {  // a return still in flight
       backoff(i);
@@ -654,24 +751,68 @@ GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, 
       return NOBLK;
     }
   }
-  atomicExch(mword_ptr(s, blk), (unsigned long long)tree << 32);  // Block::init_malloc
-  if (ac == 0) last = true;
+  st_rlx(mword_ptr(s, blk), (unsigned long long)tree << 32);  // Block::init_malloc
+  last = act_count(old) == 0;
   return blk;
 }
 
-// Gallatin::request_new_block_from_tree (gallatin.cuh:1525-1631)
-GAL_DEVICE_COLD uint32_t request_block(const state *s, uint32_t tree, uint64_t tid) {
+// Waits between attempts at a segment another thread is working on: a gather
+// takes a few microseconds, so the first waits are short; a wait that lasts
+// grows to backoff's.
+GAL_DEVICE_INLINE void backoff_gather(uint32_t i) { __nanosleep(i < 24 ? 100u : 4096u); }
+
+// The rest of a block request that took the last block of a segment
+// (gallatin.cuh:1598-1612): the segment leaves its class's tree and, with
+// gather_ahead, the class's next segment is gathered.  Split from
+// request_block so that a claim's block can be installed first: the teams
+// waiting for it do not wait for the gather, and one thread alone leaves the
+// same state either way.  Blocks may have come home between the hand-out and
+// the removal here, so the segment is listed again if it has one to give; the
+// release of a segment closes its count word before it unlists it, so a
+// listing made here and still valid when the word is read again is either
+// right or taken off by the release.
+// Only one thread of a class gathers ahead at a time, whatever its lock policy
+// (alone, a thread always finds the lock free): each would add a segment to a
+// class that needs one, and threads that take a class's last blocks together
+// would leave it holding hundreds.
+static constexpr uint32_t NOSEG = 0xFFFFFFFFu;
+GAL_DEVICE_COLD void finish_last_block(const state *s, uint32_t tree, uint32_t seg, bool listed) {
+  if (listed) {
+    veb_remove(sub_tree(s, tree), seg);
+    for (;;) {
+      fence_acq_rel();
+      unsigned long long w = ld_rlx(&s->act[seg]);
+      if (act_class(w) != tree || act_count(w) < 0) break;
+      veb_insert(sub_tree(s, tree), seg);
+      fence_acq_rel();
+      w = ld_rlx(&s->act[seg]);
+      if (act_class(w) == tree && act_count(w) >= 0) break;
+      veb_remove(sub_tree(s, tree), seg);
+    }
+  }
+  if (s->gather_ahead && try_lock(s, tree)) {
+    gather_new_segment(s, tree, false);
+    unlock(s, tree);
+  }
+}
+
+// Gallatin::request_new_block_from_tree (gallatin.cuh:1525-1631).  `emptied`
+// receives the segment whose last block this was (bit 31: it was never
+// listed), for request_done, else NOSEG.
+static constexpr uint32_t SEG_UNLISTED = 0x80000000u;
+GAL_DEVICE_COLD uint32_t request_block_begin(const state *s, uint32_t tree, uint64_t tid, uint32_t &emptied) {
   uint32_t spins = 0;
   int gather_fails = 0;
+  emptied = NOSEG;
   for (;;) {
     veb_ref sub = sub_tree(s, tree);
     uint64_t seg = s->policy == GAL_POLICY_LOWEST ? veb_find_first(sub) : veb_find_random(sub, tid);
     // classes with few blocks per segment need a segment per few requests:
     // the class lock only serialises them (serially the lock is always free)
-    const bool unlocked = blocks_in_segment(s, tree) < s->gather_unlocked_below;
     if (seg == FAIL) {
+      const bool unlocked = blocks_in_segment(s, tree) < s->gather_unlocked_below;
       if (unlocked || try_lock(s, tree)) {
-        int64_t got = gather_new_segment(s, tree);
+        int64_t got = gather_new_segment(s, tree, true);
         if (!unlocked) unlock(s, tree);
         if (got < 0) {
           // segment tree empty: nothing a retry by this thread alone changes
@@ -679,33 +820,41 @@ GAL_DEVICE_COLD uint32_t request_block(const state *s, uint32_t tree, uint64_t t
           backoff(gather_fails);
           continue;
         }
-        seg = (uint64_t)got;
-      } else {
-        if (++spins > s->spin_limit) {
-          set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_REQUEST_LOCK, tree, spins);
-          return NOBLK;
-        }
-        backoff(spins);
-        continue;
+        const uint32_t blk = (uint32_t)((uint64_t)got << s->bps_shift);
+        st_rlx(mword_ptr(s, blk), (unsigned long long)tree << 32);
+        if (blocks_in_segment(s, tree) == 1) emptied = (uint32_t)got | SEG_UNLISTED;
+        return blk;
       }
+      if (++spins > s->spin_limit) {
+        set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_REQUEST_LOCK, tree, spins);
+        return NOBLK;
+      }
+      backoff_gather(spins);
+      continue;
     }
     bool last = false;
     uint32_t blk = get_block(s, seg, tree, last);
-    if (last) {
-      veb_remove(sub, seg);
-      if (s->gather_ahead && (unlocked || try_lock(s, tree))) {
-        gather_new_segment(s, tree);
-        if (!unlocked) unlock(s, tree);
-      }
-      __threadfence();
-    }
+    if (last) emptied = (uint32_t)seg;
     if (blk != NOBLK) return blk;
+    if (last) {  // counted out, but its block never came: the segment is empty all the same
+      finish_last_block(s, tree, (uint32_t)seg, true);
+      emptied = NOSEG;
+    }
     if (++spins > s->spin_limit) {
       set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_REQUEST_RETRY, tree, seg);
       return NOBLK;
     }
-    backoff(spins);
+    backoff_gather(spins);
   }
+}
+GAL_DEVICE_INLINE void request_done(const state *s, uint32_t tree, uint32_t emptied) {
+  if (emptied != NOSEG) finish_last_block(s, tree, emptied & ~SEG_UNLISTED, !(emptied & SEG_UNLISTED));
+}
+GAL_DEVICE_INLINE uint32_t request_block(const state *s, uint32_t tree, uint64_t tid) {
+  uint32_t emptied;
+  const uint32_t blk = request_block_begin(s, tree, tid, emptied);
+  request_done(s, tree, emptied);
+  return blk;
 }
 
 // Gallatin::return_block (gallatin.cuh:1637-1726) with reserve_segment_slot,
@@ -719,9 +868,8 @@ GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
   }
   uint32_t nb = blocks_in_segment(s, tree);
   uint32_t pos = atomicAdd(&s->qfc[seg], 1u);
-  uint32_t live = pos % nb;
-  atomicExch(s->queues + (seg << s->bps_shift) + live, blk);
-  __threadfence();
+  uint32_t live = pos & (nb - 1u);
+  st_rlx(s->queues + (seg << s->bps_shift) + live, blk);
   // The reference finalises returns in position order with a CAS spin
   // (memory_table.cuh:906-910) so a hand-out never meets an empty ring entry;
   // get_block here waits (bounded) for an entry still in flight instead, so a
@@ -730,12 +878,9 @@ GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
   // re-register at the 10% crossing (gallatin.cuh:1646): live/nb >= 0.1 and
   // (live-1)/nb < 0.1 in doubles; for the power-of-two nb used here that is
   // 10*live > nb >= 10*(live-1) with live-1 taken as unsigned (live 0 never).
-  if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) {
-    veb_insert(sub_tree(s, tree), seg);
-    __threadfence();
-  }
-  const unsigned long long old = atomicAdd(&s->act[seg], 1ull);
-  __threadfence();
+  if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) veb_insert(sub_tree(s, tree), seg);
+  fence_acq_rel();  // the ring entry before the count that lets it be handed out
+  const unsigned long long old = add_acquire(&s->act[seg], 1ull);
   if ((uint32_t)(act_count(old) + 2) == nb)  // all_blocks_free: the count was nb - 2
     release_segment(s, seg, tree, act_gen(old), nb);
 }
@@ -749,8 +894,7 @@ GAL_DEVICE_INLINE void credit_frees(const state *s, uint32_t blk, uint32_t n) {
 // the block's free counter was `old` before this thread added n
 GAL_DEVICE_INLINE void credit_done(const state *s, uint32_t blk, uint32_t old, uint32_t n) {
   if (old + n == SLICES_PER_BLOCK) {
-    atomicExch(fctr_ptr(s, blk), 0u);
-    __threadfence();
+    st_rlx(fctr_ptr(s, blk), 0u);  // published by return_block's fence
     return_block(s, blk);
   } else if (old + n > SLICES_PER_BLOCK) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OVERFLOW, blk,
@@ -803,16 +947,19 @@ GAL_DEVICE_COLD bool replace_block(const state *s, uint32_t tree, uint32_t slot,
                                    uint64_t tid) {
   uint32_t *sp = s->slots + s->slot_base[tree] + slot;
   if (atomicCAS(sp, blk, NOBLK) != blk) return true;
-  __threadfence();
-  uint32_t nb = request_block(s, tree, tid);
-  if (nb == NOBLK) return false;
-  __threadfence();
-  if (atomicCAS(sp, NOBLK, nb) != NOBLK) {
-    set_error(s, GAL_DEV_ERR_SLOT_SWAP);
-    retire_block(s, nb);  // hand the block back
-    return false;
+  uint32_t emptied;
+  uint32_t nb = request_block_begin(s, tree, tid, emptied);
+  bool ok = false;
+  if (nb != NOBLK) {
+    fence_acq_rel();
+    ok = atomicCAS(sp, NOBLK, nb) == NOBLK;
+    if (!ok) {
+      set_error(s, GAL_DEV_ERR_SLOT_SWAP);
+      retire_block(s, nb);  // hand the block back
+    }
   }
-  return true;
+  request_done(s, tree, emptied);  // after the waiting teams have their block
+  return ok;
 }
 
 // Spare blocks (gal_config.spare_blocks): the slot's prepared next block is
@@ -834,10 +981,13 @@ GAL_DEVICE_COLD bool swap_spare(const state *s, uint32_t tree, uint32_t slot, ui
 GAL_DEVICE_COLD void refill_spare(const state *s, uint32_t tree, uint32_t slot, uint64_t tid) {
   const uint32_t si = s->slot_base[tree] + slot;
   if (ld_rlx(s->spares + si) != NOBLK) return;
-  const uint32_t nb = request_block(s, tree, tid);
-  if (nb == NOBLK) return;
-  __threadfence();
-  if (atomicCAS(s->spares + si, NOBLK, nb) != NOBLK) retire_block(s, nb);
+  uint32_t emptied;
+  const uint32_t nb = request_block_begin(s, tree, tid, emptied);
+  if (nb != NOBLK) {
+    fence_acq_rel();
+    if (atomicCAS(s->spares + si, NOBLK, nb) != NOBLK) retire_block(s, nb);
+  }
+  request_done(s, tree, emptied);
 }
 
 // Gallatin::boot_block (gallatin.cuh:726-787)
@@ -846,6 +996,7 @@ GAL_DEVICE_COLD bool boot_block(const state *s, uint32_t tree, uint32_t slot, ui
   uint32_t blk = request_block(s, tree, tid);
   if (blk == NOBLK) return false;
   if (ld_rlx(&s->tree_ids[blk >> s->bps_shift]) != tree) return false;
+  fence_acq_rel();
   return atomicCAS(s->slots + s->slot_base[tree] + slot, NOBLK, blk) == NOBLK;
 }
 
@@ -905,12 +1056,16 @@ GAL_DEVICE_COLD bool claim_slow_path(const state *s, uint32_t tree, uint32_t slo
 // and does nothing, and the slot that does hold the block keeps it exhausted.
 // Every failed claim still adds to the block's count, so a block left
 // exhausted in a slot soon reads far past its end: a team that reads its
-// slot's block more than STUCK_MARGIN slices past the end replaces it itself
+// slot's block more than STUCK_MARGIN slices past the end, has tried
+// STUCK_ATTEMPTS times and still finds the block in the slot replaces it itself
 // (a compare-and-swap on the slot, so at most one replacement happens).  The
-// rightful crosser swaps its block within a few claims of the end, so the
-// margin keeps the teams out of each other's way.  One thread alone never
+// rightful crosser swaps its block within a few round trips of the end; where
+// many SMs share a slot their failed claims pass the margin in that time, and
+// without the attempts (some 20 us of them) they took the swap from the crosser
+// and requested blocks that had to be handed back.  One thread alone never
 // meets an exhausted block in its slot, so serial offsets are unchanged.
 static constexpr uint32_t STUCK_MARGIN = 1u << 12;
+static constexpr int STUCK_ATTEMPTS = 16;
 template <bool NAMED>
 GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t count, uint32_t pending,
                                       slot_cache *cache = nullptr) {
@@ -977,7 +1132,8 @@ GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t co
       if (cache) {  // exhausted, replaced or foreign: the next team reads the slot again
         if ((rep || exhausted || foreign) && (int)lane == leader) atomicCAS(&cache->blk[tree], blk, NOBLK);
       }
-      if (exhausted && fresh && (old & 0xFFFFFFFFull) >= SLICES_PER_BLOCK + STUCK_MARGIN)
+      if (exhausted && fresh && attempt >= STUCK_ATTEMPTS && (old & 0xFFFFFFFFull) >= SLICES_PER_BLOCK + STUCK_MARGIN &&
+          ld_rlx(s->slots + s->slot_base[tree] + slot) == blk)
         rep = team;  // the slot has held an exhausted block for a while: replace it here
       const bool lead = rep && (int)lane == leader;
       if (credit || lead) refill = claim_slow_path(s, tree, slot, blk, credit, lead, tid);
