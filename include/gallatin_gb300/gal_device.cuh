@@ -286,6 +286,24 @@ GAL_DEVICE_INLINE bool veb_query(const veb_ref &v, uint64_t x) {
   return (ld_rlx(v.word(v.sh->layers - 1, x >> 6)) >> (x & 63)) & 1ULL;
 }
 
+// Takes a word this thread emptied off the summaries above it.
+GAL_DEVICE_INLINE void veb_unlist(const veb_ref &v, int layer, uint64_t high) {
+  while (layer > 0) {
+    uint64_t *child = v.word(layer, high);
+    layer -= 1;
+    const int low = (int)(high & 63);
+    high >>= 6;
+    fence_acq_rel();
+    const uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
+    fence_acq_rel();
+    if (ld_rlx(child) != 0) {  // an insert raced in: keep the summary bit
+      amo_or(v.word(layer, high), 1ULL << low);
+      return;
+    }
+    if (__popcll(old) != 1) return;
+  }
+}
+
 // veb_tree::remove (veb.cuh:737-755) plus the child re-check.  A remove that
 // empties a word clears the word's summary bit, then reads the word again: an
 // insert that refilled it meanwhile set the word's bit before the summary's,
@@ -303,19 +321,7 @@ GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x, uint64_t &left) 
   uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
   left = old & ~(1ULL << low);
   if (!(old & (1ULL << low))) return false;
-  while (__popcll(old) == 1 && layer > 0) {
-    uint64_t *child = v.word(layer, high);
-    layer -= 1;
-    low = (int)(high & 63);
-    high >>= 6;
-    fence_acq_rel();
-    old = amo_and(v.word(layer, high), ~(1ULL << low));
-    fence_acq_rel();
-    if (ld_rlx(child) != 0) {  // an insert raced in: keep the summary bit
-      amo_or(v.word(layer, high), 1ULL << low);
-      break;
-    }
-  }
+  if (left == 0) veb_unlist(v, layer, high);
   return true;
 }
 
@@ -564,6 +570,47 @@ GAL_DEVICE_COLD uint64_t veb_gather_run(const veb_ref &v, uint64_t needed) {
     if ((uint64_t)__popcll(fb & fmask) == n) return sb * 64 + 64 - n;
     amo_or(v.word(bottom, sb), fmask & fb);
     veb_rollback(v, sb + 1, needed - n);
+  }
+  return FAIL;
+}
+
+// A run of n segments (at most 64) for a thread that met another one searching:
+// taken from the trailing ones of one word with a compare-and-swap, as
+// veb_gather_run takes it but from any of the topmost RUN_CHOICES words that
+// have room, each thread starting at one of its own.  Nothing is held by a
+// failed try, so the threads need no lock among themselves.  FAIL: no single
+// word has room (a run across words needs the locked search).
+static constexpr int RUN_CHOICES = 16;
+GAL_DEVICE_COLD uint64_t veb_gather_in_word(const veb_ref &v, uint64_t n) {
+  const int bottom = (int)v.sh->layers - 1;
+  uint64_t *const words = v.word(bottom, 0);
+  uint32_t pick[RUN_CHOICES];
+  int choices = 0;
+  // eight loads in flight: the words below a full top cost one round trip per eight
+  for (int64_t hi = (int64_t)v.sh->nwords[bottom] - 1; hi >= 0 && choices < RUN_CHOICES; hi -= 8) {
+    uint64_t w[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) w[k] = hi - k >= 0 ? ld_rlx(words + (hi - k)) : 0ull;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+      if ((uint64_t)cfc64(w[k]) >= n && choices < RUN_CHOICES) pick[choices++] = (uint32_t)(hi - k);
+  }
+  if (choices == 0) return FAIL;
+  int at = (int)(((uint32_t)(thread_linear_id() * 0x9E3779B1u) >> 16) % (uint32_t)choices);
+  for (int tries = 0; tries < choices; tries++) {
+    uint64_t *word = words + pick[at];
+    uint64_t seen = ld_rlx(word);
+    for (int c; (uint64_t)(c = cfc64(seen)) >= n;) {
+      const uint64_t acq = bitmask((int)n) << (c - (int)n);
+      const uint64_t got = atomicCAS((unsigned long long *)word, (unsigned long long)seen,
+                                     (unsigned long long)(seen & ~acq));
+      if (got == seen) {
+        if ((seen & ~acq) == 0) veb_unlist(v, bottom, pick[at]);
+        return (uint64_t)pick[at] * 64u + (uint64_t)(c - (int)n);
+      }
+      seen = got;
+    }
+    if (++at == choices) at = 0;
   }
   return FAIL;
 }
@@ -1168,11 +1215,22 @@ GAL_DEVICE_COLD void *malloc_whole_block(const state *s, uint32_t tree) {
   return nullptr;
 }
 
-// Gallatin::malloc_segment_allocation (gallatin.cuh:790-826)
+// Gallatin::malloc_segment_allocation (gallatin.cuh:790-826).  The reference
+// queues every request on one lock; 85 runs asked for together then took 8 us
+// each, one after another.  A request that finds the lock taken looks for its
+// run inside one word by itself first and waits only if there is none.
 GAL_DEVICE_COLD void *malloc_segment_run(const state *s, uint32_t count) {
   for (int a = 0; a < SEGMENT_ATTEMPTS; a++) {
     uint32_t spins = 0;
     while (!try_lock(s, s->num_trees)) {
+      if (spins == 0 && count <= 64) {
+        const uint64_t idx = veb_gather_in_word(seg_tree(s), count);
+        if (idx != FAIL) {
+          if (cas16(&s->tree_ids[idx], FREE_TREE, (uint16_t)(s->num_trees + 1 + count)) != FREE_TREE)
+            set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+          return s->memory + (idx << s->seg_shift);
+        }
+      }
       if (++spins > s->spin_limit) {
         set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_RUN_LOCK, count, spins);
         return nullptr;
