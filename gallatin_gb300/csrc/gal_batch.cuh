@@ -40,7 +40,7 @@ struct cta_claim_smem {
 // Claim `want` slices of class `tree` for this CTA; records up to CTA_RUNS runs.
 static __device__ __noinline__ void cta_claim_class(const state *s, uint32_t tree, uint32_t want,
                                              cta_claim_smem &sm) {
-  const uint64_t tid = thread_linear_id();
+  const uint32_t tid = (uint32_t)thread_linear_id();
   uint32_t assigned = 0, nruns = 0;
   // a persistent CTA keeps claiming from the block it used last and reads the
   // pinned slot again only after a claim comes back exhausted or foreign
@@ -125,7 +125,7 @@ __device__ __forceinline__ void cta_sync(const cta_claim_smem &sm) {
 // Returns when the workers set `stop` (or after a bounded number of polls).
 GAL_DEVICE_COLD void cta_service(const state *s, cta_claim_smem &sm) {
   if (lane_id() != 0 || !s->use_spares) return;
-  const uint64_t tid = thread_linear_id();
+  const uint32_t tid = (uint32_t)thread_linear_id();
   for (uint32_t it = 0; it < (1u << 24); it++) {
     bool work = false;
     for (uint32_t t = 0; t < s->num_trees; t++) {
@@ -240,7 +240,7 @@ GAL_DEVICE_INLINE void run_cache_init(run_cache &c) {
 // prepare again (after using the run), else NOBLK.
 GAL_DEVICE_COLD uint32_t claim_run(const state *s, uint32_t tree, uint32_t want, run_cache &rc, uint32_t &run_blk,
                                    uint32_t &run_start, uint32_t &spare_slot) {
-  const uint64_t tid = thread_linear_id();
+  const uint32_t tid = (uint32_t)thread_linear_id();
   uint32_t blk = rc.blk[tree], slot = rc.slot[tree];
   spare_slot = NOBLK;
   for (int attempt = 0; attempt < CTA_CLAIM_ATTEMPTS; attempt++) {

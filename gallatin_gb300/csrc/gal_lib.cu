@@ -61,7 +61,7 @@ __global__ void k_init_words(gal::state st, uint64_t nblocks) {
   const gal::veb_shape &sh = st.veb;
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t b = i; b < nblocks; b += stride) *gal::mword_ptr(&st, (uint32_t)b) = 4097ull;
+  for (uint64_t b = i; b < nblocks; b += stride) st.mwords[b * st.mstride] = 4097ull;
   for (uint64_t g = i; g < st.num_segments; g += stride) st.act[g] = gal::act_word(0, gal::ACT_FREE, -1);
   for (uint32_t l = 0; l < sh.layers; l++) {
     uint64_t items = sh.items[l];

@@ -109,14 +109,33 @@ struct state {
   uint32_t *error;               // GAL_DEV_ERR_* bits
 };
 
+// A field of the state (or of its tree shape), which lives in global memory, on
+// the device: constant while a kernel runs, so it is read through the read-only path, whose cached lines
+// outlive fences.  Ordinary loads miss L1 after every fence or acquire (345
+// cycles each, several in a row on the block-request path).
+template <class T>
+GAL_DEVICE_INLINE __host__ T cfield(const T &f) {
+#ifdef __CUDA_ARCH__
+  static_assert(sizeof(T) == 8 || sizeof(T) == 4, "a word or a pointer");
+  if constexpr (sizeof(T) == 8) {
+    const unsigned long long v = __ldg((const unsigned long long *)&f);
+    return (T)v;
+  } else {
+    return (T)__ldg((const unsigned int *)&f);
+  }
+#else
+  return f;
+#endif
+}
+
 // ------------------------------------------------------------------ layout
 static constexpr uint32_t BLOCK_RECORD_BYTES = 32;  // block_layout 1: one sector per block
 static constexpr uint32_t LOCK_STRIDE = 8;          // u32 words between lock words (32 B)
 GAL_DEVICE_INLINE __host__ unsigned long long *mword_ptr(const state *s, uint32_t blk) {
-  return s->mwords + (uint64_t)blk * s->mstride;
+  return cfield(s->mwords) + (uint64_t)blk * cfield(s->mstride);
 }
 GAL_DEVICE_INLINE __host__ uint32_t *fctr_ptr(const state *s, uint32_t blk) {
-  return s->fctr + (uint64_t)blk * s->fstride;
+  return cfield(s->fctr) + (uint64_t)blk * cfield(s->fstride);
 }
 // A segment's count word: in the low half the reference's active count (blocks
 // left to hand out minus one; -1 when none is left or the segment is free) plus
@@ -156,7 +175,7 @@ GAL_DEVICE_INLINE uint32_t lanemask_lt() {
 // The lanes this lane may aggregate with: the whole warp (team_width 32, the
 // reference's coalesced team) or its aligned group of team_width lanes.
 GAL_DEVICE_INLINE uint32_t team_group(const state *s) {
-  const uint32_t w = s->team_width;
+  const uint32_t w = cfield(s->team_width);
   if (w >= 32) return 0xFFFFFFFFu;
   return ((1u << w) - 1u) << (lane_id() & ~(w - 1u));
 }
@@ -187,8 +206,8 @@ GAL_DEVICE_INLINE uint16_t ld_rlx(const uint16_t *p) {
   return v;
 }
 // acquire-release fence at device scope: orders this thread's earlier and
-// later memory accesses (lighter than __threadfence's sequentially
-// consistent one)
+// later memory accesses.  It costs a round trip of its own (some 800 cycles
+// with nothing outstanding, as much as an atomic), as __threadfence does.
 GAL_DEVICE_INLINE void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 GAL_DEVICE_INLINE uint64_t amo_or(uint64_t *p, uint64_t v) {
   return atomicOr((unsigned long long *)p, (unsigned long long)v);
@@ -208,16 +227,19 @@ GAL_DEVICE_INLINE void st_rlx(unsigned long long *p, unsigned long long v) {
 GAL_DEVICE_INLINE void st_rlx(uint32_t *p, uint32_t v) {
   asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+GAL_DEVICE_INLINE void st_rlx(uint16_t *p, uint16_t v) {
+  asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"(v) : "memory");
+}
 GAL_DEVICE_INLINE uint16_t cas16(uint16_t *p, uint16_t cmp, uint16_t val) {
   return (uint16_t)atomicCAS((unsigned short *)p, (unsigned short)cmp, (unsigned short)val);
 }
-GAL_DEVICE_INLINE void set_error(const state *s, uint32_t bits) { atomicOr(s->error, bits); }
+GAL_DEVICE_INLINE void set_error(const state *s, uint32_t bits) { atomicOr(cfield(s->error), bits); }
 // error word plus the first error's site and two values (error[2..9] as 4 u64:
 // site, a, b, taken) for gal_error_info
 GAL_DEVICE_COLD void set_error_info(const state *s, uint32_t bits, uint64_t site, uint64_t a,
                                     uint64_t b) {
-  atomicOr(s->error, bits);
-  unsigned long long *info = (unsigned long long *)(s->error + 2);
+  atomicOr(cfield(s->error), bits);
+  unsigned long long *info = (unsigned long long *)(cfield(s->error) + 2);
   if (atomicCAS(&info[3], 0ull, 1ull) == 0ull) {
     info[0] = site;
     info[1] = a;
@@ -259,7 +281,7 @@ GAL_DEVICE_INLINE uint64_t murmur64a_u64(uint64_t key, uint64_t seed) {
 
 GAL_DEVICE_INLINE uint64_t bitmask(int n) { return n >= 64 ? ~0ULL : ((1ULL << n) - 1ULL); }
 GAL_DEVICE_INLINE uint32_t blocks_in_segment(const state *s, uint32_t tree) {
-  return 1u << (s->bps_shift - tree);
+  return 1u << (cfield(s->bps_shift) - tree);
 }
 GAL_DEVICE_INLINE uint64_t thread_linear_id() {
   return (uint64_t)(threadIdx.x + blockIdx.x * blockDim.x);  // 32-bit as veb.cuh:948
@@ -272,22 +294,25 @@ struct veb_ref {
   uint64_t *w;
   const veb_shape *sh;
   uint64_t seed;
-  GAL_DEVICE_INLINE uint64_t *word(int layer, uint64_t high) const { return w + sh->off[layer] + high; }
+  GAL_DEVICE_INLINE uint64_t *word(int layer, uint64_t high) const { return w + cfield(sh->off[layer]) + high; }
 };
 
 GAL_DEVICE_INLINE int veb_find_next(const veb_ref &v, int layer, uint64_t high, int low) {
-  if (high >= v.sh->items[layer]) return -1;  // layer::find_next, veb.cuh:250-275
+  if (high >= cfield(v.sh->items[layer])) return -1;  // layer::find_next, veb.cuh:250-275
   uint64_t b = ld_rlx(v.word(layer, high));
   if (low == -1) return __ffsll((long long)b) - 1;
   return __ffsll((long long)(b & ~bitmask(low + 1))) - 1;
 }
 
 GAL_DEVICE_INLINE bool veb_query(const veb_ref &v, uint64_t x) {
-  return (ld_rlx(v.word(v.sh->layers - 1, x >> 6)) >> (x & 63)) & 1ULL;
+  return (ld_rlx(v.word(cfield(v.sh->layers) - 1, x >> 6)) >> (x & 63)) & 1ULL;
 }
 
 // Takes a word this thread emptied off the summaries above it.
-GAL_DEVICE_INLINE void veb_unlist(const veb_ref &v, int layer, uint64_t high) {
+GAL_DEVICE_COLD void veb_unlist(uint64_t *w, const veb_shape *sh, uint32_t word) {
+  const veb_ref v{w, sh, 0};
+  int layer = (int)cfield(sh->layers) - 1;
+  uint64_t high = word;
   while (layer > 0) {
     uint64_t *child = v.word(layer, high);
     layer -= 1;
@@ -315,13 +340,13 @@ GAL_DEVICE_INLINE void veb_unlist(const veb_ref &v, int layer, uint64_t high) {
 // a clear summary bit, where top-down searches never find its items.
 // `left` receives the other items the bottom word held.
 GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x, uint64_t &left) {
-  int layer = (int)v.sh->layers - 1;
-  uint64_t high = x >> 6;
-  int low = (int)(x & 63);
-  uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
+  const int layer = (int)cfield(v.sh->layers) - 1;
+  const uint64_t high = x >> 6;
+  const int low = (int)(x & 63);
+  const uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
   left = old & ~(1ULL << low);
   if (!(old & (1ULL << low))) return false;
-  if (left == 0) veb_unlist(v, layer, high);
+  if (left == 0) veb_unlist(v.w, v.sh, (uint32_t)high);
   return true;
 }
 
@@ -330,27 +355,30 @@ GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x) {
   return veb_remove(v, x, left);
 }
 
+// Lists a bottom word this thread found empty in the summaries above it.
+GAL_DEVICE_COLD void veb_list_above(uint64_t *w, const veb_shape *sh, uint32_t word) {
+  const veb_ref v{w, sh, 0};
+  uint64_t high = word, old = 0;
+  for (int layer = (int)cfield(sh->layers) - 2; layer >= 0 && old == 0; layer--) {
+    fence_acq_rel();
+    old = amo_or(v.word(layer, high >> 6), 1ULL << (high & 63));
+    high >>= 6;
+  }
+}
+
 // veb_tree::insert_force_update (veb.cuh:775-798); the fence orders each
 // word's set before its summary's (see veb_remove)
 GAL_DEVICE_INLINE bool veb_insert(const veb_ref &v, uint64_t x) {
-  int layer = (int)v.sh->layers - 1;
-  uint64_t high = x >> 6;
-  int low = (int)(x & 63);
-  uint64_t old = amo_or(v.word(layer, high), 1ULL << low);
-  if (old & (1ULL << low)) return false;
-  while (__popcll(old) == 0 && layer > 0) {
-    layer -= 1;
-    low = (int)(high & 63);
-    high >>= 6;
-    fence_acq_rel();
-    old = amo_or(v.word(layer, high), 1ULL << low);
-  }
-  return true;
+  const int layer = (int)cfield(v.sh->layers) - 1;
+  const uint64_t high = x >> 6;
+  const uint64_t old = amo_or(v.word(layer, high), 1ULL << (x & 63));
+  if (old == 0) veb_list_above(v.w, v.sh, (uint32_t)high);
+  return !((old >> (x & 63)) & 1ULL);
 }
 
 // veb_tree::successor_thorough (veb.cuh:878-916): smallest item > q
 GAL_DEVICE_COLD uint64_t veb_successor(const veb_ref &v, uint64_t q) {
-  const int bottom = (int)v.sh->layers - 1;
+  const int bottom = (int)cfield(v.sh->layers) - 1;
   uint64_t high = q >> 6;
   int low = (int)(q & 63);
   int layer = bottom;
@@ -387,37 +415,54 @@ GAL_DEVICE_INLINE uint64_t veb_lock_offset(const veb_ref &v, uint64_t start) {
 }
 
 // Trees of up to 64 bottom words (4,096 segments) are searched top-down from
-// the one summary word above them, held in a register: `top` has the bottom
-// words that are not empty (a one-layer tree is its only bottom word).  Each
-// search below
-// then costs two or three dependent loads, where climbing from a start word
-// and coming down again for every start tried cost eight to ten (a block
-// request spent 6 of its 13 us there).
-GAL_DEVICE_INLINE bool veb_shallow(const veb_ref &v) { return v.sh->nwords[v.sh->layers - 1] <= 64; }
-GAL_DEVICE_INLINE uint64_t veb_top(const veb_ref &v) {
-  return v.sh->layers > 1 ? ld_rlx(v.w + v.sh->off[v.sh->layers - 2]) : 1ull;
+// the one summary word above them: `top` has the bottom words that are not
+// empty (a one-layer tree is its only bottom word).  Bottom word 0 is loaded
+// along with it, and segments are taken lowest first, so a search costs one or
+// two dependent loads (an L2 load of a word another SM has just changed takes
+// ~700 cycles); climbing from a start word and coming down again for every
+// start tried took eight to ten of them.
+struct veb_low {
+  uint64_t top, word0;
+};
+GAL_DEVICE_INLINE bool veb_shallow(const veb_ref &v) {
+  return cfield(v.sh->nwords[cfield(v.sh->layers) - 1]) <= 64;
 }
-GAL_DEVICE_INLINE uint64_t *veb_bottom(const veb_ref &v) { return v.w + v.sh->off[v.sh->layers - 1]; }
+GAL_DEVICE_INLINE uint64_t *veb_bottom(const veb_ref &v) {
+  return v.w + cfield(v.sh->off[cfield(v.sh->layers) - 1]);
+}
+GAL_DEVICE_INLINE veb_low veb_load_low(const veb_ref &v, const uint64_t *bottom) {
+  const uint32_t layers = cfield(v.sh->layers);
+  veb_low l;
+  l.top = layers > 1 ? ld_rlx(v.w + cfield(v.sh->off[layers - 2])) : 1ull;
+  l.word0 = ld_rlx(bottom);
+  return l;
+}
+GAL_DEVICE_INLINE uint64_t veb_low_word(const veb_low &l, const uint64_t *bottom, uint64_t high) {
+  return high ? ld_rlx(bottom + high) : l.word0;
+}
 
 // veb_tree::malloc_first (veb.cuh:979-991): takes the smallest item.  Threads
 // that lose it to one another would all go for the next smallest together, one
 // winner per round trip; each loser goes on from the word as its own attempt
 // left it, at a place of its own, so k contenders are served in a few round
 // trips.  One thread alone never loses and always gets the smallest.
-GAL_DEVICE_COLD uint64_t veb_malloc_first(const veb_ref &v) {
-  if (!veb_shallow(v)) {
-    for (int a = 0; a < VEB_ATTEMPTS; a++) {
-      uint64_t o = veb_lock_offset(v, 0);
-      if (o != FAIL) return o;
-    }
-    return FAIL;
+// `l` is the start of the search, loaded by the caller.
+GAL_DEVICE_COLD uint64_t veb_malloc_first_deep(uint64_t *w, const veb_shape *sh) {
+  const veb_ref v{w, sh, 0};
+  for (int a = 0; a < VEB_ATTEMPTS; a++) {
+    uint64_t o = veb_lock_offset(v, 0);
+    if (o != FAIL) return o;
   }
+  return FAIL;
+}
+GAL_DEVICE_INLINE uint64_t veb_malloc_first(const veb_ref &v, veb_low l) {
+  if (!veb_shallow(v)) return veb_malloc_first_deep(v.w, v.sh);
   uint64_t *bottom = veb_bottom(v);
   const uint32_t spread = (uint32_t)(thread_linear_id() * 0x9E3779B1u) >> 26;
-  for (int a = 0; a < VEB_ATTEMPTS; a++) {
-    for (uint64_t top = veb_top(v); top; top &= top - 1ull) {
+  for (int a = 0; a < VEB_ATTEMPTS; a++, l = veb_load_low(v, bottom)) {
+    for (uint64_t top = l.top; top; top &= top - 1ull) {
       const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
-      uint64_t word = ld_rlx(bottom + high);
+      uint64_t word = veb_low_word(l, bottom, high);
       for (uint32_t turn = 0; word; turn = spread) {
         const uint64_t turned = (word >> turn) | (turn ? word << (64u - turn) : 0ull);
         const uint64_t low = ((uint64_t)(__ffsll((long long)turned) - 1) + turn) & 63u;
@@ -428,67 +473,107 @@ GAL_DEVICE_COLD uint64_t veb_malloc_first(const veb_ref &v) {
   return FAIL;
 }
 
-// The smallest listed item at or above `start`, which must not exceed an item
-// last seen listed in bottom word `last` (its content then: `last_word`).
-GAL_DEVICE_INLINE uint64_t veb_at_or_above(const uint64_t *bottom, uint64_t top, uint64_t start, uint64_t last,
-                                           uint64_t last_word) {
-  uint64_t high = start >> 6;
-  uint64_t word = (high == last ? last_word : ld_rlx(bottom + high)) & ~bitmask((int)(start & 63u));
-  while (!word) {  // reaches `last` at the latest, whose remembered word holds an item above start
-    const uint64_t above = top & ~bitmask((int)high + 1);
-    high = above ? (uint64_t)(__ffsll((long long)above) - 1) : last;
-    word = high >= last ? last_word : ld_rlx(bottom + high);
+GAL_DEVICE_COLD uint64_t veb_find_random_deep(uint64_t *w, const veb_shape *sh, uint64_t seed, uint64_t tid) {
+  const veb_ref v{w, sh, seed};
+  const uint64_t U = cfield(sh->items[cfield(sh->layers) - 1]);
+  const uint64_t h1 = murmur64a_u64(tid, seed);
+  const uint64_t h2 = murmur64a_u64(tid, h1);
+  uint64_t empty_from = U;  // no item in [empty_from, U)
+  for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
+    uint64_t start = (h1 + a * h2) % U;
+    if (start >= empty_from) continue;
+    if (veb_query(v, start)) return start;
+    uint64_t idx = veb_successor(v, start);
+    if (idx != FAIL) return idx;
+    empty_from = start;
   }
-  return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
+  return veb_successor(v, 0);
 }
 
 // veb_tree::find_random_valid_index (veb.cuh:946-977): of 15 hashed starts the
 // first with a listed item at or above it gives the smallest such item; if none
 // has one, the smallest item above 0.  A start has one exactly when it does not
-// exceed the largest listed item, so that is found first (two loads) and the
-// starts are tried in registers.  A deeper tree is searched from each start;
-// one that found nothing shows that no item lies in [start, U), and later
-// starts at or above the lowest such start are skipped.
-GAL_DEVICE_COLD uint64_t veb_find_random(const veb_ref &v, uint64_t tid) {
-  const uint64_t U = v.sh->items[v.sh->layers - 1];
-  const uint64_t h1 = murmur64a_u64(tid, v.seed);
-  const uint64_t h2 = murmur64a_u64(tid, h1);
-  if (!veb_shallow(v)) {
-    uint64_t empty_from = U;  // no item in [empty_from, U)
-    for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
-      uint64_t start = (h1 + a * h2) % U;
-      if (start >= empty_from) continue;
-      if (veb_query(v, start)) return start;
-      uint64_t idx = veb_successor(v, start);
-      if (idx != FAIL) return idx;
-      empty_from = start;
-    }
-    return veb_successor(v, 0);
-  }
+// exceed the largest listed item, so the starts are tried in registers once
+// that is known, and a tree that lists one item other than 0 needs none (the
+// hashes took 1,200 cycles).  A deeper tree is searched from each start; one
+// that found nothing shows that no item lies in [start, U), and later starts at
+// or above the lowest such start are skipped.
+GAL_DEVICE_INLINE uint64_t veb_find_random(const veb_ref &v, uint64_t tid) {
+  const uint64_t U = cfield(v.sh->items[cfield(v.sh->layers) - 1]);
+  if (!veb_shallow(v)) return veb_find_random_deep(v.w, v.sh, v.seed, tid);
   const uint64_t *bottom = veb_bottom(v);
-  uint64_t top = veb_top(v), last = 0, last_word = 0;
+  const veb_low l = veb_load_low(v, bottom);
+  uint64_t top = l.top, last = 0, last_word = 0;  // the highest word with an item
   while (top) {
     last = 63u - (uint64_t)__clzll((long long)top);
-    last_word = ld_rlx(bottom + last);
+    last_word = veb_low_word(l, bottom, last);
     if (last_word) break;
     top &= ~(1ull << last);  // emptied since its summary was read
   }
   if (!last_word) return FAIL;
   const uint64_t largest = (last << 6) + 63u - (uint64_t)__clzll((long long)last_word);
-  for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
-    const uint64_t start = (U & (U - 1ull)) == 0 ? (h1 + a * h2) & (U - 1ull) : (h1 + a * h2) % U;
-    if (start <= largest) return veb_at_or_above(bottom, top, start, last, last_word);
+  uint64_t start = 1;
+  if ((top & (top - 1ull)) != 0 || (last_word & (last_word - 1ull)) != 0 || largest == 0) {
+    const uint64_t h1 = murmur64a_u64(tid, v.seed);
+    const uint64_t h2 = murmur64a_u64(tid, h1);
+    if ((U & (U - 1ull)) == 0) {  // only the low bits of the starts count
+      const uint32_t mask = (uint32_t)U - 1u;
+      uint32_t at = (uint32_t)h1;
+#pragma unroll 5
+      for (int a = 0; a < VEB_ATTEMPTS; a++, at += (uint32_t)h2)
+        if ((at & mask) <= largest) {
+          start = at & mask;
+          break;
+        }
+    } else {
+      for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++) {
+        const uint64_t at = (h1 + a * h2) % U;
+        if (at <= largest) {
+          start = at;
+          break;
+        }
+      }
+    }
+    if (start > largest) return FAIL;  // item 0 alone, and no start found it
   }
-  return largest ? veb_at_or_above(bottom, top, 1, last, last_word) : FAIL;
+  // the smallest item at or above start
+  uint64_t high = start >> 6;
+  uint64_t word = (high == last ? last_word : veb_low_word(l, bottom, high)) & ~bitmask((int)(start & 63u));
+  while (!word) {  // reaches `last` at the latest, whose remembered word holds an item above start
+    const uint64_t above = top & ~bitmask((int)high + 1);
+    high = above ? (uint64_t)(__ffsll((long long)above) - 1) : last;
+    word = high >= last ? last_word : veb_low_word(l, bottom, high);
+  }
+  return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
+}
+
+// Any listed item, a different one for different `spread`s (FAIL: none): for a
+// thread that another has beaten to the item the rule above gives, which
+// threads that search together mostly agree on.
+GAL_DEVICE_INLINE uint64_t veb_find_any(const veb_ref &v, uint32_t spread) {
+  if (!veb_shallow(v)) return veb_find_random(v, spread);
+  const uint64_t *bottom = veb_bottom(v);
+  const veb_low l = veb_load_low(v, bottom);
+  uint64_t top = l.top;
+  for (uint32_t k = top ? spread % (uint32_t)__popcll(top) : 0; k; k--) top = top & (top - 1ull);
+  for (; top; top &= top - 1ull) {
+    const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
+    uint64_t word = veb_low_word(l, bottom, high);
+    if (!word) continue;
+    for (uint32_t k = (spread >> 8) % (uint32_t)__popcll(word); k; k--) word &= word - 1ull;
+    return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
+  }
+  return FAIL;
 }
 
 // veb_tree::find_first_valid_index (veb.cuh:940-944): smallest listed id
 GAL_DEVICE_INLINE uint64_t veb_find_first(const veb_ref &v) {
   if (veb_shallow(v)) {
     const uint64_t *bottom = veb_bottom(v);
-    for (uint64_t top = veb_top(v); top; top &= top - 1ull) {
+    const veb_low l = veb_load_low(v, bottom);
+    for (uint64_t top = l.top; top; top &= top - 1ull) {
       const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
-      const uint64_t word = ld_rlx(bottom + high);
+      const uint64_t word = veb_low_word(l, bottom, high);
       if (word) return (high << 6) + (uint64_t)(__ffsll((long long)word) - 1);
     }
     return FAIL;
@@ -504,7 +589,7 @@ GAL_DEVICE_INLINE int cfc64(uint64_t b) {  // alloc_utils.cuh:440-453
 }
 
 GAL_DEVICE_INLINE void veb_rollback(const veb_ref &v, uint64_t start_block, uint64_t nbits) {
-  const int bottom = (int)v.sh->layers - 1;  // layer::rollback, veb.cuh:305-321
+  const int bottom = (int)cfield(v.sh->layers) - 1;  // layer::rollback, veb.cuh:305-321
   while (nbits > 64) {
     amo_or(v.word(bottom, start_block), ~0ULL);
     nbits -= 64;
@@ -516,11 +601,11 @@ GAL_DEVICE_INLINE void veb_rollback(const veb_ref &v, uint64_t start_block, uint
 // layer::gather_multiple (veb.cuh:323-452) on the bottom layer: claims a run
 // ending in the trailing ones of a word, scanning words from the top down.
 GAL_DEVICE_COLD uint64_t veb_gather_run(const veb_ref &v, uint64_t needed) {
-  const int bottom = (int)v.sh->layers - 1;
-  uint64_t sb = v.sh->nwords[bottom] - 1;
+  const int bottom = (int)cfield(v.sh->layers) - 1;
+  uint64_t sb = cfield(v.sh->nwords[bottom]) - 1;
   // every pass either moves down a word or retries one that changed under it;
   // bound the retries so heavy interference ends in a clean failure
-  uint64_t budget = 8ull * v.sh->nwords[bottom] + 1024;
+  uint64_t budget = 8ull * cfield(v.sh->nwords[bottom]) + 1024;
   while (sb != 0) {
     if (budget-- == 0) return FAIL;
     uint64_t n = needed;
@@ -582,12 +667,12 @@ GAL_DEVICE_COLD uint64_t veb_gather_run(const veb_ref &v, uint64_t needed) {
 // word has room (a run across words needs the locked search).
 static constexpr int RUN_CHOICES = 16;
 GAL_DEVICE_COLD uint64_t veb_gather_in_word(const veb_ref &v, uint64_t n) {
-  const int bottom = (int)v.sh->layers - 1;
+  const int bottom = (int)cfield(v.sh->layers) - 1;
   uint64_t *const words = v.word(bottom, 0);
   uint32_t pick[RUN_CHOICES];
   int choices = 0;
   // eight loads in flight: the words below a full top cost one round trip per eight
-  for (int64_t hi = (int64_t)v.sh->nwords[bottom] - 1; hi >= 0 && choices < RUN_CHOICES; hi -= 8) {
+  for (int64_t hi = (int64_t)cfield(v.sh->nwords[bottom]) - 1; hi >= 0 && choices < RUN_CHOICES; hi -= 8) {
     uint64_t w[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) w[k] = hi - k >= 0 ? ld_rlx(words + (hi - k)) : 0ull;
@@ -605,7 +690,7 @@ GAL_DEVICE_COLD uint64_t veb_gather_in_word(const veb_ref &v, uint64_t n) {
       const uint64_t got = atomicCAS((unsigned long long *)word, (unsigned long long)seen,
                                      (unsigned long long)(seen & ~acq));
       if (got == seen) {
-        if ((seen & ~acq) == 0) veb_unlist(v, bottom, pick[at]);
+        if ((seen & ~acq) == 0) veb_unlist(v.w, v.sh, pick[at]);
         return (uint64_t)pick[at] * 64u + (uint64_t)(c - (int)n);
       }
       seen = got;
@@ -620,7 +705,7 @@ GAL_DEVICE_COLD uint64_t veb_gather_multiple(const veb_ref &v, uint64_t n) {
   uint64_t found = veb_gather_run(v, n);
   if (found == FAIL) return FAIL;
   uint64_t lo = found;
-  for (int i = (int)v.sh->layers - 2; i >= 0; i--) {
+  for (int i = (int)cfield(v.sh->layers) - 2; i >= 0; i--) {
     uint64_t hi = (lo + n - 1) / 64 + 1;
     lo = lo / 64;
     n = hi - lo;
@@ -638,7 +723,7 @@ GAL_DEVICE_COLD uint64_t veb_gather_multiple(const veb_ref &v, uint64_t n) {
 
 // veb_tree::return_multiple (veb.cuh:1198-1218, layer form veb.cuh:495-523)
 GAL_DEVICE_COLD void veb_return_multiple(const veb_ref &v, uint64_t start, uint64_t n) {
-  const int bottom = (int)v.sh->layers - 1;
+  const int bottom = (int)cfield(v.sh->layers) - 1;
   uint64_t bi = start / 64;
   int bs = (int)(start % 64);
   uint64_t left = n;
@@ -666,64 +751,107 @@ GAL_DEVICE_COLD void veb_return_multiple(const veb_ref &v, uint64_t start, uint6
   }
 }
 
-GAL_DEVICE_INLINE veb_ref seg_tree(const state *s) { return veb_ref{s->seg_tree, &s->veb, s->seed}; }
+GAL_DEVICE_INLINE veb_ref seg_tree(const state *s) { return veb_ref{cfield(s->seg_tree), &s->veb, cfield(s->seed)}; }
 GAL_DEVICE_INLINE veb_ref sub_tree(const state *s, uint32_t t) {
-  return veb_ref{s->sub_trees + (uint64_t)t * s->veb.words, &s->veb, s->seed + t};
+  return veb_ref{cfield(s->sub_trees) + (uint64_t)t * cfield(s->veb.words), &s->veb, cfield(s->seed) + t};
 }
 
 // ------------------------------------------------------------------ locks
 // one lock word per class (and one for runs) in a 32-byte sector of its own;
 // the reference keeps them as bits of one word (gallatin.cuh:1513-1519)
 GAL_DEVICE_INLINE bool try_lock(const state *s, uint32_t bit) {
-  return atomicExch(s->locks + bit * LOCK_STRIDE, 1u) == 0u;
+  return atomicExch(cfield(s->locks) + bit * LOCK_STRIDE, 1u) == 0u;
 }
+// What the locks keep apart is set by atomics one by one; a thread that sees a
+// lock open before the last of them only searches or gathers once more.
 GAL_DEVICE_INLINE void unlock(const state *s, uint32_t bit) {
-  fence_acq_rel();
-  st_rlx(s->locks + bit * LOCK_STRIDE, 0u);
+  st_rlx(cfield(s->locks) + bit * LOCK_STRIDE, 0u);
 }
 
 // ------------------------------------------------------------------ table
-// alloc_table::setup_segment (memory_table.cuh:746-818).  `taken` blocks (0 or
-// 1) are handed out with the set-up itself.
-GAL_DEVICE_COLD bool setup_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t taken) {
-  // the high half of a free segment's count word changes only here
-  const uint32_t high = (uint32_t)(ld_rlx(&s->act[seg]) >> 32);
-  if (cas16(&s->tree_ids[seg], FREE_TREE, (uint16_t)tree) != FREE_TREE) return false;
+// alloc_table::setup_segment (memory_table.cuh:746-818) in two steps, the second
+// after a fence.  The segment was taken from the segment tree and is this
+// thread's alone; `taken` of its blocks (0 or 1) are handed out with the set-up.
+GAL_DEVICE_INLINE bool setup_begin(const state *s, uint64_t seg, uint32_t tree, uint32_t taken) {
+  if (ld_rlx(&cfield(s->tree_ids)[seg]) != FREE_TREE) return false;
+  st_rlx(&cfield(s->tree_ids)[seg], (uint16_t)tree);
   const uint32_t nb = blocks_in_segment(s, tree);
-  uint32_t *q = s->queues + (seg << s->bps_shift);
+  uint32_t *q = cfield(s->queues) + (seg << cfield(s->bps_shift));
   if (nb >= 4) {
     for (uint32_t i = 0; i < nb; i += 4) *(uint4 *)(q + i) = make_uint4(NOBLK, NOBLK, NOBLK, NOBLK);
   } else {
     for (uint32_t i = 0; i < nb; i++) q[i] = NOBLK;
   }
-  st_rlx(&s->qc[seg], taken);
-  st_rlx(&s->qfc[seg], 0u);
-  st_rlx(&s->fqfc[seg], 0u);
-  fence_acq_rel();
-  // count -1 -> nb - 1 - taken, the class and a new generation, by addition: a
-  // reservation attempt still in flight from before the segment's release gives
-  // its one back into this count, as it took it from the count it found
-  const uint32_t next = (((high >> 8) + 1u) << 8) | tree;
-  atomicAdd(&s->act[seg], ((unsigned long long)(next - high) << 32) + nb - taken);
+  st_rlx(&cfield(s->qc)[seg], taken);
+  st_rlx(&cfield(s->qfc)[seg], 0u);
+  st_rlx(&cfield(s->fqfc)[seg], 0u);
   return true;
 }
+// count -1 -> nb - 1 - taken, class ACT_FREE -> tree, the next generation, by
+// addition: a reservation attempt still in flight from before the segment's
+// release gives its one back into this count, as it took it from the count it
+// found, and the word need not be read (its high half changes only here and
+// in the release: (gen << 8 | ACT_FREE) + tree + 1 is (gen + 1) << 8 | tree).
+// Returns the word it found, so that the count is open before the caller lists
+// the segment: a thread that found it refusing would take it off again for good.
+GAL_DEVICE_INLINE unsigned long long setup_open(const state *s, uint64_t seg, uint32_t tree, uint32_t taken) {
+  static_assert(ACT_FREE == 0xFFu, "one more than ACT_FREE carries into the generation");
+  return atomicAdd(&cfield(s->act)[seg],
+                   ((unsigned long long)(tree + 1u) << 32) + blocks_in_segment(s, tree) - taken);
+}
 
-// Gallatin::gather_new_segment (gallatin.cuh:1465-1510).  With `take` the
-// segment's first block (pos 0) is the caller's: it is counted out before the
-// segment is listed, and a segment of one block is not listed at all, as it
-// would be taken off again by the same thread.
-GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool take) {
-  uint64_t seg = veb_malloc_first(seg_tree(s));
+// Gallatin::gather_new_segment (gallatin.cuh:1465-1510): the smallest free
+// segment becomes the class's (-1: none).  With `take` its first block (pos 0)
+// is the caller's: it is counted out before the segment is listed, and a segment
+// of one block is not listed at all, as it would be taken off again by the same
+// thread.  `l`: the segment tree's first words, which the caller loads while it
+// waits for the class lock.  `more`: further segments wanted, for threads that
+// wait for the lock; as many as the same word of the segment tree has are
+// gathered along, their set-ups side by side, so that they cost little more
+// than the one (16 segments one after another took 110 us of a call that
+// wanted 256 blocks).
+GAL_DEVICE_INLINE veb_low free_segments_low(const state *s) {
+  const veb_ref v = seg_tree(s);
+  return veb_load_low(v, veb_bottom(v));
+}
+GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool take, veb_low l, uint32_t more = 0) {
+  const veb_ref free_segs = seg_tree(s);
+  const uint64_t seg = veb_malloc_first(free_segs, l);
   if (seg == FAIL) return -1;
-  if (!setup_segment(s, seg, tree, take ? 1u : 0u)) {
+  const uint64_t base = seg & ~63ull;
+  uint64_t extra = 0;
+  if (more && veb_shallow(free_segs)) {
+    uint64_t *const word = veb_bottom(free_segs) + (seg >> 6);
+    uint64_t seen = ld_rlx(word);
+    for (uint32_t k = 0; k < more && seen; k++, seen &= seen - 1ull) extra |= seen & (0ull - seen);
+    if (extra) {
+      const uint64_t old = amo_and(word, ~extra);
+      extra &= old;
+      if (extra && (old & ~extra) == 0) veb_unlist(free_segs.w, free_segs.sh, (uint32_t)(seg >> 6));
+    }
+  }
+  bool ok = setup_begin(s, seg, tree, take ? 1u : 0u);
+  if (!ok) {
     set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
-    return -1;
+    if (!extra) return -1;
   }
-  if (!take || blocks_in_segment(s, tree) > 1) {
-    fence_acq_rel();
-    veb_insert(sub_tree(s, tree), seg);
+  for (uint64_t b = extra; b; b &= b - 1ull) {
+    const uint64_t g = base + (uint64_t)__ffsll((long long)b) - 1u;
+    if (!setup_begin(s, g, tree, 0)) {
+      set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+      extra &= ~(b & (0ull - b));
+    }
   }
-  return (int64_t)seg;
+  fence_acq_rel();
+  unsigned long long closed = act_word(0, ACT_FREE, 0);
+  if (ok) closed &= setup_open(s, seg, tree, take ? 1u : 0u);
+  for (uint64_t b = extra; b; b &= b - 1ull)
+    closed &= setup_open(s, base + (uint64_t)__ffsll((long long)b) - 1u, tree, 0);
+  if (act_class(closed) != ACT_FREE) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+  const veb_ref sub = sub_tree(s, tree);
+  if (ok && (!take || blocks_in_segment(s, tree) > 1)) veb_insert(sub, seg);
+  for (uint64_t b = extra; b; b &= b - 1ull) veb_insert(sub, base + (uint64_t)__ffsll((long long)b) - 1u);
+  return ok ? (int64_t)seg : -1;
 }
 
 // Releases segment `seg` of class `tree` when its count word still reads
@@ -733,11 +861,13 @@ GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool t
 // memory_table.cuh:1226-1241).
 GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
   const unsigned long long home = act_word(gen, tree, (int32_t)nb - 1);
-  if (atomicCAS(&s->act[seg], home, act_word(gen, ACT_FREE, -1)) != home) return;
+  if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return;
   fence_acq_rel();
   veb_remove(sub_tree(s, tree), seg);
   fence_acq_rel();
-  if (cas16(&s->tree_ids[seg], (uint16_t)tree, FREE_TREE) != (uint16_t)tree) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+  // closed and unlisted, the segment is this thread's alone
+  if (ld_rlx(&cfield(s->tree_ids)[seg]) != (uint16_t)tree) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+  st_rlx(&cfield(s->tree_ids)[seg], FREE_TREE);
   fence_acq_rel();
   veb_insert(seg_tree(s), seg);
 }
@@ -750,11 +880,11 @@ GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree
 // hand-out yet the segment is a fresh one whose gatherer takes its first
 // block next, so it stays.
 GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
-  const unsigned long long old = add_acquire(&s->act[seg], 1ull);
+  const unsigned long long old = add_acquire(&cfield(s->act)[seg], 1ull);
   const uint32_t tree = act_class(old);
-  if (tree >= s->num_trees) return;
+  if (tree >= cfield(s->num_trees)) return;
   const uint32_t nb = blocks_in_segment(s, tree);
-  if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&s->qc[seg]) != 0)
+  if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&cfield(s->qc)[seg]) != 0)
     release_segment(s, seg, tree, act_gen(old), nb);
 }
 
@@ -772,9 +902,9 @@ GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
 // word is stored, not yet published: whoever installs the block fences first.
 GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, bool &last) {
   last = false;
-  const unsigned long long seen = ld_rlx(&s->act[seg]);
+  const unsigned long long seen = ld_rlx(&cfield(s->act)[seg]);
   if (act_class(seen) != tree || act_count(seen) < 0) return NOBLK;  // another class's, or nothing left
-  const unsigned long long old = add_acquire(&s->act[seg], ~0ull);  // minus one
+  const unsigned long long old = add_acquire(&cfield(s->act)[seg], ~0ull);  // minus one
   if (act_count(old) < 0 || act_class(old) != tree) {
     // the last block went to another thread meanwhile, or the segment was
     // released and set up for another class
@@ -782,14 +912,14 @@ GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, 
     return NOBLK;
   }
   uint32_t nb = blocks_in_segment(s, tree);
-  uint32_t pos = atomicAdd(&s->qc[seg], 1u);
+  uint32_t pos = atomicAdd(&cfield(s->qc)[seg], 1u);
   uint32_t blk;
   if (pos < nb) {
-    blk = (uint32_t)(seg << s->bps_shift) + pos;
+    blk = (uint32_t)(seg << cfield(s->bps_shift)) + pos;
   } else {
-    uint32_t *e = s->queues + (seg << s->bps_shift) + (pos & (nb - 1u));
+    uint32_t *e = cfield(s->queues) + (seg << cfield(s->bps_shift)) + (pos & (nb - 1u));
     blk = atomicExch(e, NOBLK);
-    for (uint32_t i = 0; blk == NOBLK && i < s->spin_limit; i++) {  // a return still in flight
+    for (uint32_t i = 0; blk == NOBLK && i < cfield(s->spin_limit); i++) {  // a return still in flight
       backoff(i);
       blk = atomicExch(e, NOBLK);
     }
@@ -805,129 +935,166 @@ GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, 
 
 // Waits between attempts at a segment another thread is working on: a gather
 // takes a few microseconds, so the first waits are short; a wait that lasts
-// grows to backoff's.
-GAL_DEVICE_INLINE void backoff_gather(uint32_t i) { __nanosleep(i < 24 ? 100u : 4096u); }
+// grows to backoff's.  (Growing after 24 tries left the last of 152 threads
+// that asked one class together waiting up to 290 us.)
+GAL_DEVICE_INLINE void backoff_gather(uint32_t i) { __nanosleep(i < 64 ? 100u : i < 1024 ? 400u : 4096u); }
+
+// Threads that wait for the lock of class `tree` to gather a segment, counted
+// beside the lock, and the segments wanted for them besides the one that is
+// gathered anyway.  A thread that never waited leaves the count at 0.
+static constexpr uint32_t MORE_SEGMENTS = 7;
+GAL_DEVICE_INLINE uint32_t *waiters_of(const state *s, uint32_t tree) {
+  return cfield(s->locks) + tree * LOCK_STRIDE + 1;
+}
+GAL_DEVICE_INLINE uint32_t more_segments(const state *s, uint32_t tree, uint32_t waiting) {
+  return min(MORE_SEGMENTS, waiting / blocks_in_segment(s, tree));
+}
+
+// Takes a segment that has no block to give (or is another class's by now) off
+// its class's tree: by the thread that took its last block, or by any that
+// finds it listed meanwhile, so that nobody waits for the former.  Blocks may
+// have come home since, so the segment is listed again if it has one to give.
+// The release of a segment closes its count word before it unlists it, so a
+// listing made here and still valid when the word is read again is either right
+// or taken off by the release.  One thread alone never finds such a segment.
+GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
+  while (veb_remove(sub_tree(s, tree), seg)) {
+    unsigned long long w = ld_rlx(&cfield(s->act)[seg]);
+    if (act_class(w) != tree || act_count(w) < 0) return;
+    veb_insert(sub_tree(s, tree), seg);
+    fence_acq_rel();
+    w = ld_rlx(&cfield(s->act)[seg]);
+    if (act_class(w) == tree && act_count(w) >= 0) return;
+  }
+}
 
 // The rest of a block request that took the last block of a segment
-// (gallatin.cuh:1598-1612): the segment leaves its class's tree and, with
-// gather_ahead, the class's next segment is gathered.  Split from
+// (gallatin.cuh:1598-1612): with gather_ahead the class's next segment is
+// gathered, and the emptied one leaves its class's tree.  Split from
 // request_block so that a claim's block can be installed first: the teams
 // waiting for it do not wait for the gather, and one thread alone leaves the
-// same state either way.  Blocks may have come home between the hand-out and
-// the removal here, so the segment is listed again if it has one to give; the
-// release of a segment closes its count word before it unlists it, so a
-// listing made here and still valid when the word is read again is either
-// right or taken off by the release.
+// same state either way.  The next segment is listed before the emptied one is
+// taken off, so the class's word does not empty and its summaries stay as they
+// are.
 // Only one thread of a class gathers ahead at a time, whatever its lock policy
 // (alone, a thread always finds the lock free): each would add a segment to a
 // class that needs one, and threads that take a class's last blocks together
 // would leave it holding hundreds.
 static constexpr uint32_t NOSEG = 0xFFFFFFFFu;
-GAL_DEVICE_COLD void finish_last_block(const state *s, uint32_t tree, uint32_t seg, bool listed) {
-  if (listed) {
-    veb_remove(sub_tree(s, tree), seg);
-    for (;;) {
-      fence_acq_rel();
-      unsigned long long w = ld_rlx(&s->act[seg]);
-      if (act_class(w) != tree || act_count(w) < 0) break;
-      veb_insert(sub_tree(s, tree), seg);
-      fence_acq_rel();
-      w = ld_rlx(&s->act[seg]);
-      if (act_class(w) == tree && act_count(w) >= 0) break;
-      veb_remove(sub_tree(s, tree), seg);
+static constexpr uint32_t SEG_UNLISTED = 0x80000000u;  // with a segment: it was never listed
+GAL_DEVICE_COLD void finish_emptied(const state *s, uint32_t tree, uint32_t emptied) {
+  if (cfield(s->gather_ahead)) {
+    const veb_low l = free_segments_low(s);
+    const uint32_t waiting = ld_rlx(waiters_of(s, tree));
+    if (try_lock(s, tree)) {
+      gather_new_segment(s, tree, false, l, more_segments(s, tree, waiting));
+      unlock(s, tree);
     }
   }
-  if (s->gather_ahead && try_lock(s, tree)) {
-    gather_new_segment(s, tree, false);
-    unlock(s, tree);
-  }
+  if (!(emptied & SEG_UNLISTED)) unlist_refusing(s, tree, emptied);
+}
+// The steps of a block request are functions of their own with few arguments:
+// what a caller keeps across a call stays in registers at every level of the
+// chain, and the chain's depth is what a kernel that calls malloc is compiled
+// for (as one function with its helpers inlined: 26 more registers).
+// A listed segment of the class (FAIL: none); after a wait any of them.
+GAL_DEVICE_COLD uint64_t find_segment(const state *s, uint32_t tree, uint32_t tid, uint32_t waited) {
+  const veb_ref sub = sub_tree(s, tree);
+  if (cfield(s->policy) == GAL_POLICY_LOWEST) return veb_find_first(sub);
+  if (waited) return veb_find_any(sub, (tid + waited) * 0x9E3779B1u >> 8);
+  return veb_find_random(sub, tid);
+}
+// A new segment for a request that found none listed (first block taken);
+// -1: none is free, -2: another thread of the class is gathering one.
+// Classes with few blocks per segment need a segment per few requests: the
+// class lock only serialises them (serially the lock is always free).
+GAL_DEVICE_COLD int64_t gather_on_demand(const state *s, uint32_t tree) {
+  const veb_low l = free_segments_low(s);
+  if (blocks_in_segment(s, tree) < cfield(s->gather_unlocked_below)) return gather_new_segment(s, tree, true, l);
+  const uint32_t waiting = ld_rlx(waiters_of(s, tree));
+  if (ld_rlx(cfield(s->locks) + tree * LOCK_STRIDE) != 0u || !try_lock(s, tree)) return -2;
+  const int64_t got = gather_new_segment(s, tree, true, l, more_segments(s, tree, waiting));
+  unlock(s, tree);
+  return got;
 }
 
-// Gallatin::request_new_block_from_tree (gallatin.cuh:1525-1631).  `emptied`
-// receives the segment whose last block this was (bit 31: it was never
-// listed), for request_done, else NOSEG.
-static constexpr uint32_t SEG_UNLISTED = 0x80000000u;
-GAL_DEVICE_COLD uint32_t request_block_begin(const state *s, uint32_t tree, uint64_t tid, uint32_t &emptied) {
-  uint32_t spins = 0;
-  int gather_fails = 0;
-  emptied = NOSEG;
+// Gallatin::request_new_block_from_tree (gallatin.cuh:1525-1631): the block in
+// the low half (NOBLK: none), and in the high half, for request_done, the
+// segment whose last block it was, else NOSEG.
+GAL_DEVICE_INLINE uint32_t requested_block(uint64_t r) { return (uint32_t)r; }
+GAL_DEVICE_COLD uint64_t request_block_begin(const state *s, uint32_t tree, uint32_t tid) {
+  uint32_t waited = 0, blk = NOBLK, emptied = NOSEG;
+  uint32_t gather_fails = 0, counted = 0;  // counted: among the waiters
   for (;;) {
-    veb_ref sub = sub_tree(s, tree);
-    uint64_t seg = s->policy == GAL_POLICY_LOWEST ? veb_find_first(sub) : veb_find_random(sub, tid);
-    // classes with few blocks per segment need a segment per few requests:
-    // the class lock only serialises them (serially the lock is always free)
+    const uint64_t seg = find_segment(s, tree, tid, waited);
     if (seg == FAIL) {
-      const bool unlocked = blocks_in_segment(s, tree) < s->gather_unlocked_below;
-      if (unlocked || try_lock(s, tree)) {
-        int64_t got = gather_new_segment(s, tree, true);
-        if (!unlocked) unlock(s, tree);
-        if (got < 0) {
-          // segment tree empty: nothing a retry by this thread alone changes
-          if (++gather_fails >= GATHER_RETRIES) return NOBLK;
-          backoff(gather_fails);
-          continue;
-        }
-        const uint32_t blk = (uint32_t)((uint64_t)got << s->bps_shift);
+      const int64_t got = gather_on_demand(s, tree);
+      if (got >= 0) {
+        blk = (uint32_t)got << cfield(s->bps_shift);
         st_rlx(mword_ptr(s, blk), (unsigned long long)tree << 32);
         if (blocks_in_segment(s, tree) == 1) emptied = (uint32_t)got | SEG_UNLISTED;
-        return blk;
+        break;
       }
-      if (++spins > s->spin_limit) {
-        set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_REQUEST_LOCK, tree, spins);
-        return NOBLK;
+      if (got == -1) {
+        // segment tree empty: nothing a retry by this thread alone changes
+        if (++gather_fails >= (uint32_t)GATHER_RETRIES) break;
+        backoff(gather_fails);
+        continue;
       }
-      backoff_gather(spins);
-      continue;
-    }
-    bool last = false;
-    uint32_t blk = get_block(s, seg, tree, last);
-    if (last) emptied = (uint32_t)seg;
-    if (blk != NOBLK) return blk;
-    if (last) {  // counted out, but its block never came: the segment is empty all the same
-      finish_last_block(s, tree, (uint32_t)seg, true);
+      if (!counted) atomicAdd(waiters_of(s, tree), 1u);
+      counted = 1;
+    } else {
+      bool last = false;
+      blk = get_block(s, seg, tree, last);
+      if (last) emptied = (uint32_t)seg;
+      if (blk != NOBLK) break;
+      if (last) finish_emptied(s, tree, (uint32_t)seg);  // counted out, but its block never came
+      else unlist_refusing(s, tree, seg);
       emptied = NOSEG;
     }
-    if (++spins > s->spin_limit) {
-      set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_REQUEST_RETRY, tree, seg);
-      return NOBLK;
+    if (++waited > cfield(s->spin_limit)) {
+      set_error_info(s, GAL_DEV_ERR_TIMEOUT, seg == FAIL ? SITE_REQUEST_LOCK : SITE_REQUEST_RETRY, tree,
+                     seg == FAIL ? (uint64_t)waited : seg);
+      break;
     }
-    backoff_gather(spins);
+    backoff_gather(waited);
   }
+  if (counted) atomicSub(waiters_of(s, tree), 1u);
+  return ((uint64_t)emptied << 32) | blk;
 }
-GAL_DEVICE_INLINE void request_done(const state *s, uint32_t tree, uint32_t emptied) {
-  if (emptied != NOSEG) finish_last_block(s, tree, emptied & ~SEG_UNLISTED, !(emptied & SEG_UNLISTED));
+GAL_DEVICE_INLINE void request_done(const state *s, uint32_t tree, uint64_t r) {
+  if ((uint32_t)(r >> 32) != NOSEG) finish_emptied(s, tree, (uint32_t)(r >> 32));
 }
-GAL_DEVICE_INLINE uint32_t request_block(const state *s, uint32_t tree, uint64_t tid) {
-  uint32_t emptied;
-  const uint32_t blk = request_block_begin(s, tree, tid, emptied);
-  request_done(s, tree, emptied);
-  return blk;
+GAL_DEVICE_INLINE uint32_t request_block(const state *s, uint32_t tree, uint32_t tid) {
+  const uint64_t r = request_block_begin(s, tree, tid);
+  request_done(s, tree, r);
+  return requested_block(r);
 }
 
 // Gallatin::return_block (gallatin.cuh:1637-1726) with reserve_segment_slot,
 // finalize_free_queue and finish_freeing_block (memory_table.cuh:906-910,1158-1241)
 GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
-  uint64_t seg = blk >> s->bps_shift;
-  uint16_t tree = ld_rlx(&s->tree_ids[seg]);
-  if (tree >= s->num_trees) {
+  uint64_t seg = blk >> cfield(s->bps_shift);
+  uint16_t tree = ld_rlx(&cfield(s->tree_ids)[seg]);
+  if (tree >= cfield(s->num_trees)) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_RETURN_BAD_TREE, blk, tree);
     return;
   }
   uint32_t nb = blocks_in_segment(s, tree);
-  uint32_t pos = atomicAdd(&s->qfc[seg], 1u);
+  uint32_t pos = atomicAdd(&cfield(s->qfc)[seg], 1u);
   uint32_t live = pos & (nb - 1u);
-  st_rlx(s->queues + (seg << s->bps_shift) + live, blk);
+  st_rlx(cfield(s->queues) + (seg << cfield(s->bps_shift)) + live, blk);
   // The reference finalises returns in position order with a CAS spin
   // (memory_table.cuh:906-910) so a hand-out never meets an empty ring entry;
   // get_block here waits (bounded) for an entry still in flight instead, so a
   // return only counts itself, leaving the same counter value.
-  atomicAdd(&s->fqfc[seg], 1u);
+  atomicAdd(&cfield(s->fqfc)[seg], 1u);
   // re-register at the 10% crossing (gallatin.cuh:1646): live/nb >= 0.1 and
   // (live-1)/nb < 0.1 in doubles; for the power-of-two nb used here that is
   // 10*live > nb >= 10*(live-1) with live-1 taken as unsigned (live 0 never).
   if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) veb_insert(sub_tree(s, tree), seg);
   fence_acq_rel();  // the ring entry before the count that lets it be handed out
-  const unsigned long long old = add_acquire(&s->act[seg], 1ull);
+  const unsigned long long old = add_acquire(&cfield(s->act)[seg], 1ull);
   if ((uint32_t)(act_count(old) + 2) == nb)  // all_blocks_free: the count was nb - 2
     release_segment(s, seg, tree, act_gen(old), nb);
 }
@@ -973,9 +1140,9 @@ GAL_DEVICE_INLINE void free_block_slices(const state *s, uint32_t blk) {
 // Returns the slot index; `blk` receives the block read from it (one read per
 // probed slot, the last one doubling as the reference's get_my_block read).
 GAL_DEVICE_INLINE uint32_t pick_slot(const state *s, uint32_t tree, uint32_t &blk) {
-  const uint32_t n = s->slot_count[tree];
-  const uint32_t *slots = s->slots + s->slot_base[tree];
-  uint32_t smid = s->smid_override >= 0 ? (uint32_t)s->smid_override : sm_id();
+  const uint32_t n = cfield(s->slot_count[tree]);
+  const uint32_t *slots = cfield(s->slots) + cfield(s->slot_base[tree]);
+  uint32_t smid = cfield(s->smid_override) >= 0 ? (uint32_t)cfield(s->smid_override) : sm_id();
   int my = (int)(smid % n);
   int original = my;
   int counter = 0;
@@ -989,24 +1156,27 @@ GAL_DEVICE_INLINE uint32_t pick_slot(const state *s, uint32_t tree, uint32_t &bl
   return (uint32_t)my;
 }
 
-// Gallatin::replace_block (gallatin.cuh:1083-1138)
-GAL_DEVICE_COLD bool replace_block(const state *s, uint32_t tree, uint32_t slot, uint32_t blk,
-                                   uint64_t tid) {
-  uint32_t *sp = s->slots + s->slot_base[tree] + slot;
-  if (atomicCAS(sp, blk, NOBLK) != blk) return true;
-  uint32_t emptied;
-  uint32_t nb = request_block_begin(s, tree, tid, emptied);
+// Requests a block for the empty slot or spare word `at`.
+GAL_DEVICE_COLD bool request_into(const state *s, uint32_t tree, uint32_t *at, uint32_t tid, bool slot) {
+  const uint64_t r = request_block_begin(s, tree, tid);
   bool ok = false;
-  if (nb != NOBLK) {
+  if (requested_block(r) != NOBLK) {
     fence_acq_rel();
-    ok = atomicCAS(sp, NOBLK, nb) == NOBLK;
+    ok = atomicCAS(at, NOBLK, requested_block(r)) == NOBLK;
     if (!ok) {
-      set_error(s, GAL_DEV_ERR_SLOT_SWAP);
-      retire_block(s, nb);  // hand the block back
+      if (slot) set_error(s, GAL_DEV_ERR_SLOT_SWAP);
+      retire_block(s, requested_block(r));  // hand the block back
     }
   }
-  request_done(s, tree, emptied);  // after the waiting teams have their block
+  request_done(s, tree, r);  // after the waiting teams have their block
   return ok;
+}
+
+// Gallatin::replace_block (gallatin.cuh:1083-1138)
+GAL_DEVICE_INLINE bool replace_block(const state *s, uint32_t tree, uint32_t slot, uint32_t blk, uint32_t tid) {
+  uint32_t *sp = cfield(s->slots) + cfield(s->slot_base[tree]) + slot;
+  if (atomicCAS(sp, blk, NOBLK) != blk) return true;
+  return request_into(s, tree, sp, tid, true);
 }
 
 // Spare blocks (gal_config.spare_blocks): the slot's prepared next block is
@@ -1014,44 +1184,37 @@ GAL_DEVICE_COLD bool replace_block(const state *s, uint32_t tree, uint32_t slot,
 // an empty slot for the length of a segment search; the search then refills
 // the spare.  swap_spare returns whether the caller should refill (it falls
 // back to replace_block when no spare was ready).
-GAL_DEVICE_COLD bool swap_spare(const state *s, uint32_t tree, uint32_t slot, uint32_t blk, uint64_t tid) {
-  const uint32_t si = s->slot_base[tree] + slot;
-  const uint32_t nx = atomicExch(s->spares + si, NOBLK);
+GAL_DEVICE_INLINE bool swap_spare(const state *s, uint32_t tree, uint32_t slot, uint32_t blk, uint32_t tid) {
+  const uint32_t si = cfield(s->slot_base[tree]) + slot;
+  const uint32_t nx = atomicExch(cfield(s->spares) + si, NOBLK);
   if (nx == NOBLK) {
     replace_block(s, tree, slot, blk, tid);
-  } else if (atomicCAS(s->slots + si, blk, nx) != blk) {
+  } else if (atomicCAS(cfield(s->slots) + si, blk, nx) != blk) {
     retire_block(s, nx);  // the slot moved on: give the spare back
     return false;
   }
   return true;
 }
-GAL_DEVICE_COLD void refill_spare(const state *s, uint32_t tree, uint32_t slot, uint64_t tid) {
-  const uint32_t si = s->slot_base[tree] + slot;
-  if (ld_rlx(s->spares + si) != NOBLK) return;
-  uint32_t emptied;
-  const uint32_t nb = request_block_begin(s, tree, tid, emptied);
-  if (nb != NOBLK) {
-    fence_acq_rel();
-    if (atomicCAS(s->spares + si, NOBLK, nb) != NOBLK) retire_block(s, nb);
-  }
-  request_done(s, tree, emptied);
+GAL_DEVICE_INLINE void refill_spare(const state *s, uint32_t tree, uint32_t slot, uint32_t tid) {
+  uint32_t *at = cfield(s->spares) + cfield(s->slot_base[tree]) + slot;
+  if (ld_rlx(at) == NOBLK) request_into(s, tree, at, tid, false);
 }
 
 // Gallatin::boot_block (gallatin.cuh:726-787)
-GAL_DEVICE_COLD bool boot_block(const state *s, uint32_t tree, uint32_t slot, uint64_t tid) {
-  if (slot >= s->slot_count[tree]) return false;
+GAL_DEVICE_COLD bool boot_block(const state *s, uint32_t tree, uint32_t slot, uint32_t tid) {
+  if (slot >= cfield(s->slot_count[tree])) return false;
   uint32_t blk = request_block(s, tree, tid);
   if (blk == NOBLK) return false;
-  if (ld_rlx(&s->tree_ids[blk >> s->bps_shift]) != tree) return false;
+  if (ld_rlx(&cfield(s->tree_ids)[blk >> cfield(s->bps_shift)]) != tree) return false;
   fence_acq_rel();
-  return atomicCAS(s->slots + s->slot_base[tree] + slot, NOBLK, blk) == NOBLK;
+  return atomicCAS(cfield(s->slots) + cfield(s->slot_base[tree]) + slot, NOBLK, blk) == NOBLK;
 }
 
 // ------------------------------------------------------------------ addresses
 GAL_DEVICE_INLINE char *slice_ptr(const state *s, uint32_t blk, uint64_t idx, uint32_t tree) {
-  uint64_t seg = blk >> s->bps_shift;
-  uint64_t q = blk & ((1u << s->bps_shift) - 1u);
-  return s->memory + (seg << s->seg_shift) + (((q << 12) + idx) << (s->min_shift + tree));
+  uint64_t seg = blk >> cfield(s->bps_shift);
+  uint64_t q = blk & ((1u << cfield(s->bps_shift)) - 1u);
+  return cfield(s->memory) + (seg << cfield(s->seg_shift)) + (((q << 12) + idx) << (cfield(s->min_shift) + tree));
 }
 
 // ------------------------------------------------------------------ malloc tiers
@@ -1085,14 +1248,16 @@ GAL_DEVICE_INLINE void slot_cache_init(slot_cache &c) {
 // The rare part of a claim, out of line so the claim's common path keeps few
 // values live across calls: credits the slices this lane gives back and, for
 // the team's leader when the block must be replaced, swaps in the slot's spare
-// (or replaces the block).  Returns whether the spare wants a refill.
-GAL_DEVICE_COLD bool claim_slow_path(const state *s, uint32_t tree, uint32_t slot, uint32_t blk, uint32_t credit,
-                                     bool lead, uint64_t tid) {
+// (or replaces the block).  Returns the slot when its spare wants a refill,
+// else NOBLK.
+GAL_DEVICE_COLD uint32_t claim_slow_path(const state *s, uint32_t tree, uint32_t slot, uint32_t blk, uint32_t credit,
+                                         bool lead) {
   if (credit) credit_frees(s, blk, credit);
-  if (!lead) return false;
-  if (s->use_spares) return swap_spare(s, tree, slot, blk, tid);
+  if (!lead) return NOBLK;
+  const uint32_t tid = (uint32_t)thread_linear_id();
+  if (cfield(s->use_spares)) return swap_spare(s, tree, slot, blk, tid) ? slot : NOBLK;
   replace_block(s, tree, slot, blk, tid);
-  return false;
+  return NOBLK;
 }
 
 // A block is exhausted by exactly one claim -- the one that crosses slice
@@ -1113,12 +1278,21 @@ GAL_DEVICE_COLD bool claim_slow_path(const state *s, uint32_t tree, uint32_t slo
 // meets an exhausted block in its slot, so serial offsets are unchanged.
 static constexpr uint32_t STUCK_MARGIN = 1u << 12;
 static constexpr int STUCK_ATTEMPTS = 16;
+// What an attempt needs after a call off its common path.  Kept in memory across
+// the call (volatile), not in registers: the compiler stacks the registers of a
+// caller and of the whole chain it calls, so what is held here while a block is
+// requested would be held by every kernel that calls malloc.
+struct parked {
+  volatile uint64_t state, result;
+  volatile uint32_t tree, count, live;
+  volatile int attempt;
+};
 template <bool NAMED>
 GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t count, uint32_t pending,
                                       slot_cache *cache = nullptr) {
-  const uint32_t lane = lane_id();
-  const uint64_t tid = thread_linear_id();
+  parked keep;
   for (int attempt = 0; attempt < SLICE_ATTEMPTS; attempt++) {
+    const uint32_t lane = lane_id();
     const uint32_t active = NAMED ? pending : active_lanes();
     const uint32_t team = __match_any_sync(active, tree) & team_group(s);
     const int leader = __ffs(team) - 1;
@@ -1180,16 +1354,42 @@ GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t co
         if ((rep || exhausted || foreign) && (int)lane == leader) atomicCAS(&cache->blk[tree], blk, NOBLK);
       }
       if (exhausted && fresh && attempt >= STUCK_ATTEMPTS && (old & 0xFFFFFFFFull) >= SLICES_PER_BLOCK + STUCK_MARGIN &&
-          ld_rlx(s->slots + s->slot_base[tree] + slot) == blk)
+          ld_rlx(cfield(s->slots) + cfield(s->slot_base[tree]) + slot) == blk)
         rep = team;  // the slot has held an exhausted block for a while: replace it here
       const bool lead = rep && (int)lane == leader;
-      if (credit || lead) refill = claim_slow_path(s, tree, slot, blk, credit, lead, tid);
-      __syncwarp(live);
-      if (!NAMED && refill) refill_spare(s, tree, slot, tid);  // the team's other lanes go on
+      uint32_t group = live;
+      if (credit || lead) {
+        keep.state = (uint64_t)s;
+        keep.result = (uint64_t)result;
+        keep.tree = tree;
+        keep.count = count;
+        keep.live = live;
+        keep.attempt = attempt;
+        const uint32_t r = claim_slow_path(s, tree, slot, blk, credit, lead);
+        refill = r != NOBLK;
+        slot = r;
+        s = (const state *)keep.state;
+        result = (void *)keep.result;
+        tree = keep.tree;
+        count = keep.count;
+        group = keep.live;
+        attempt = keep.attempt;
+      }
+      __syncwarp(group);
     }
-    if (NAMED) {
-      pending = __ballot_sync(active, result == nullptr);
-      if (refill) refill_spare(s, tree, slot, tid);  // the team's other lanes go on
+    if (NAMED) pending = __ballot_sync(active, result == nullptr);
+    if (refill) {  // the team's other lanes go on
+      keep.state = (uint64_t)s;
+      keep.result = (uint64_t)result;
+      keep.tree = tree;
+      keep.count = count;
+      keep.attempt = attempt;
+      refill_spare(s, tree, slot, (uint32_t)thread_linear_id());
+      s = (const state *)keep.state;
+      result = (void *)keep.result;
+      tree = keep.tree;
+      count = keep.count;
+      attempt = keep.attempt;
     }
     if (result) return result;
   }
@@ -1197,22 +1397,26 @@ GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t co
 }
 
 // Gallatin::malloc_block_allocation (gallatin.cuh:828-861), Block::malloc_fill_block
-GAL_DEVICE_COLD void *malloc_whole_block(const state *s, uint32_t tree) {
-  const uint64_t tid = thread_linear_id();
-  for (int a = 0; a < BLOCK_ATTEMPTS; a++) {
-    uint32_t blk = request_block(s, tree, tid);
+GAL_DEVICE_INLINE void *malloc_whole_block(const state *s, uint32_t tree) {
+  volatile uint32_t kept = tree, attempts = BLOCK_ATTEMPTS;  // see `parked`
+  while (attempts) {
+    attempts = attempts - 1u;
+    const uint32_t blk = request_block(s, kept, (uint32_t)thread_linear_id());
     if (blk == NOBLK) return nullptr;
     unsigned long long old = atomicAdd(mword_ptr(s, blk), (unsigned long long)SLICES_PER_BLOCK);
     uint32_t old_count = (uint32_t)old;
-    if ((uint32_t)(old >> 32) != tree) set_error(s, GAL_DEV_ERR_BLOCK_TREE);
+    if ((uint32_t)(old >> 32) != kept) set_error(s, GAL_DEV_ERR_BLOCK_TREE);
     atomicAdd(fctr_ptr(s, blk), (SLICES_PER_BLOCK - 1) - old_count);
-    if (old_count != 0) {
-      credit_frees(s, blk, 1);
-      continue;
-    }
-    return slice_ptr(s, blk, 0, tree);
+    if (old_count == 0) return slice_ptr(s, blk, 0, kept);
+    credit_frees(s, blk, 1);
   }
   return nullptr;
+}
+
+// marks the run of `count` segments from idx, taken by this thread
+GAL_DEVICE_INLINE void own_run(const state *s, uint64_t idx, uint32_t count) {
+  if (ld_rlx(&cfield(s->tree_ids)[idx]) != FREE_TREE) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
+  else st_rlx(&cfield(s->tree_ids)[idx], (uint16_t)(cfield(s->num_trees) + 1 + count));
 }
 
 // Gallatin::malloc_segment_allocation (gallatin.cuh:790-826).  The reference
@@ -1222,16 +1426,15 @@ GAL_DEVICE_COLD void *malloc_whole_block(const state *s, uint32_t tree) {
 GAL_DEVICE_COLD void *malloc_segment_run(const state *s, uint32_t count) {
   for (int a = 0; a < SEGMENT_ATTEMPTS; a++) {
     uint32_t spins = 0;
-    while (!try_lock(s, s->num_trees)) {
+    while (!try_lock(s, cfield(s->num_trees))) {
       if (spins == 0 && count <= 64) {
         const uint64_t idx = veb_gather_in_word(seg_tree(s), count);
         if (idx != FAIL) {
-          if (cas16(&s->tree_ids[idx], FREE_TREE, (uint16_t)(s->num_trees + 1 + count)) != FREE_TREE)
-            set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
-          return s->memory + (idx << s->seg_shift);
+          own_run(s, idx, count);
+          return cfield(s->memory) + (idx << cfield(s->seg_shift));
         }
       }
-      if (++spins > s->spin_limit) {
+      if (++spins > cfield(s->spin_limit)) {
         set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_RUN_LOCK, count, spins);
         return nullptr;
       }
@@ -1239,12 +1442,11 @@ GAL_DEVICE_COLD void *malloc_segment_run(const state *s, uint32_t count) {
     }
     uint64_t idx = veb_gather_multiple(seg_tree(s), count);
     if (idx != FAIL) {
-      if (cas16(&s->tree_ids[idx], FREE_TREE, (uint16_t)(s->num_trees + 1 + count)) != FREE_TREE)
-        set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
-      unlock(s, s->num_trees);
-      return s->memory + (idx << s->seg_shift);
+      own_run(s, idx, count);
+      unlock(s, cfield(s->num_trees));
+      return cfield(s->memory) + (idx << cfield(s->seg_shift));
     }
-    unlock(s, s->num_trees);
+    unlock(s, cfield(s->num_trees));
   }
   return nullptr;
 }
@@ -1259,14 +1461,14 @@ GAL_DEVICE_COLD void zero_fill(void *p, uint64_t size) {
   for (uint64_t i = 0; i < n; i++) q[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 GAL_DEVICE_INLINE void *handed_out(const state *s, void *p, uint64_t size) {
-  if (p && s->zero_fill) zero_fill(p, size);
+  if (p && cfield(s->zero_fill)) zero_fill(p, size);
   return p;
 }
 
 // the block and segment tiers of Gallatin::malloc (gallatin.cuh:1203-1258)
 GAL_DEVICE_COLD void *malloc_large(const state *s, uint64_t size, int block_tree) {
-  if (block_tree < (int)s->num_trees) return malloc_whole_block(s, (uint32_t)block_tree);
-  return malloc_segment_run(s, (uint32_t)((size - 1) >> s->seg_shift) + 1);
+  if (block_tree < (int)cfield(s->num_trees)) return malloc_whole_block(s, (uint32_t)block_tree);
+  return malloc_segment_run(s, (uint32_t)((size - 1) >> cfield(s->seg_shift)) + 1);
 }
 
 // Gallatin::malloc (gallatin.cuh:1186-1276) called by the lanes in `callers`
@@ -1275,13 +1477,17 @@ GAL_DEVICE_COLD void *malloc_large(const state *s, uint64_t size, int block_tree
 // of the same class share a team.
 template <bool NAMED>
 GAL_DEVICE_INLINE void *malloc_from(const state *s, uint64_t size, uint32_t callers, slot_cache *cache = nullptr) {
-  const int T = (int)s->num_trees;
+  const int T = (int)cfield(s->num_trees);
   const int bits = ceil_log2(size);
-  const int t = (size >> s->min_shift) == 0 ? 0 : bits - (int)s->min_shift;
-  const int block_tree = bits - (int)(s->min_shift + 12);
+  const int t = (size >> cfield(s->min_shift)) == 0 ? 0 : bits - (int)cfield(s->min_shift);
+  const int block_tree = bits - (int)(cfield(s->min_shift) + 12);
   const bool slices = t < T || block_tree < 0;
   const uint32_t members = __ballot_sync(callers, slices);
-  if (!slices) return handed_out(s, malloc_large(s, size, block_tree), size);
+  if (!slices) {
+    const volatile uint64_t kept = size;  // see `parked`
+    void *p = malloc_large(s, size, block_tree);
+    return handed_out(s, p, kept);
+  }
   // big slices (4 KiB < size <= 32 KiB by default): runs of the last class
   const bool big = t >= T;
   const uint32_t count = 1u << (big ? t - (T - 1) : 0);
@@ -1314,8 +1520,8 @@ GAL_DEVICE_INLINE void *malloc_team(const state *s, uint64_t size, uint32_t call
 
 // multi-segment free (gallatin.cuh:1394-1417, 1283-1302), id reset first
 GAL_DEVICE_COLD void free_segment_run(const state *s, uint64_t seg, uint16_t tree) {
-  uint32_t count = (uint32_t)tree - s->num_trees - 1;
-  if (cas16(&s->tree_ids[seg], tree, FREE_TREE) != tree) {
+  uint32_t count = (uint32_t)tree - cfield(s->num_trees) - 1;
+  if (cas16(&cfield(s->tree_ids)[seg], tree, FREE_TREE) != tree) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_RUN_TWICE, seg, tree);
     return;
   }
@@ -1325,35 +1531,35 @@ GAL_DEVICE_COLD void free_segment_run(const state *s, uint64_t seg, uint16_t tre
 
 // Gallatin::free (gallatin.cuh:1378-1461)
 GAL_DEVICE_INLINE void free(const state *s, void *ptr) {
-  uint64_t off = (uint64_t)((char *)ptr - s->memory);
-  uint64_t seg = off >> s->seg_shift;
-  if (seg >= s->num_segments) {
+  uint64_t off = (uint64_t)((char *)ptr - cfield(s->memory));
+  uint64_t seg = off >> cfield(s->seg_shift);
+  if (seg >= cfield(s->num_segments)) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OUTSIDE, off, 0);
     return;
   }
-  uint16_t tree = ld_rlx(&s->tree_ids[seg]);
-  if (tree >= s->num_trees) {
-    if (tree == FREE_TREE || tree == s->num_trees) {
+  uint16_t tree = ld_rlx(&cfield(s->tree_ids)[seg]);
+  if (tree >= cfield(s->num_trees)) {
+    if (tree == FREE_TREE || tree == cfield(s->num_trees)) {
       set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_FREE_SEGMENT, off, tree);
       return;
     }
     free_segment_run(s, seg, tree);
     return;
   }
-  uint64_t in_seg = off & ((1ull << s->seg_shift) - 1ull);
-  uint32_t blk = (uint32_t)(seg << s->bps_shift) + (uint32_t)(in_seg >> (s->min_shift + tree + 12));
+  uint64_t in_seg = off & ((1ull << cfield(s->seg_shift)) - 1ull);
+  uint32_t blk = (uint32_t)(seg << cfield(s->bps_shift)) + (uint32_t)(in_seg >> (cfield(s->min_shift) + tree + 12));
   free_block_slices(s, blk);
 }
 
 // block id of a live pointer (slice or whole block), NOBLK for a segment run
 GAL_DEVICE_INLINE uint32_t block_of(const state *s, const void *ptr, uint16_t &tree_out) {
-  uint64_t off = (uint64_t)((const char *)ptr - s->memory);
-  uint64_t seg = off >> s->seg_shift;
-  uint16_t tree = seg < s->num_segments ? ld_rlx(&s->tree_ids[seg]) : FREE_TREE;
+  uint64_t off = (uint64_t)((const char *)ptr - cfield(s->memory));
+  uint64_t seg = off >> cfield(s->seg_shift);
+  uint16_t tree = seg < cfield(s->num_segments) ? ld_rlx(&cfield(s->tree_ids)[seg]) : FREE_TREE;
   tree_out = tree;
-  if (tree >= s->num_trees) return NOBLK;
-  uint64_t in_seg = off & ((1ull << s->seg_shift) - 1ull);
-  return (uint32_t)(seg << s->bps_shift) + (uint32_t)(in_seg >> (s->min_shift + tree + 12));
+  if (tree >= cfield(s->num_trees)) return NOBLK;
+  uint64_t in_seg = off & ((1ull << cfield(s->seg_shift)) - 1ull);
+  return (uint32_t)(seg << cfield(s->bps_shift)) + (uint32_t)(in_seg >> (cfield(s->min_shift) + tree + 12));
 }
 
 // Frees the pointers p[k] with go[k] set, as N calls of free() would, but
@@ -1370,9 +1576,9 @@ GAL_DEVICE_INLINE void free_n(const state *s, void *const (&p)[N], const bool (&
 #pragma unroll
   for (int k = 0; k < N; k++) {
     tree[k] = FREE_TREE;
-    off[k] = go[k] ? (uint64_t)((char *)p[k] - s->memory) : 0;
-    if (go[k] && (off[k] >> s->seg_shift) < s->num_segments)
-      tree[k] = classes ? classes[off[k] >> s->seg_shift] : ld_rlx(&s->tree_ids[off[k] >> s->seg_shift]);
+    off[k] = go[k] ? (uint64_t)((char *)p[k] - cfield(s->memory)) : 0;
+    if (go[k] && (off[k] >> cfield(s->seg_shift)) < cfield(s->num_segments))
+      tree[k] = classes ? classes[off[k] >> cfield(s->seg_shift)] : ld_rlx(&cfield(s->tree_ids)[off[k] >> cfield(s->seg_shift)]);
   }
   uint32_t blk[N], old[N], cnt[N];
   bool lead[N];
@@ -1381,13 +1587,13 @@ GAL_DEVICE_INLINE void free_n(const state *s, void *const (&p)[N], const bool (&
     lead[k] = false;
     blk[k] = NOBLK;
     if (!go[k]) continue;
-    if (tree[k] >= s->num_trees) {  // segment runs and bad pointers: the scalar path
+    if (tree[k] >= cfield(s->num_trees)) {  // segment runs and bad pointers: the scalar path
       gal::free(s, p[k]);
       continue;
     }
-    uint64_t in_seg = off[k] & ((1ull << s->seg_shift) - 1ull);
-    blk[k] = (uint32_t)((off[k] >> s->seg_shift) << s->bps_shift) +
-             (uint32_t)(in_seg >> (s->min_shift + tree[k] + 12));
+    uint64_t in_seg = off[k] & ((1ull << cfield(s->seg_shift)) - 1ull);
+    blk[k] = (uint32_t)((off[k] >> cfield(s->seg_shift)) << cfield(s->bps_shift)) +
+             (uint32_t)(in_seg >> (cfield(s->min_shift) + tree[k] + 12));
   }
 #pragma unroll
   for (int k = 0; k < N; k++) {
@@ -1408,8 +1614,8 @@ GAL_DEVICE_INLINE void free_n(const state *s, void *const (&p)[N], const bool (&
 // __syncthreads().  Returns false (nothing staged) for larger arenas.
 static constexpr uint32_t CLASS_STAGE_BYTES = 32768;
 GAL_DEVICE_INLINE bool stage_classes(const state *s, uint16_t *smem) {
-  if (s->num_segments * 2 > CLASS_STAGE_BYTES) return false;
-  for (uint64_t g = threadIdx.x; g < s->num_segments; g += blockDim.x) smem[g] = ld_rlx(&s->tree_ids[g]);
+  if (cfield(s->num_segments) * 2 > CLASS_STAGE_BYTES) return false;
+  for (uint64_t g = threadIdx.x; g < cfield(s->num_segments); g += blockDim.x) smem[g] = ld_rlx(&cfield(s->tree_ids)[g]);
   return true;
 }
 
@@ -1423,16 +1629,16 @@ GAL_DEVICE_INLINE uint32_t export_mword(const state *s, uint32_t blk) {
 GAL_DEVICE_INLINE uint64_t allocated_size(const state *s, uint64_t size) {
   if (size < 16) size = 16;
   int bits = ceil_log2(size);
-  int tree = bits - (int)s->min_shift;
-  if (tree > (int)s->num_trees) {
-    int block_tree = bits - (int)(s->min_shift + 12);
-    if (block_tree > (int)s->num_trees) return (((size - 1) >> s->seg_shift) + 1) << s->seg_shift;
+  int tree = bits - (int)cfield(s->min_shift);
+  if (tree > (int)cfield(s->num_trees)) {
+    int block_tree = bits - (int)(cfield(s->min_shift) + 12);
+    if (block_tree > (int)cfield(s->num_trees)) return (((size - 1) >> cfield(s->seg_shift)) + 1) << cfield(s->seg_shift);
   }
   return 1ull << bits;
 }
 
 GAL_DEVICE_INLINE bool owns(const state *s, const void *p) {
-  return (uint64_t)((const char *)p - s->memory) < (s->num_segments << s->seg_shift);
+  return (uint64_t)((const char *)p - cfield(s->memory)) < (cfield(s->num_segments) << cfield(s->seg_shift));
 }
 
 }  // namespace gal
