@@ -21,6 +21,7 @@ HEADERS = [
     os.path.join(ROOT, "include", "gallatin_gb300", "gal_device.cuh"),
     os.path.join(CSRC, "gal_batch.cuh"),
     os.path.join(CSRC, "gal_boot.cuh"),
+    os.path.join(CSRC, "gal_bulk.cuh"),
     os.path.join(CSRC, "churn.cuh"),
     os.path.join(CSRC, "workload.cuh"),
     os.path.join(CSRC, "gal_internal.h"),

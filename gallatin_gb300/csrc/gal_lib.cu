@@ -15,6 +15,7 @@
 #include "../../include/gallatin_gb300/gal_device.cuh"
 #include "gal_batch.cuh"
 #include "gal_boot.cuh"
+#include "gal_bulk.cuh"
 #include "gal_internal.h"
 
 struct gal_handle {
@@ -30,6 +31,7 @@ struct gal_handle {
   uint64_t arena_bytes = 0;
   gal_state_dims dims{};
   int grid_free = 0;  // persistent grid of the batched free kernel (0: not yet known)
+  int sms = 1;        // SMs of the device
 };
 
 namespace {
@@ -242,12 +244,9 @@ __global__ void k_free_per_thread(const gal::state *s, void *const *ptrs, uint64
 
 constexpr int BATCH_THREADS = 512;
 
-// Batched malloc: one thread per request, warp teams claiming with one
-// atomicAdd per team on their SM's pinned block (gal::malloc), compiled for
-// four CTAs of 256 threads per SM (64 registers).  On the mixed 16 B-4 KiB
-// churn's requests this served 64 Mi mallocs in 2.2 ms per step, against
-// 2.6 ms for the same kernel without a register bound and for a persistent
-// grid keeping the pinned blocks in shared memory (gal::malloc_cached).
+// Batched malloc of short lists: one thread per request, warp teams claiming
+// with one atomicAdd per team on their SM's pinned block (gal::malloc), compiled
+// for four CTAs of 256 threads per SM (64 registers).
 constexpr int MALLOC_THREADS = 256;
 
 __global__ void __launch_bounds__(MALLOC_THREADS, 4)
@@ -255,6 +254,21 @@ __global__ void __launch_bounds__(MALLOC_THREADS, 4)
   for (uint64_t i = (uint64_t)blockIdx.x * MALLOC_THREADS + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * MALLOC_THREADS)
     out[i] = gal::malloc(s, sizes[i]);
+}
+
+// Longer lists: chunks of K x 512 requests, one claim per class and chunk
+// (gal_bulk.cuh).  Below BULK_FROM requests the barriers of a chunk cost as much
+// as the claims they save (4,096 mixed: 2 us more than one request per thread;
+// 30,000: 19 against 17 us; 100,003: 25 against 27; 1 Mi x 256 B: 62 against
+// 253; 4 Mi mixed, one slot per SM: 67 against 98).  K is the smallest that fits
+// the list in one wave of two CTAs per SM: larger chunks claim less often,
+// smaller ones start more SMs (262,144 mixed: 17, 11, 11, 21 us at K = 1, 2, 4, 8).
+constexpr uint64_t BULK_FROM = 1u << 15;
+template <int K>
+__global__ void __launch_bounds__(gal::BULK_THREADS, 2)
+    k_malloc_bulk(const gal::state *s, const uint64_t *sizes, uint64_t n, void **out) {
+  __shared__ gal::bulk_smem sm;
+  gal::bulk_malloc<K>(s, sizes, n, (uint64_t)blockIdx.x * (K * gal::BULK_THREADS), out, sm);
 }
 
 // Batched free: each thread takes FREE_PER_THREAD entries per pass of a
@@ -370,6 +384,8 @@ int build(uint64_t num_bytes, uint64_t seed, const gal_config *cfg_in, bool boot
   h->num_bytes = num_bytes;
   h->seed = seed;
   cudaGetDevice(&h->device);
+  cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device);
+  if (h->sms < 1) h->sms = 1;
   gal::state &st = h->st;
   st.num_segments = S;
   st.seed = seed;
@@ -388,9 +404,7 @@ int build(uint64_t num_bytes, uint64_t seed, const gal_config *cfg_in, bool boot
   // pinned slots: first, halving per tree, floored (shared_block_storage.cuh:260-267);
   // pinned_slots_first == 0 asks for one slot per SM in every size class
   if (cfg.pinned_slots_first == 0) {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device);
-    cfg.pinned_slots_first = cfg.pinned_slots_min = (uint32_t)(sms > 0 ? sms : 1);
+    cfg.pinned_slots_first = cfg.pinned_slots_min = (uint32_t)h->sms;
     h->cfg = cfg;
   }
   uint64_t n = cfg.pinned_slots_first, total = 0;
@@ -852,8 +866,19 @@ int gal_malloc_batched(gal_handle *h, const uint64_t *sizes, uint64_t n, void **
   if (!n) return GAL_OK;
   gal_device_guard on_dev(h->device);
   CUDA_TRY(on_dev.err);
-  k_malloc_batched<<<grid_for(n, MALLOC_THREADS), MALLOC_THREADS, 0, (cudaStream_t)stream>>>(h->d_state, sizes,
-                                                                                          n, out);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (n < BULK_FROM) {
+    k_malloc_batched<<<grid_for(n, MALLOC_THREADS), MALLOC_THREADS, 0, st>>>(h->d_state, sizes, n, out);
+  } else {
+    auto bulk = [&](auto kern, int k) {
+      kern<<<grid_for(n, gal::BULK_THREADS * k), gal::BULK_THREADS, 0, st>>>(h->d_state, sizes, n, out);
+    };
+    const uint64_t wave = 2ull * (uint64_t)h->sms * gal::BULK_THREADS;  // requests one wave serves, one per thread
+    if (n <= wave) bulk(k_malloc_bulk<1>, 1);
+    else if (n <= 2 * wave) bulk(k_malloc_bulk<2>, 2);
+    else if (n <= 4 * wave) bulk(k_malloc_bulk<4>, 4);
+    else bulk(k_malloc_bulk<8>, 8);
+  }
   CUDA_TRY(cudaGetLastError());
   return GAL_OK;
 }

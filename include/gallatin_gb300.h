@@ -326,9 +326,10 @@ int gal_free_per_thread(gal_handle *h, void *const *ptrs, uint64_t n, void *stre
 int gal_trim(gal_handle *h, void *stream);
 
 /* Batched form: the same results contract as gal_malloc_per_thread /
- * gal_free_per_thread.  Mallocs run one request per thread in a kernel
- * compiled for four CTAs of 256 threads per SM, warp teams claiming with one
- * atomicAdd per team; frees take four entries per thread on a persistent
+ * gal_free_per_thread.  Mallocs of 32 Ki requests or more run in chunks, a
+ * CTA ranking its requests per size class and claiming the slices of each with
+ * one atomicAdd; shorter lists one request per thread, warp teams claiming with
+ * one atomicAdd per team.  Frees take four entries per thread on a persistent
  * grid, look the segment classes up in a copy staged in shared memory, and
  * form warp teams per block (one free-counter atomic per team). */
 int gal_malloc_batched(gal_handle *h, const uint64_t *sizes, uint64_t n,
