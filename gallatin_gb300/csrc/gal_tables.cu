@@ -5,24 +5,38 @@
 //
 // Table t holds n_t pairs of 64-bit keys and values.  Its bucket array (one
 // 64-bit head word per bucket, bit 0 the bucket's lock) and every 128-byte
-// node come from the allocator.  A node: next pointer, a 7-bit used mask and
-// seven key/value pairs (8 + 8 + 7 x 16 = 128 B, the 128 B class).
+// node come from the allocator.  A node: next pointer, a 7-bit used mask, one
+// tag byte (eight hash bits) and a key/value pair for each of seven places
+// (8 + 1 + 7 + 7 x 16 = 128 B, the 128 B class).
 //
-// Phases, each one launch over all tables (ops flattened, table by binary
-// search over the offsets held in shared memory):
+// Phases, each a kernel of its own over all tables (ops flattened, table by
+// binary search over the offsets held in shared memory):
 //   insert every key; delete the keys whose coin is set (a node left empty is
 //   unlinked and freed); look up every key (deleted ones must be absent);
 //   reinsert the deleted keys; look up every key (all present, right value);
 //   count the live pairs of every table; free every node and bucket array.
 // Node allocation inside an insert: per thread under the bucket lock (plain
-// form), or CTA-aggregated (batched form: threads that found no room ask
-// together through gal::cta_malloc, then lock again and link the node, or
-// free it when another thread made room meanwhile).
+// form), or CTA-aggregated (batched form: every thread holds a node ready, and
+// the threads that used theirs ask for the next together through
+// gal::cta_malloc; a node left over at the end is freed).
+//
+// Bound by latency: an op is a chain of scattered round trips (lock 800 cycles,
+// a node 700-1,000 from L2, more from DRAM, a release 800-1,600).  What kept the
+// phases from overlapping them was divergence: lanes that held a lock waited for
+// the warp's others to get theirs, so an instruction ran for 6 to 8 lanes, each
+// group paid fences and claims of its own, and a node was searched one key at a
+// time.  Now a lane tries its lock once per turn; the lanes that got theirs
+// search, allocate, change and release together and fetch their next op, the
+// others (one in twenty, so most warps have one) keep theirs for the next turn.
+// 8.6 M pairs in 128 tables, one slot per SM, in ms, before and now: insert 2.22,
+// 0.68; delete 1.47, 0.33; lookups 0.43 + 0.71, 0.16 + 0.20; reinsert 1.70, 0.49;
+// teardown 0.81, 0.11.
 //
 // Keys: a bijective 64-bit mix of (table << 32 | index) so the keys of a table
 // are distinct and uniform; value = another mix of the key; coin = bit 0 of a
 // third mix.  gallatin_gb300/tables.py restates them on the host.
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 #include <string.h>
 
@@ -62,10 +76,8 @@ constexpr uint32_t FULL = (1u << SLOTS) - 1u;
 
 struct node {
   unsigned long long next;
-  uint32_t used;
-  uint32_t pad;
-  unsigned long long key[SLOTS];
-  unsigned long long val[SLOTS];
+  unsigned long long meta;  // byte 0: used mask; byte 1 + k: tag of place k
+  ulonglong2 pair[SLOTS];   // key, value: one 16-byte load or store
 };
 static_assert(sizeof(node) == 128, "one 128 B slice per node");
 
@@ -90,9 +102,9 @@ __device__ __forceinline__ uint64_t table_key(uint32_t t, uint64_t i, uint64_t s
 }
 __device__ __forceinline__ uint64_t table_val(uint64_t key) { return mix64(key ^ 0x5851F42D4C957F2Dull); }
 __device__ __forceinline__ bool table_coin(uint64_t key) { return mix64(key + 0x2545F4914F6CDD1Dull) & 1u; }
-__device__ __forceinline__ uint64_t bucket_of(uint64_t key, uint64_t nb) {
-  return mix64(key ^ 0x9E3779B97F4A7C15ull) & (nb - 1u);
-}
+__device__ __forceinline__ uint64_t table_hash(uint64_t key) { return mix64(key ^ 0x9E3779B97F4A7C15ull); }
+__device__ __forceinline__ uint64_t bucket_of(uint64_t hash, uint64_t nb) { return hash & (nb - 1u); }
+__device__ __forceinline__ uint32_t tag_of(uint64_t hash) { return (uint32_t)(hash >> 56); }
 
 // per-thread counters, summed per warp once at the end of a phase kernel
 struct counters {
@@ -111,23 +123,14 @@ __device__ __forceinline__ void flush(unsigned long long *stats, const counters 
   }
 }
 
-// bucket lock: bit 0 of the head word; bounded wait
-__device__ __forceinline__ bool lock_bucket(const gal::state *s, unsigned long long *hp,
-                                            unsigned long long &head) {
-  for (uint32_t i = 0; i < s->spin_limit; i++) {
-    unsigned long long h = gal::ld_rlx((const uint64_t *)hp);
-    if (!(h & 1ull) && atomicCAS(hp, h, h | 1ull) == h) {
-      __threadfence();
-      head = h;
-      return true;
-    }
-    gal::backoff(i);
-  }
-  return false;
+// Bucket lock: bit 0 of the head word.  One try (a round trip whether or not
+// somebody holds it); true: `head` is the list, this thread's until it unlocks.
+__device__ __forceinline__ bool try_lock_bucket(unsigned long long *hp, unsigned long long &head) {
+  asm volatile("atom.acquire.gpu.global.or.b64 %0, [%1], 1;" : "=l"(head) : "l"(hp) : "memory");
+  return !(head & 1ull);
 }
 __device__ __forceinline__ void unlock_bucket(unsigned long long *hp, unsigned long long head) {
-  __threadfence();
-  atomicExch(hp, head & ~1ull);
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(hp), "l"(head) : "memory");
 }
 
 // the table of flattened op i
@@ -141,207 +144,214 @@ __device__ __forceinline__ uint32_t table_of(const uint64_t *off, uint32_t ntab,
   return lo;
 }
 
-// Under the lock: the key's place, or a node with room.  found: key present
-// (n, slot); else room: a node with a free slot (n, slot), or n == 0.
+// The used places of a node whose tag is `tag`.
+__device__ __forceinline__ uint32_t tagged(unsigned long long meta, uint32_t tag) {
+  const uint32_t all = tag * 0x01010101u;
+  const uint32_t lo = __vcmpeq4((uint32_t)(meta >> 8), all) & 0x01010101u;
+  const uint32_t hi = __vcmpeq4((uint32_t)(meta >> 40), all) & 0x00010101u;
+  // one bit per byte, gathered by the product's bits 24-27
+  return (((lo * 0x01020408u) >> 24) | ((hi * 0x01020408u) >> 24) << 4) & (uint32_t)meta & FULL;
+}
+__device__ __forceinline__ unsigned long long with_place(unsigned long long meta, uint32_t k, uint32_t tag) {
+  return (meta & ~(0xFFull << (8 + 8 * k))) | (unsigned long long)tag << (8 + 8 * k) | 1ull << k;
+}
+
+// Under the lock: the key's place (found: n, slot, meta, val, prev: its
+// predecessor or 0 for the head, next), else a node with room (n, slot, meta), or n == 0.
+// Node words are read past L1: another SM may have written them under the same
+// bucket lock since this SM last cached the line.  One 16-byte load answers for
+// a node unless a tag matches (the key's own, or one time in 256): loading all
+// seven keys took five loads a node, each a scattered line per lane, and bound
+// the lookups by L1 (84 % of its throughput).
 struct probe {
   node *n;
   uint32_t slot;
   bool found;
-  node *prev;  // predecessor of a found key's node (0: the head)
+  unsigned long long meta;
+  node *prev;
+  unsigned long long next;
+  unsigned long long val;
 };
-__device__ __forceinline__ probe find(unsigned long long head, uint64_t key) {
-  probe r{nullptr, 0, false, nullptr};
-  node *room = nullptr;
-  uint32_t room_slot = 0;
+__device__ __forceinline__ probe find(unsigned long long head, uint64_t key, uint32_t tag) {
+  probe r{};
   node *prev = nullptr;
-  for (node *n = (node *)(head & ~1ull); n; prev = n, n = (node *)__ldcg(&n->next)) {
-    uint32_t used = __ldcg(&n->used);
-    for (uint32_t m = used; m; m &= m - 1u) {
-      uint32_t k = (uint32_t)__ffs(m) - 1u;
-      if (__ldcg(&n->key[k]) == key) {
-        r.n = n;
-        r.slot = k;
-        r.found = true;
-        r.prev = prev;
-        return r;
-      }
+  for (node *n = (node *)(head & ~1ull); n;) {
+    const ulonglong2 w = __ldcg((const ulonglong2 *)n);  // link, meta
+    for (uint32_t m = tagged(w.y, tag); m; m &= m - 1u) {
+      const uint32_t k = (uint32_t)__ffs(m) - 1u;
+      const ulonglong2 kv = __ldcg(&n->pair[k]);
+      if (kv.x == key) return probe{n, k, true, w.y, prev, w.x, kv.y};
     }
-    if (!room && used != FULL) {
-      room = n;
-      room_slot = (uint32_t)__ffs(~used & FULL) - 1u;
+    if (!r.n && ((uint32_t)w.y & FULL) != FULL) {
+      r.n = n;
+      r.slot = (uint32_t)__ffs(~(uint32_t)w.y & FULL) - 1u;
+      r.meta = w.y;
     }
+    prev = n;
+    n = (node *)w.x;
   }
-  r.n = room;
-  r.slot = room_slot;
   return r;
 }
 
-// node words are read past L1 (__ldcg): another SM may have written them
-// under the same bucket lock since this SM last cached the line
-__device__ __forceinline__ void put(node *n, uint32_t slot, uint64_t key, uint64_t val) {
-  n->key[slot] = key;
-  n->val[slot] = val;
-  n->used = __ldcg(&n->used) | (1u << slot);
+// One turn of an insert, by a whole warp together: true when the op is done.
+// A bucket without room takes `spare`, when there is one (null afterwards);
+// MALLOC: else a node from the allocator under the lock.  The warp meets before
+// the malloc, whose teams are the lanes that call together: lanes that left the
+// search one by one claimed one by one.
+template <bool MALLOC>
+__device__ __forceinline__ bool insert_turn(const gal::state *s, unsigned long long *hp, bool go, uint64_t key,
+                                            uint32_t tag, node *&spare, counters &lc) {
+  unsigned long long head = 0;
+  const bool mine = go && try_lock_bucket(hp, head);
+  probe p{};
+  if (mine) p = find(head, key, tag);
+  const bool full = mine && !p.n;
+  __syncwarp();
+  if (MALLOC) {
+    if (full) {
+      spare = (node *)gal::malloc(s, sizeof(node));
+      if (spare) count(lc, S_NODES);
+    }
+    __syncwarp();
+  }
+  if (!mine) return false;
+  node *n = p.n;
+  if (full) {
+    n = spare;
+    spare = nullptr;
+    if (n) {
+      n->next = head;
+      head = (unsigned long long)n;
+    } else {
+      count(lc, S_MFAIL);
+    }
+  }
+  if (n) {
+    n->pair[p.slot] = make_ulonglong2(key, table_val(key));
+    if (!p.found) {
+      n->meta = with_place(p.meta, p.slot, tag);
+      count(lc, S_INSERTED);
+    }
+  }
+  unlock_bucket(hp, head);
+  return true;
 }
 
-// Insert under the lock.  spare: a node the caller already holds (batched
-// form) or null; returns true when spare was used.
-__device__ bool insert_locked(const gal::state *s, unsigned long long *hp, unsigned long long &head,
-                              uint64_t key, uint64_t val, node *spare, bool may_malloc,
-                              counters &lc, bool &need) {
-  need = false;
-  probe p = find(head, key);
-  if (p.found) {
-    p.n->val[p.slot] = val;
-    return false;
-  }
-  if (p.n) {
-    put(p.n, p.slot, key, val);
-    count(lc, S_INSERTED);
-    return false;
-  }
-  node *n = spare;
-  if (!n && may_malloc) {
-    n = (node *)gal::malloc(s, sizeof(node));
-    if (!n) {
-      count(lc, S_MFAIL);
-      return false;
+__device__ __forceinline__ bool delete_turn(const gal::state *s, unsigned long long *hp, bool go, uint64_t key,
+                                            uint32_t tag, counters &lc) {
+  unsigned long long head = 0;
+  const bool mine = go && try_lock_bucket(hp, head);
+  probe p{};
+  if (mine) p = find(head, key, tag);
+  __syncwarp();
+  node *dead = nullptr;
+  if (mine) {
+    if (p.found) {
+      const unsigned long long meta = p.meta & ~(1ull << p.slot);
+      count(lc, S_DELETED);
+      if ((uint32_t)meta & FULL) {
+        p.n->meta = meta;
+      } else {  // unlink and free the empty node
+        if (p.prev) p.prev->next = p.next;
+        else head = p.next;
+        dead = p.n;
+      }
     }
-    count(lc, S_NODES);
+    unlock_bucket(hp, head);
   }
-  if (!n) {
-    need = true;
-    return false;
+  __syncwarp();
+  if (dead) {
+    gal::free(s, dead);
+    count(lc, S_NODES_FREED);
   }
-  n->next = head & ~1ull;
-  n->used = 1u;
-  n->key[0] = key;
-  n->val[0] = val;
-  head = (unsigned long long)n;
-  count(lc, S_INSERTED);
-  return n == spare;
+  return mine;
+}
+
+__device__ __forceinline__ void lookup_op(const unsigned long long *hp, uint64_t key, uint32_t tag, bool expect,
+                                          counters &lc) {
+  const probe p = find(__ldcg(hp), key, tag);
+  if (expect && !p.found) count(lc, S_MISSING);
+  if (!expect && p.found) count(lc, S_UNEXPECTED);
+  if (expect && p.found && p.val != table_val(key)) count(lc, S_WRONG);
 }
 
 // phase ops
 enum : int { PH_INSERT = 0, PH_DELETE = 1, PH_CHECK_DELETED = 2, PH_REINSERT = 3, PH_CHECK_ALL = 4 };
 
-__device__ void lookup_check(const table_desc &d, uint64_t key, bool expect, counters &lc) {
-  unsigned long long head = __ldcg(&d.heads[bucket_of(key, d.nbuckets)]);
-  probe p = find(head, key);
-  if (expect && !p.found) count(lc, S_MISSING);
-  if (!expect && p.found) count(lc, S_UNEXPECTED);
-  if (expect && p.found && __ldcg(&p.n->val[p.slot]) != table_val(key)) count(lc, S_WRONG);
-}
-
-__device__ void delete_key(const gal::state *s, const table_desc &d, uint64_t key, counters &lc) {
-  unsigned long long *hp = &d.heads[bucket_of(key, d.nbuckets)];
-  unsigned long long head;
-  if (!lock_bucket(s, hp, head)) {
-    count(lc, S_LOCK);
-    return;
-  }
-  probe p = find(head, key);
-  node *dead = nullptr;
-  if (p.found) {
-    uint32_t used = __ldcg(&p.n->used) & ~(1u << p.slot);
-    p.n->used = used;
-    count(lc, S_DELETED);
-    if (used == 0) {  // unlink and free the empty node
-      unsigned long long nx = __ldcg(&p.n->next);
-      if (p.prev) p.prev->next = nx;
-      else head = nx;
-      dead = p.n;
-    }
-  }
-  unlock_bucket(hp, head);
-  if (dead) {
-    gal::free(s, dead);
-    count(lc, S_NODES_FREED);
-  }
-}
-
-__device__ void insert_plain(const gal::state *s, const table_desc &d, uint64_t key, counters &lc) {
-  unsigned long long *hp = &d.heads[bucket_of(key, d.nbuckets)];
-  unsigned long long head;
-  if (!lock_bucket(s, hp, head)) {
-    count(lc, S_LOCK);
-    return;
-  }
-  bool need;
-  insert_locked(s, hp, head, key, table_val(key), nullptr, true, lc, need);
-  unlock_bucket(hp, head);
-}
-
-__global__ void __launch_bounds__(TBT)
-    k_tables_phase(const gal::state *s, int phase, int batched, uint32_t ntab, const uint64_t *offsets,
-                   const table_desc *desc, uint64_t seed, unsigned long long *stats) {
-  __shared__ uint64_t off[MAX_TABLES + 1];
+// One phase; BATCHED: nodes of an insert phase come from gal::cta_malloc.
+// Registers for five CTAs per SM where the phase allocates, although the
+// allocator's rare paths then spill (insert 0.88, 0.84, 0.81 ms at 3, 4 and 5
+// CTAs), and for six where it only frees or reads.
+template <int PHASE, bool BATCHED>
+__global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSERT ? 5 : 6)
+    k_tables_phase(const gal::state *s, uint32_t ntab, const uint64_t *offsets, const table_desc *desc, uint64_t seed,
+                   unsigned long long *stats) {
+  constexpr bool INSERTS = PHASE == PH_INSERT || PHASE == PH_REINSERT;
+  constexpr bool LOCKS = INSERTS || PHASE == PH_DELETE;
+  extern __shared__ uint64_t off[];  // [ntab + 1]
   __shared__ gal::cta_claim_smem cm;
   for (uint32_t i = threadIdx.x; i <= ntab; i += blockDim.x) off[i] = offsets[i];
-  gal::cta_claim_init(cm);
+  if (INSERTS && BATCHED) gal::cta_claim_init(cm);
   __syncthreads();
   counters lc = {};
   const uint64_t total = off[ntab];
   const uint64_t stride = (uint64_t)gridDim.x * TBT;
-  // the batched insert needs every thread of the CTA at each cta_malloc: the
-  // loop runs the same number of iterations in all of them
-  for (uint64_t base = (uint64_t)blockIdx.x * TBT; base < total; base += stride) {
-    const uint64_t i = base + threadIdx.x;
-    const bool has = i < total;
-    uint32_t t = 0;
-    uint64_t key = 0;
-    if (has) {
-      t = table_of(off, ntab, i);
-      key = table_key(t, i - off[t], seed);
+  uint64_t i = (uint64_t)blockIdx.x * TBT + threadIdx.x;  // this thread's next op
+  unsigned long long *hp = nullptr;
+  uint64_t key = 0;
+  uint32_t tag = 0, waited = 0;
+  bool go = false, coin = false;
+  // the op at i, if it is one of the phase's (half are not where the coin selects)
+  auto fetch = [&]() {
+    const uint32_t t = table_of(off, ntab, i);
+    const table_desc d = desc[t];
+    key = table_key(t, i - off[t], seed);
+    coin = table_coin(key);
+    const uint64_t hash = table_hash(key);
+    tag = tag_of(hash);
+    hp = d.heads + bucket_of(hash, d.nbuckets);
+    go = d.heads && (PHASE == PH_INSERT || !LOCKS || coin);
+    waited = 0;
+    i += stride;
+  };
+  if (LOCKS) {
+    constexpr int FETCHES = PHASE == PH_INSERT ? 1 : 3;  // seven lanes in eight have an op then
+    node *spare = nullptr;
+    for (;;) {
+#pragma unroll 1
+      for (int f = 0; f < FETCHES && __any_sync(0xFFFFFFFFu, !go && i < total); f++)
+        if (!go && i < total) fetch();
+      const bool more = go || i < total;
+      if (INSERTS && BATCHED) {
+        if (!__syncthreads_or(more)) break;
+        node *n = (node *)gal::cta_malloc(s, sizeof(node), go && !spare, cm);
+        if (n) {
+          spare = n;
+          count(lc, S_NODES);
+        }
+      } else if (!__any_sync(0xFFFFFFFFu, more)) {
+        break;
+      }
+      const bool done = INSERTS ? insert_turn<!BATCHED>(s, hp, go, key, tag, spare, lc)
+                                : delete_turn(s, hp, go, key, tag, lc);
+      if (done) go = false;
+      if (go && ++waited > s->spin_limit) {
+        count(lc, S_LOCK);
+        go = false;
+      }
     }
-    const table_desc d = has ? desc[t] : table_desc{nullptr, 1};
-    const bool ok = has && d.heads != nullptr;
-    const bool coin = ok && table_coin(key);
-    if (phase == PH_INSERT || phase == PH_REINSERT) {
-      const bool mine = ok && (phase == PH_INSERT || coin);
-      if (!batched) {
-        if (mine) insert_plain(s, d, key, lc);
-        continue;
-      }
-      // batched: try without allocating, then ask for nodes together
-      bool need = false;
-      unsigned long long *hp = mine ? &d.heads[bucket_of(key, d.nbuckets)] : nullptr;
-      if (mine) {
-        unsigned long long head;
-        if (lock_bucket(s, hp, head)) {
-          insert_locked(s, hp, head, key, table_val(key), nullptr, false, lc, need);
-          unlock_bucket(hp, head);
-        } else {
-          count(lc, S_LOCK);
-        }
-      }
-      node *spare = (node *)gal::cta_malloc(s, sizeof(node), need, cm);
-      if (need && !spare) count(lc, S_MFAIL);
-      if (spare) {
-        count(lc, S_NODES);
-        unsigned long long head;
-        bool used = false;
-        if (lock_bucket(s, hp, head)) {
-          bool again;
-          used = insert_locked(s, hp, head, key, table_val(key), spare, false, lc, again);
-          unlock_bucket(hp, head);
-        } else {
-          count(lc, S_LOCK);
-        }
-        if (!used) {  // another thread made room meanwhile
-          gal::free(s, spare);
-          count(lc, S_SPARE);
-        }
-      }
-    } else if (phase == PH_DELETE) {
-      if (ok && coin) delete_key(s, d, key, lc);
-    } else if (phase == PH_CHECK_DELETED) {
-      if (ok) lookup_check(d, key, !coin, lc);
-    } else {
-      if (ok) lookup_check(d, key, true, lc);
+    if (spare) {  // held ready to the end
+      gal::free(s, spare);
+      count(lc, S_SPARE);
     }
+  } else {
+    while (i < total) {
+      fetch();
+      if (go) lookup_op(hp, key, tag, PHASE == PH_CHECK_ALL || !coin, lc);
+    }
+    __syncwarp();
   }
-  flush(stats, lc);  // every thread ran the same iterations: the warps are whole
+  flush(stats, lc);  // whole warps
 }
 
 // one CTA per table: its bucket array from the allocator, zeroed
@@ -361,53 +371,86 @@ __global__ void __launch_bounds__(TBT)
   }
   __syncthreads();
   if (!heads) return;
-  for (uint64_t b = threadIdx.x; b < nb; b += blockDim.x) heads[b] = 0ull;
+  for (uint64_t b = threadIdx.x; b < nb / 2; b += blockDim.x) ((ulonglong2 *)heads)[b] = make_ulonglong2(0, 0);
 }
 
-// one CTA per table: live pairs, compared with the expected count
-__global__ void __launch_bounds__(TBT)
-    k_tables_count(const uint64_t *offsets, const table_desc *desc, unsigned long long *stats) {
-  __shared__ unsigned long long live;
-  const uint32_t t = blockIdx.x;
-  const table_desc d = desc[t];
-  if (threadIdx.x == 0) live = 0;
-  __syncthreads();
+// The kernels below walk every bucket: TABLE_CTAS CTAs per table, as one per
+// table left the chip to the largest (128 tables of 4 Ki-256 Ki pairs: count
+// 404, dump 3,101, teardown 805 us).
+constexpr int TABLE_CTAS = 32;
+#define EACH_BUCKET(b, d)                                                                               \
+  for (uint64_t b = (uint64_t)blockIdx.y * TBT + threadIdx.x; b < (d).nbuckets; b += (uint64_t)gridDim.y * TBT)
+
+// live pairs of every table
+__global__ void __launch_bounds__(TBT) k_tables_count(const table_desc *desc, unsigned long long *live) {
+  const table_desc d = desc[blockIdx.x];
   if (!d.heads) return;
-  unsigned long long mine = 0;
-  for (uint64_t b = threadIdx.x; b < d.nbuckets; b += blockDim.x)
-    for (node *n = (node *)(__ldcg(&d.heads[b]) & ~1ull); n; n = (node *)__ldcg(&n->next))
-      mine += (unsigned long long)__popc(__ldcg(&n->used));
-  atomicAdd(&live, mine);
-  __syncthreads();
-  if (threadIdx.x == 0 && live != offsets[t + 1] - offsets[t]) count_global(stats, S_COUNT_MISMATCH);
+  uint32_t mine = 0;
+  EACH_BUCKET(b, d)
+    for (node *n = (node *)(__ldcg(&d.heads[b]) & ~1ull); n;) {
+      const ulonglong2 w = __ldcg((const ulonglong2 *)n);
+      mine += (uint32_t)__popc((uint32_t)w.y & FULL);
+      n = (node *)w.x;
+    }
+  mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&live[blockIdx.x], (unsigned long long)mine);
+}
+// ... compared with the expected counts
+__global__ void __launch_bounds__(TBT)
+    k_tables_compare(uint32_t ntab, const uint64_t *offsets, const table_desc *desc, const unsigned long long *live,
+                     unsigned long long *stats) {
+  const uint32_t t = blockIdx.x * TBT + threadIdx.x;
+  if (t < ntab && desc[t].heads && live[t] != offsets[t + 1] - offsets[t]) count_global(stats, S_COUNT_MISMATCH);
 }
 
-// one CTA per table: (key, value) pairs of table `which` appended to out
-__global__ void k_tables_dump(const table_desc *desc, uint32_t which, unsigned long long *keys,
-                              unsigned long long *vals, uint64_t cap, unsigned long long *n_out) {
+// (key, value) pairs of table `which` appended to out, a warp's pairs of one
+// turn with one reservation
+__global__ void __launch_bounds__(TBT)
+    k_tables_dump(const table_desc *desc, uint32_t which, unsigned long long *keys, unsigned long long *vals,
+                  uint64_t cap, unsigned long long *n_out) {
   const table_desc d = desc[which];
   if (!d.heads) return;
-  for (uint64_t b = threadIdx.x; b < d.nbuckets; b += blockDim.x)
-    for (node *n = (node *)(__ldcg(&d.heads[b]) & ~1ull); n; n = (node *)__ldcg(&n->next)) {
-      uint32_t used = __ldcg(&n->used);
-      for (uint32_t m = used; m; m &= m - 1u) {
-        uint32_t k = (uint32_t)__ffs(m) - 1u;
-        unsigned long long at = atomicAdd(n_out, 1ull);
-        if (at < cap) {
-          keys[at] = __ldcg(&n->key[k]);
-          vals[at] = __ldcg(&n->val[k]);
-        }
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint64_t b0 = (uint64_t)blockIdx.y * TBT; b0 < d.nbuckets; b0 += (uint64_t)gridDim.y * TBT) {
+    const uint64_t b = b0 + threadIdx.x;
+    node *n = b < d.nbuckets ? (node *)(__ldcg(&d.heads[b]) & ~1ull) : nullptr;
+    while (__any_sync(0xFFFFFFFFu, n != nullptr)) {
+      ulonglong2 w[8] = {};
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+        if (n) w[k] = __ldcg((const ulonglong2 *)n + k);
+      const unsigned long long *words = (const unsigned long long *)w;  // link, meta, pairs
+      const uint32_t used = n ? (uint32_t)w[0].y & FULL : 0u, mine = (uint32_t)__popc(used);
+      uint32_t upto = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+        if (lane >= (uint32_t)o) upto += v;
       }
+      unsigned long long at = 0;
+      if (lane == 31 && upto) at = atomicAdd(n_out, (unsigned long long)upto);
+      at = __shfl_sync(0xFFFFFFFFu, at, 31) + upto - mine;
+#pragma unroll
+      for (int k = 0; k < (int)SLOTS; k++)
+        if ((used >> k) & 1u) {
+          if (at < cap) {
+            keys[at] = words[2 + 2 * k];
+            vals[at] = words[3 + 2 * k];
+          }
+          at++;
+        }
+      n = n ? (node *)w[0].x : nullptr;
     }
+  }
 }
 
-// one CTA per table: every node and the bucket array back to the allocator
+// every node back to the allocator, then (k_tables_drop) every bucket array
 __global__ void __launch_bounds__(TBT)
     k_tables_destroy(const gal::state *s, const table_desc *desc, unsigned long long *stats) {
   const table_desc d = desc[blockIdx.x];
   if (!d.heads) return;
   uint32_t freed = 0;
-  for (uint64_t b = threadIdx.x; b < d.nbuckets; b += blockDim.x) {
+  EACH_BUCKET(b, d) {
     node *n = (node *)(__ldcg(&d.heads[b]) & ~1ull);
     while (n) {
       node *nx = (node *)__ldcg(&n->next);
@@ -416,9 +459,12 @@ __global__ void __launch_bounds__(TBT)
       n = nx;
     }
   }
-  count_global(stats, S_NODES_FREED, freed);
-  __syncthreads();
-  if (threadIdx.x == 0) gal::free(s, d.heads);
+  freed = __reduce_add_sync(0xFFFFFFFFu, freed);
+  if ((threadIdx.x & 31) == 0) count_global(stats, S_NODES_FREED, freed);
+}
+__global__ void __launch_bounds__(TBT) k_tables_drop(const gal::state *s, uint32_t ntab, const table_desc *desc) {
+  const uint32_t t = blockIdx.x * TBT + threadIdx.x;
+  if (t < ntab && desc[t].heads) gal::free(s, desc[t].heads);
 }
 
 }  // namespace
@@ -440,19 +486,23 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
   memset(res, 0, sizeof(*res));
   const gal::state *d = (const gal::state *)gal_device_state(h);
   int rc = GAL_OK;
-  uint64_t *d_off = nullptr;
-  table_desc *d_desc = nullptr;
-  unsigned long long *stats = nullptr, *d_keys = nullptr, *d_vals = nullptr, *d_n = nullptr;
+  // one device buffer: offsets, descriptors, per-table counts, counters, and
+  // the dumped pairs with their number
+  const bool dump = dump_keys && dump_vals && dump_n && dump_table < n_tables && dump_cap;
+  // (the pairs on 256-byte boundaries: a copy from an odd word ran at 4 GB/s)
+  const size_t head_words = ((size_t)n_tables * 4 + 1 + S_N + 1 + 31) / 32 * 32;
+  const size_t pair_words = dump ? ((size_t)dump_cap + 31) / 32 * 32 : 0;
+  static_assert(sizeof(table_desc) == 16, "two words per table");
+  uint64_t *buf = nullptr;
   cudaEvent_t ev[8] = {};  // phase boundaries 0-5, teardown 6-7
   unsigned long long hs[S_N];
-  int dev = 0, sms = 0, per_sm = 0;
+  int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tables_phase, TBT, 0);
   const uint64_t total = offsets[n_tables];
   const uint64_t need_ctas = (total + TBT - 1) / TBT;
-  const unsigned grid = (unsigned)std::min<uint64_t>(need_ctas ? need_ctas : 1,
-                                                     (uint64_t)sms * (per_sm > 0 ? per_sm : 1));
+  const size_t smem = (n_tables + 1) * sizeof(uint64_t);
+  const dim3 all_buckets(n_tables, TABLE_CTAS);
 #define TK(x)                        \
   do {                               \
     if ((x) != cudaSuccess) {        \
@@ -460,31 +510,44 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
       goto done;                     \
     }                                \
   } while (0)
-  TK(cudaMalloc(&d_off, (n_tables + 1) * sizeof(uint64_t)));
-  TK(cudaMalloc(&d_desc, n_tables * sizeof(table_desc)));
-  TK(cudaMalloc(&stats, sizeof(hs)));
+  TK(cudaMalloc(&buf, (head_words + 2 * pair_words) * sizeof(uint64_t)));
+  {
+  table_desc *d_desc = (table_desc *)buf;
+  uint64_t *d_off = buf + 2 * (size_t)n_tables;
+  unsigned long long *live = (unsigned long long *)(d_off + n_tables + 1), *stats = live + n_tables;
+  unsigned long long *d_n = stats + S_N, *d_keys = (unsigned long long *)buf + head_words, *d_vals = d_keys + pair_words;
   TK(cudaMemcpy(d_off, offsets, (n_tables + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice));
-  TK(cudaMemset(stats, 0, sizeof(hs)));
+  TK(cudaMemset(live, 0, (n_tables + S_N + 1) * sizeof(uint64_t)));
   for (auto &e : ev) TK(cudaEventCreate(&e));
   k_tables_setup<<<n_tables, TBT>>>(d, d_off, d_desc, stats);
   TK(cudaGetLastError());
   TK(cudaEventRecord(ev[0]));
   {
-    const int phases[5] = {PH_INSERT, PH_DELETE, PH_CHECK_DELETED, PH_REINSERT, PH_CHECK_ALL};
-    for (int k = 0; k < 5; k++) {
-      k_tables_phase<<<grid, TBT>>>(d, phases[k], batched, n_tables, d_off, d_desc, seed, stats);
-      TK(cudaGetLastError());
-      TK(cudaEventRecord(ev[k + 1]));
-    }
+    auto phase = [&](auto kern) {
+      int per_sm = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TBT, smem);
+      const uint64_t fit = (uint64_t)sms * (per_sm > 0 ? per_sm : 1);
+      kern<<<(unsigned)std::min<uint64_t>(need_ctas ? need_ctas : 1, fit), TBT, smem>>>(d, n_tables, d_off, d_desc,
+                                                                                        seed, stats);
+      return cudaGetLastError();
+    };
+    TK(batched ? phase(k_tables_phase<PH_INSERT, true>) : phase(k_tables_phase<PH_INSERT, false>));
+    TK(cudaEventRecord(ev[1]));
+    TK(phase(k_tables_phase<PH_DELETE, false>));
+    TK(cudaEventRecord(ev[2]));
+    TK(phase(k_tables_phase<PH_CHECK_DELETED, false>));
+    TK(cudaEventRecord(ev[3]));
+    TK(batched ? phase(k_tables_phase<PH_REINSERT, true>) : phase(k_tables_phase<PH_REINSERT, false>));
+    TK(cudaEventRecord(ev[4]));
+    TK(phase(k_tables_phase<PH_CHECK_ALL, false>));
+    TK(cudaEventRecord(ev[5]));
   }
-  k_tables_count<<<n_tables, TBT>>>(d_off, d_desc, stats);
+  k_tables_count<<<all_buckets, TBT>>>(d_desc, live);
   TK(cudaGetLastError());
-  if (dump_keys && dump_vals && dump_n && dump_table < n_tables && dump_cap) {
-    TK(cudaMalloc(&d_keys, dump_cap * 8));
-    TK(cudaMalloc(&d_vals, dump_cap * 8));
-    TK(cudaMalloc(&d_n, 8));
-    TK(cudaMemset(d_n, 0, 8));
-    k_tables_dump<<<1, TBT>>>(d_desc, dump_table, d_keys, d_vals, dump_cap, d_n);
+  k_tables_compare<<<(n_tables + TBT - 1) / TBT, TBT>>>(n_tables, d_off, d_desc, live, stats);
+  TK(cudaGetLastError());
+  if (dump) {
+    k_tables_dump<<<dim3(1, TABLE_CTAS * 8), TBT>>>(d_desc, dump_table, d_keys, d_vals, dump_cap, d_n);
     TK(cudaGetLastError());
     TK(cudaMemcpy(dump_n, d_n, 8, cudaMemcpyDeviceToHost));
     uint64_t got = *dump_n < dump_cap ? *dump_n : dump_cap;
@@ -492,13 +555,16 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
     TK(cudaMemcpy(dump_vals, d_vals, got * 8, cudaMemcpyDeviceToHost));
   }
   TK(cudaEventRecord(ev[6]));
-  k_tables_destroy<<<n_tables, TBT>>>(d, d_desc, stats);
+  k_tables_destroy<<<all_buckets, TBT>>>(d, d_desc, stats);
+  TK(cudaGetLastError());
+  k_tables_drop<<<(n_tables + TBT - 1) / TBT, TBT>>>(d, n_tables, d_desc);
   TK(cudaGetLastError());
   TK(cudaEventRecord(ev[7]));
   TK(cudaEventSynchronize(ev[7]));
   TK(cudaEventElapsedTime(&res->ms[5], ev[6], ev[7]));
   for (int k = 0; k < 5; k++) TK(cudaEventElapsedTime(&res->ms[k], ev[k], ev[k + 1]));
   TK(cudaMemcpy(hs, stats, sizeof(hs), cudaMemcpyDeviceToHost));
+  }
   res->total_pairs = total;
   res->inserted = hs[S_INSERTED];
   res->deleted = hs[S_DELETED];
@@ -521,12 +587,7 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
 done:
   for (auto &e : ev)
     if (e) cudaEventDestroy(e);
-  if (d_off) cudaFree(d_off);
-  if (d_desc) cudaFree(d_desc);
-  if (stats) cudaFree(stats);
-  if (d_keys) cudaFree(d_keys);
-  if (d_vals) cudaFree(d_vals);
-  if (d_n) cudaFree(d_n);
+  if (buf) cudaFree(buf);
   return rc;
 }
 
