@@ -261,7 +261,7 @@ __device__ __forceinline__ bool delete_turn(const gal::state *s, unsigned long l
   }
   __syncwarp();
   if (dead) {
-    gal::free(s, dead);
+    gal::free_sized(s, dead, sizeof(node));
     count(lc, S_NODES_FREED);
   }
   return mine;
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
       }
     }
     if (spare) {  // held ready to the end
-      gal::free(s, spare);
+      gal::free_sized(s, spare, sizeof(node));
       count(lc, S_SPARE);
     }
   } else {
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(TBT)
     node *n = (node *)(__ldcg(&d.heads[b]) & ~1ull);
     while (n) {
       node *nx = (node *)__ldcg(&n->next);
-      gal::free(s, n);
+      gal::free_sized(s, n, sizeof(node));
       freed++;
       n = nx;
     }

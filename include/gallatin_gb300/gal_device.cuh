@@ -1551,6 +1551,23 @@ GAL_DEVICE_INLINE void free(const state *s, void *ptr) {
   free_block_slices(s, blk);
 }
 
+// free of a live pointer whose request size the caller knows: a slice's class
+// follows from the size, so the pointer's segment need not be looked up (the
+// first of free's two dependent round trips).
+GAL_DEVICE_INLINE void free_sized(const state *s, void *ptr, uint64_t size) {
+  const int T = (int)cfield(s->num_trees), min_shift = (int)cfield(s->min_shift);
+  const int bits = size > 1 ? 64 - __clzll((long long)(size - 1)) : 0;
+  const int t = max(bits - min_shift, 0);
+  if (t >= T && bits >= min_shift + 12) {  // a block or segments
+    gal::free(s, ptr);
+    return;
+  }
+  const uint64_t off = (uint64_t)((char *)ptr - cfield(s->memory));
+  const uint64_t in_seg = off & ((1ull << cfield(s->seg_shift)) - 1ull);
+  free_block_slices(s, (uint32_t)((off >> cfield(s->seg_shift)) << cfield(s->bps_shift)) +
+                           (uint32_t)(in_seg >> (min_shift + min(t, T - 1) + 12)));
+}
+
 // block id of a live pointer (slice or whole block), NOBLK for a segment run
 GAL_DEVICE_INLINE uint32_t block_of(const state *s, const void *ptr, uint16_t &tree_out) {
   uint64_t off = (uint64_t)((const char *)ptr - cfield(s->memory));
