@@ -30,7 +30,7 @@ struct gal_handle {
   char *arena = nullptr;
   uint64_t arena_bytes = 0;
   gal_state_dims dims{};
-  int grid_free = 0;  // persistent grid of the batched free kernel (0: not yet known)
+  int grid_free[4] = {};  // persistent grids of the batched free kernels (0: not yet known)
   int sms = 1;        // SMs of the device
 };
 
@@ -242,8 +242,6 @@ __global__ void k_free_per_thread(const gal::state *s, void *const *ptrs, uint64
   if (p) gal::free(s, p);
 }
 
-constexpr int BATCH_THREADS = 512;
-
 // Batched malloc of short lists: one thread per request, warp teams claiming
 // with one atomicAdd per team on their SM's pinned block (gal::malloc), compiled
 // for four CTAs of 256 threads per SM (64 registers).
@@ -271,40 +269,25 @@ __global__ void __launch_bounds__(gal::BULK_THREADS, 2)
   gal::bulk_malloc<K>(s, sizes, n, (uint64_t)blockIdx.x * (K * gal::BULK_THREADS), out, sm);
 }
 
-// Batched free: each thread takes FREE_PER_THREAD entries per pass of a
-// persistent grid and frees them with gal::free_n (table lookups and
-// free-counter atomics issued back to back, warp teams per block).  The list
-// holds n entries, or *d_count when that is given and smaller (a count that
-// an earlier kernel on the stream wrote).
-constexpr int FREE_PER_THREAD = 4;
-
-__global__ void __launch_bounds__(BATCH_THREADS)
-    k_free_batched(const gal::state *s, void *const *ptrs, uint64_t n,
-                   const unsigned long long *d_count, int stage) {
-  // the pointers were allocated before this call, and a live pointer's
-  // segment keeps its class: a copy of the classes staged now serves them
+// Batched free: a persistent grid, a CTA taking chunks of 256 K entries and
+// counting them by block in shared memory (gal_bulk.cuh).  K is the smallest of
+// 1, 2, 4 and 8 whose chunks the grid takes at once: larger chunks share more
+// blocks, smaller ones start more SMs.  The list holds n
+// entries, or *d_count when that is given and smaller (a count that an earlier
+// kernel on the stream wrote).  With stage, the segments' classes are copied to
+// shared memory first: the pointers were allocated before this call, and a live
+// pointer's segment keeps its class.
+template <int K>
+__global__ void __launch_bounds__(gal::BULK_FREE_THREADS, 4)
+    k_free_bulk(const gal::state *s, void *const *ptrs, uint64_t n, const unsigned long long *d_count, int stage) {
+  __shared__ gal::bulk_free_smem<K> sm;
   extern __shared__ uint16_t classes[];
   const bool staged = stage && gal::stage_classes(s, classes);
+  gal::bulk_free_init(sm);
   __syncthreads();
   if (d_count && *d_count < n) n = *d_count;
-  // a warp takes 32 x FREE_PER_THREAD consecutive entries; lane l holds entries
-  // l, l + 32, ... so neighbouring lanes hold neighbouring entries (which share
-  // blocks) in each of the FREE_PER_THREAD team formations
-  const uint64_t per_warp = 32ull * FREE_PER_THREAD;
-  const uint64_t warp = ((uint64_t)blockIdx.x * BATCH_THREADS + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * BATCH_THREADS) >> 5;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t w0 = warp * per_warp; w0 < n; w0 += nwarps * per_warp) {
-    void *p[FREE_PER_THREAD];
-    bool go[FREE_PER_THREAD];
-#pragma unroll
-    for (int k = 0; k < FREE_PER_THREAD; k++) {
-      const uint64_t i = w0 + (uint64_t)k * 32u + lane;
-      p[k] = i < n ? ptrs[i] : nullptr;
-      go[k] = p[k] != nullptr;
-    }
-    gal::free_n<FREE_PER_THREAD>(s, p, go, staged ? classes : nullptr);
-  }
+  for (uint64_t base = (uint64_t)blockIdx.x * sm.CHUNK; base < n; base += (uint64_t)gridDim.x * sm.CHUNK)
+    gal::bulk_free(s, ptrs, n, base, staged ? classes : nullptr, sm);
 }
 
 template <class K>
@@ -893,14 +876,24 @@ int gal_free_batched_n(gal_handle *h, void *const *ptrs, const unsigned long lon
   if (!max_n) return GAL_OK;
   gal_device_guard on_dev(h->device);
   CUDA_TRY(on_dev.err);
-  unsigned g = grid_for((max_n + FREE_PER_THREAD - 1) / FREE_PER_THREAD, BATCH_THREADS);
   const size_t stage = h->st.num_segments * 2 <= gal::CLASS_STAGE_BYTES ? h->st.num_segments * 2 : 0;
-  if (!h->grid_free) h->grid_free = persistent_grid(h->device, k_free_batched, BATCH_THREADS, stage);
-  unsigned p = (unsigned)h->grid_free;
-  k_free_batched<<<g < p ? g : p, BATCH_THREADS, stage, (cudaStream_t)stream>>>(h->d_state, ptrs, max_n,
-                                                                                d_count, stage > 0);
-  CUDA_TRY(cudaGetLastError());
-  return GAL_OK;
+  const uint64_t fit = (uint64_t)h->sms * 4 * gal::BULK_FREE_THREADS;  // entries a full grid takes at one each
+  auto bulk = [&](auto kern, int slot, int k) {
+    int &grid = h->grid_free[slot];
+    if (!grid) {
+      CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gal::CLASS_STAGE_BYTES));
+      grid = persistent_grid(h->device, kern, gal::BULK_FREE_THREADS, stage);
+    }
+    const unsigned g = grid_for(max_n, gal::BULK_FREE_THREADS * k), p = (unsigned)grid;
+    kern<<<g < p ? g : p, gal::BULK_FREE_THREADS, stage, (cudaStream_t)stream>>>(h->d_state, ptrs, max_n, d_count,
+                                                                                stage > 0);
+    CUDA_TRY(cudaGetLastError());
+    return GAL_OK;
+  };
+  if (max_n <= fit) return bulk(k_free_bulk<1>, 0, 1);
+  if (max_n <= 2 * fit) return bulk(k_free_bulk<2>, 1, 2);
+  if (max_n <= 4 * fit) return bulk(k_free_bulk<4>, 2, 4);
+  return bulk(k_free_bulk<8>, 3, 8);
 }
 
 }  // extern "C"

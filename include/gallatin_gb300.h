@@ -329,9 +329,9 @@ int gal_trim(gal_handle *h, void *stream);
  * gal_free_per_thread.  Mallocs of 32 Ki requests or more run in chunks, a
  * CTA ranking its requests per size class and claiming the slices of each with
  * one atomicAdd; shorter lists one request per thread, warp teams claiming with
- * one atomicAdd per team.  Frees take four entries per thread on a persistent
- * grid, look the segment classes up in a copy staged in shared memory, and
- * form warp teams per block (one free-counter atomic per team). */
+ * one atomicAdd per team.  Frees run in chunks on a persistent grid, look the
+ * segment classes up in a copy staged in shared memory, and count the chunk's
+ * pointers by block (one free-counter atomic per block and chunk). */
 int gal_malloc_batched(gal_handle *h, const uint64_t *sizes, uint64_t n,
                        void **out_ptrs, void *stream);
 int gal_free_batched(gal_handle *h, void *const *ptrs, uint64_t n, void *stream);

@@ -122,3 +122,64 @@ def test_arena_runs_out(G, torch_mod, size, n):
 def torch_mod():
     import torch
     return torch
+
+
+@pytest.mark.parametrize("order", ["same", "reversed", "shuffled"])
+@pytest.mark.parametrize("n,cfg", [(2047, {}), (2048, TUNED), (2049, {}), (300000, TUNED),
+                                   (311297, {}), (700001, TUNED), (257, {}),
+                                   (50000, dict(min_size=16, max_size=16, bytes_per_segment=64 << 10))],
+                         ids=["2047", "2048", "2049", "two-each", "four-each", "eight-each", "257", "unstaged"])
+def test_frees_in_any_order_with_gaps(G, torch_mod, n, cfg, order):
+    """Lists with null entries, in the order of the mallocs or not, of classes
+    looked up in shared memory or (32,768 segments) not: what is freed comes
+    back, what is not stays."""
+    torch = torch_mod
+    rng = np.random.default_rng(n)
+    sizes = np.rint(2.0 ** rng.uniform(0, 4 if "max_size" in cfg else 12.5, n)).astype(np.int64)
+    g = G.Gallatin.generate_on_device((2 if "max_size" in cfg else 16) << 30, 42, zero_arena=0, **cfg)
+    try:
+        fresh = g.export()
+        ptrs = torch.zeros(n, dtype=torch.int64, device="cuda")
+        g.malloc_batched(torch.from_numpy(sizes).cuda(), ptrs)
+        assert bool((ptrs != 0).all())
+        at = np.arange(n) if order == "same" else np.arange(n)[::-1].copy() if order == "reversed" else rng.permutation(n)
+        lst = ptrs[torch.from_numpy(at).cuda()]
+        gap = torch.from_numpy(rng.random(n) < 0.3).cuda()
+        first = lst.clone()
+        first[gap] = 0
+        g.free_batched(first)
+        second = lst.clone()
+        second[~gap] = 0
+        assert g.error_word() == 0, g.error_info()
+        counted = torch.zeros(1, dtype=torch.int64, device="cuda")
+        for k in (0, 1, min(n, 2048), n // 2):  # the rest, up to counts the device knows
+            counted[0] = k
+            part = second.clone()
+            g.free_batched_n(part, counted)
+            second[:k] = 0
+        counted[0] = n + 5  # more than the list holds
+        g.free_batched_n(second, counted)
+        g.trim()
+        assert g.error_word() == 0, g.error_info()
+        assert g.export().diff(fresh, fields=TREE_FIELDS) == []
+    finally:
+        g.close()
+
+
+def test_frees_of_runs_and_of_pointers_that_are_none(G, torch_mod):
+    torch = torch_mod
+    g = G.Gallatin.generate_on_device(4 << 30, 42, zero_arena=0)
+    try:
+        sizes = torch.full((4000,), 64, dtype=torch.int64, device="cuda")
+        sizes[::1000] = 40 << 20
+        ptrs = torch.zeros(4000, dtype=torch.int64, device="cuda")
+        g.malloc_per_thread(sizes, ptrs)
+        g.free_batched(ptrs)
+        assert g.error_word() == 0 and g.stats().multi_segment_allocs == 0
+        for bad in (g.arena_base + g.arena_bytes + 64,          # outside
+                    g.arena_base + g.arena_bytes - 64):         # in a free segment
+            g.free_batched(torch.full((3,), bad, dtype=torch.int64, device="cuda"))
+            assert g.error_word() == 0x2
+            g.clear_error()
+    finally:
+        g.close()
