@@ -311,8 +311,8 @@ int gal_replay_warp_trace(gal_handle *h, const uint64_t *steps, uint64_t nsteps,
  * global_malloc, global_allocator.cuh:72-76). */
 int gal_malloc_per_thread(gal_handle *h, const uint64_t *sizes, uint64_t n,
                           void **out_ptrs, void *stream);
-/* One device thread per pointer: free(ptrs[i]) unless NULL
- * (global_free, global_allocator.cuh:78-82). */
+/* free(ptrs[i]) for every i unless NULL (global_free,
+ * global_allocator.cuh:78-82); the same kernels as gal_free_batched. */
 int gal_free_per_thread(gal_handle *h, void *const *ptrs, uint64_t n, void *stream);
 
 /* Give back what the pinned slots hold (no counterpart in the reference; the

@@ -1143,7 +1143,7 @@ GAL_DEVICE_INLINE uint32_t pick_slot(const state *s, uint32_t tree, uint32_t &bl
   const uint32_t n = cfield(s->slot_count[tree]);
   const uint32_t *slots = cfield(s->slots) + cfield(s->slot_base[tree]);
   uint32_t smid = cfield(s->smid_override) >= 0 ? (uint32_t)cfield(s->smid_override) : sm_id();
-  int my = (int)(smid % n);
+  int my = (int)(smid < n ? smid : (n & (n - 1u)) == 0 ? smid & (n - 1u) : smid % n);
   int original = my;
   int counter = 0;
   uint32_t v = ld_rlx(&slots[my]);
@@ -1336,27 +1336,35 @@ GAL_DEVICE_INLINE void *malloc_slices(const state *s, uint32_t tree, uint32_t co
       unsigned long long old = 0;
       if ((int)lane == last) old = atomicAdd(mword_ptr(s, blk), (unsigned long long)total);
       old = __shfl_sync(live, old, last);
-      const uint64_t alloc = (old & 0xFFFFFFFFull) + prefix;
-      const bool start_valid = alloc <= SLICES_PER_BLOCK - 1;
-      const bool end_valid = alloc + count <= SLICES_PER_BLOCK;
-      const bool should_replace = start_valid && alloc + count > SLICES_PER_BLOCK - 1;
+      // (counts past 2^24 are as exhausted as any: sums below stay in 32 bits)
+      const uint32_t cnt = min((uint32_t)old, 1u << 24);
       const bool foreign = (uint32_t)(old >> 32) != tree;
-      const bool valid = start_valid && end_valid;
-      if (valid && !foreign) result = slice_ptr(s, blk, alloc, tree);
-      // slices this lane gives back: the rest of a run, or the part of it past
-      // the block's end (block_correct_frees), and a claimed slice of a block
-      // that serves another class now (Block::check_valid failed)
-      const uint32_t credit = (start_valid ? (end_valid ? count - 1 : (uint32_t)(SLICES_PER_BLOCK - alloc)) : 0u) +
-                              (valid && foreign ? 1u : 0u);
-      uint32_t rep = __ballot_sync(live, should_replace) & team;
-      const bool exhausted = !foreign && (__ballot_sync(live, start_valid) & team) == 0;
-      if (cache) {  // exhausted, replaced or foreign: the next team reads the slot again
-        if ((rep || exhausted || foreign) && (int)lane == leader) atomicCAS(&cache->blk[tree], blk, NOBLK);
+      uint32_t credit = 0;
+      bool lead = false;
+      if (!foreign && count == 1 && cnt + total < SLICES_PER_BLOCK) {  // all but one claim in hundreds
+        result = slice_ptr(s, blk, cnt + prefix, tree);
+      } else {
+        const uint32_t alloc = cnt + prefix;
+        const bool start_valid = alloc <= SLICES_PER_BLOCK - 1;
+        const bool end_valid = alloc + count <= SLICES_PER_BLOCK;
+        const bool valid = start_valid && end_valid;
+        if (valid && !foreign) result = slice_ptr(s, blk, alloc, tree);
+        // slices this lane gives back: the rest of a run, or the part of it past
+        // the block's end (block_correct_frees), and a claimed slice of a block
+        // that serves another class now (Block::check_valid failed)
+        credit = (start_valid ? (end_valid ? count - 1 : SLICES_PER_BLOCK - alloc) : 0u) + (valid && foreign ? 1u : 0u);
+        // the team's lanes take consecutive slices: one of them holds slice 4095
+        // exactly when the claim crosses it
+        bool replace = cnt < SLICES_PER_BLOCK && cnt + total >= SLICES_PER_BLOCK;
+        const bool exhausted = !foreign && cnt >= SLICES_PER_BLOCK;
+        if (cache) {  // exhausted, replaced or foreign: the next team reads the slot again
+          if ((replace || exhausted || foreign) && (int)lane == leader) atomicCAS(&cache->blk[tree], blk, NOBLK);
+        }
+        if (exhausted && fresh && attempt >= STUCK_ATTEMPTS && cnt >= SLICES_PER_BLOCK + STUCK_MARGIN &&
+            ld_rlx(cfield(s->slots) + cfield(s->slot_base[tree]) + slot) == blk)
+          replace = true;  // the slot has held an exhausted block for a while: replace it here
+        lead = replace && (int)lane == leader;
       }
-      if (exhausted && fresh && attempt >= STUCK_ATTEMPTS && (old & 0xFFFFFFFFull) >= SLICES_PER_BLOCK + STUCK_MARGIN &&
-          ld_rlx(cfield(s->slots) + cfield(s->slot_base[tree]) + slot) == blk)
-        rep = team;  // the slot has held an exhausted block for a while: replace it here
-      const bool lead = rep && (int)lane == leader;
       uint32_t group = live;
       if (credit || lead) {
         keep.state = (uint64_t)s;
@@ -1477,10 +1485,10 @@ GAL_DEVICE_COLD void *malloc_large(const state *s, uint64_t size, int block_tree
 // of the same class share a team.
 template <bool NAMED>
 GAL_DEVICE_INLINE void *malloc_from(const state *s, uint64_t size, uint32_t callers, slot_cache *cache = nullptr) {
-  const int T = (int)cfield(s->num_trees);
-  const int bits = ceil_log2(size);
-  const int t = (size >> cfield(s->min_shift)) == 0 ? 0 : bits - (int)cfield(s->min_shift);
-  const int block_tree = bits - (int)(cfield(s->min_shift) + 12);
+  const int T = (int)cfield(s->num_trees), min_shift = (int)cfield(s->min_shift);
+  const int bits = size > 1 ? 64 - __clzll((long long)(size - 1)) : 0;  // ceil(log2)
+  const int t = max(bits - min_shift, 0);
+  const int block_tree = bits - (min_shift + 12);
   const bool slices = t < T || block_tree < 0;
   const uint32_t members = __ballot_sync(callers, slices);
   if (!slices) {
