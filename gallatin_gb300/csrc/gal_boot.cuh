@@ -10,9 +10,9 @@
 //
 //   * Blocks of one segment must come home in slot order (their ring entries);
 //     blocks of different segments have nothing in common but bits of the
-//     trees, whose end state does not depend on the order.  So the slots are
-//     retired 1,024 at a time, each thread finding how many earlier blocks of
-//     the same segment come home with its own.
+//     trees, whose end state does not depend on the order.  So spares and slots
+//     are retired 3,072 at a time, each thread finding how many earlier blocks
+//     of the same segment come home with its own.
 //   * A class whose tree lists no segment boots from fresh segments only: slot
 //     i gets block i mod nb of the class's (i / nb)-th gathered segment, and the
 //     segments gathered, class by class, are the smallest free ids in order.
@@ -31,16 +31,19 @@ namespace gal {
 static constexpr int BOOT_THREADS = 1024;
 static constexpr int BOOT_WARPS = BOOT_THREADS / 32;
 
+static constexpr int RETIRE = 3;  // spares and slots a thread retires at a time
+
 struct boot_smem {
-  uint16_t key[BOOT_WARPS][32];    // retire: segments completed by a warp ...
-  uint16_t count[BOOT_WARPS][32];  // ... and how many blocks of each
-  uint32_t nkeys[BOOT_WARPS];
+  // retire: (row, segment, blocks), one per segment a warp completed blocks of
+  unsigned long long done[RETIRE * BOOT_THREADS];
+  uint16_t before[RETIRE * BOOT_THREADS];  // of an entry's segment in earlier rows ...
+  uint16_t all[RETIRE * BOOT_THREADS];     // ... and in all
+  uint32_t ndone, nclose;
   uint32_t scan[BOOT_WARPS];
-  uint32_t total_free;
   uint16_t list[BOOT_THREADS];     // boot: the gathered segments of a tile
   uint32_t fast[GAL_MAX_TREES];    // the class lists no segment and its lock is free
   uint32_t first[GAL_MAX_TREES + 1];
-  uint32_t lone0;                  // class t0 takes segment 0 and finds it no more
+  uint32_t lone[GAL_MAX_TREES];    // the class would lose segment 0 (finds_lone_zero)
 };
 
 // Whether veb_find_random finds segment 0 when its tree lists nothing else: it
@@ -48,102 +51,143 @@ struct boot_smem {
 static __device__ bool finds_lone_zero(const state *s, uint32_t t) {
   if (s->policy == GAL_POLICY_LOWEST) return true;
   const uint64_t U = s->num_segments;
+  const bool pow2 = (U & (U - 1)) == 0;
   const uint64_t h1 = murmur64a_u64(0, s->seed + t);
   const uint64_t h2 = murmur64a_u64(0, h1);
   for (uint64_t a = 0; a < (uint64_t)VEB_ATTEMPTS; a++)
-    if ((h1 + a * h2) % U == 0) return true;
+    if ((pow2 ? (h1 + a * h2) & (U - 1) : (h1 + a * h2) % U) == 0) return true;
   return false;
 }
 // Segments that n blocks of class t take, `lone` of them from segment 0
 static __device__ uint32_t boot_segments(const state *s, uint32_t t, uint32_t n, uint32_t lone) {
   const uint32_t nb = blocks_in_segment(s, t);
+  const uint32_t shift = (uint32_t)__ffs(nb) - 1u;
   n -= lone;
   if (lone && n == 0) return 1;
-  return lone + (s->gather_ahead ? n / nb + 1u : (n + nb - 1u) / nb);
+  return lone + (s->gather_ahead ? (n >> shift) + 1u : (n + nb - 1u) >> shift);
 }
 
-// Threads i of a tile hold a block taken from a slot or spare (NOBLK: none), in
-// slot order: what k retire_block calls in that order do.
-static __device__ void retire_tile(const state *s, uint32_t blk, boot_smem &sm) {
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  bool home = false;
-  uint32_t seg = 0, nb = 1;
-  uint16_t tree = 0;
-  if (blk != NOBLK) {
-    const unsigned long long old = atomicAdd(mword_ptr(s, blk), (unsigned long long)SLICES_PER_BLOCK);
-    const uint32_t handed_out = (uint32_t)old;
-    if (handed_out < SLICES_PER_BLOCK) {
-      const uint32_t n = SLICES_PER_BLOCK - handed_out;
-      const uint32_t freed = atomicAdd(fctr_ptr(s, blk), n);
-      if (freed + n == SLICES_PER_BLOCK) {
-        st_rlx(fctr_ptr(s, blk), 0u);
-        seg = blk >> s->bps_shift;
-        tree = ld_rlx(&s->tree_ids[seg]);
-        home = tree < s->num_trees;
-        if (home) nb = blocks_in_segment(s, tree);
-        else set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_RETURN_BAD_TREE, blk, tree);
-      } else if (freed + n > SLICES_PER_BLOCK) {
-        set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OVERFLOW, blk, ((uint64_t)freed << 32) | n);
-      }
+// blk[k] of thread i is the (k * BOOT_THREADS + i)-th block of a tile, in the
+// order in which one thread would retire them (NOBLK: none): what as many
+// retire_block calls do.
+static __device__ void retire_tile(const state *s, const uint32_t (&blk)[RETIRE], boot_smem &sm) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, lt = lanemask_lt();
+  uint32_t handed_out[RETIRE], freed[RETIRE], seg[RETIRE], returned[RETIRE], same[RETIRE];
+  uint32_t entry[RETIRE];
+  uint16_t tree[RETIRE];
+  bool home[RETIRE];
+  if (threadIdx.x == 0) sm.ndone = 0;
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++)
+    handed_out[k] = blk[k] == NOBLK
+                        ? SLICES_PER_BLOCK
+                        : (uint32_t)atomicAdd(mword_ptr(s, blk[k]), (unsigned long long)SLICES_PER_BLOCK);
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++)
+    freed[k] = handed_out[k] < SLICES_PER_BLOCK ? atomicAdd(fctr_ptr(s, blk[k]), SLICES_PER_BLOCK - handed_out[k]) : 0u;
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++) {
+    const uint32_t n = SLICES_PER_BLOCK - min(handed_out[k], SLICES_PER_BLOCK);
+    home[k] = n && freed[k] + n == SLICES_PER_BLOCK;
+    seg[k] = home[k] ? blk[k] >> s->bps_shift : 0u;
+    tree[k] = home[k] ? ld_rlx(&s->tree_ids[seg[k]]) : FREE_TREE;
+    returned[k] = home[k] ? ld_rlx(&s->qfc[seg[k]]) : 0u;
+    if (n && freed[k] + n > SLICES_PER_BLOCK)
+      set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OVERFLOW, blk[k], ((uint64_t)freed[k] << 32) | n);
+  }
+  __syncthreads();  // ndone
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++) {
+    if (home[k]) st_rlx(fctr_ptr(s, blk[k]), 0u);
+    if (home[k] && tree[k] >= s->num_trees) {
+      set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_RETURN_BAD_TREE, blk[k], tree[k]);
+      home[k] = false;
+    }
+    // a warp's blocks by segment; the first lane of each segment speaks for it
+    same[k] = __match_any_sync(0xFFFFFFFFu, home[k] ? seg[k] : 0xFFFFFFFFu);
+    entry[k] = ~0u;
+    if (home[k] && (int)lane == __ffs(same[k]) - 1) {
+      entry[k] = atomicAdd(&sm.ndone, 1u);
+      sm.done[entry[k]] = (unsigned long long)(k * BOOT_WARPS + warp) << 32 | seg[k] << 16 | (uint32_t)__popc(same[k]);
     }
   }
-  const uint32_t returned = home ? ld_rlx(&s->qfc[seg]) : 0u;
-  // a warp's blocks by segment; the first lane of each segment speaks for it
-  const uint32_t same = __match_any_sync(0xFFFFFFFFu, home ? seg : 0xFFFFFFFFu);
-  const bool speaks = home && (int)lane == __ffs(same) - 1;
-  const uint32_t speakers = __ballot_sync(0xFFFFFFFFu, speaks);
-  if (speaks) {
-    const uint32_t at = (uint32_t)__popc(speakers & lanemask_lt());
-    sm.key[warp][at] = (uint16_t)seg;
-    sm.count[warp][at] = (uint16_t)__popc(same);
+  __syncthreads();  // also: every thread has read its segments' return positions
+  // a thread per entry, not per lane that made one: a hundred entries keep four
+  // warps at this, where every warp at its own took 15 us
+  const uint32_t ndone = sm.ndone;
+  for (uint32_t i = threadIdx.x; i < ndone; i += BOOT_THREADS) {
+    const unsigned long long own = sm.done[i];
+    uint32_t before = 0, all = 0;
+#pragma unroll 4
+    for (uint32_t e = 0; e < ndone; e++) {
+      const unsigned long long d = sm.done[e];
+      const uint32_t n = ((uint32_t)(d ^ own) >> 16) == 0 ? (uint32_t)d & 0xFFFFu : 0u;
+      all += n;
+      if ((d >> 32) < (own >> 32)) before += n;
+    }
+    sm.before[i] = (uint16_t)before;
+    sm.all[i] = (uint16_t)all;
   }
-  if (lane == 0) sm.nkeys[warp] = (uint32_t)__popc(speakers);
-  __syncthreads();  // also: every thread has read its segment's return position
-  uint32_t before = 0, all = 0;
-  if (speaks)
-    for (uint32_t w = 0; w < (uint32_t)BOOT_WARPS; w++)
-      for (uint32_t k = 0; k < sm.nkeys[w]; k++)
-        if (sm.key[w][k] == seg) {
-          all += sm.count[w][k];
-          if (w < warp) before += sm.count[w][k];
-        }
-  const bool closes = speaks && before == 0;  // the first warp of a segment settles its counters
-  before = __shfl_sync(0xFFFFFFFFu, before, __ffs(same) - 1);
-  if (home) {
-    const uint32_t live = (returned + before + (uint32_t)__popc(same & lanemask_lt())) & (nb - 1u);
-    st_rlx(s->queues + ((uint64_t)seg << s->bps_shift) + live, blk);
-    if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) veb_insert(sub_tree(s, tree), seg);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++) {
+    const uint32_t before = entry[k] != ~0u ? sm.before[entry[k]] : 0u;
+    const uint32_t rank = __shfl_sync(0xFFFFFFFFu, before, __ffs(same[k]) - 1) + (uint32_t)__popc(same[k] & lt);
+    if (home[k]) {
+      const uint32_t nb = blocks_in_segment(s, tree[k]);
+      const uint32_t live = (returned[k] + rank) & (nb - 1u);
+      st_rlx(s->queues + ((uint64_t)seg[k] << s->bps_shift) + live, blk[k]);
+      if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) veb_insert(sub_tree(s, tree[k]), seg[k]);
+    }
   }
+  if (threadIdx.x == 0) sm.nclose = 0;
   fence_acq_rel();
+  __syncthreads();  // also: done is read
+  // the first of a segment settles its counters: listed, so that every thread
+  // has one (a release is a chain of some ten round trips)
+#pragma unroll
+  for (int k = 0; k < RETIRE; k++)
+    if (entry[k] != ~0u && sm.before[entry[k]] == 0)
+      sm.done[atomicAdd(&sm.nclose, 1u)] = (unsigned long long)tree[k] << 32 | seg[k] << 16 | sm.all[entry[k]];
   __syncthreads();
-  if (closes) {
-    atomicAdd(&s->qfc[seg], all);
-    atomicAdd(&s->fqfc[seg], all);
-    const unsigned long long old = atomicAdd(&s->act[seg], (unsigned long long)all);
-    if (act_count(old) + (int32_t)all == (int32_t)nb - 1) release_segment(s, seg, tree, act_gen(old), nb);
+  for (uint32_t e = threadIdx.x; e < sm.nclose; e += BOOT_THREADS) {
+    const unsigned long long d = sm.done[e];
+    const uint32_t t = (uint32_t)(d >> 32), g = (uint32_t)d >> 16, n = (uint32_t)d & 0xFFFFu;
+    const uint32_t nb = blocks_in_segment(s, t);
+    atomicAdd(&s->qfc[g], n);
+    atomicAdd(&s->fqfc[g], n);
+    const unsigned long long old = atomicAdd(&s->act[g], (unsigned long long)n);
+    if (act_count(old) + (int32_t)n == (int32_t)nb - 1) release_segment(s, g, t, act_gen(old), nb);
   }
   __syncthreads();
 }
 
-// every block in the n words at `from`, which are left empty
-static __device__ void retire_all(const state *s, uint32_t *from, uint32_t n, boot_smem &sm) {
-  for (uint32_t base = 0; base < n; base += BOOT_THREADS) {
-    const uint32_t i = base + threadIdx.x;
-    retire_tile(s, i < n ? atomicExch(from + i, NOBLK) : NOBLK, sm);
+// every spare and pinned block, spares first; the words are left empty
+static __device__ void retire_all(const state *s, boot_smem &sm) {
+  const uint32_t n = s->total_slots;
+  for (uint32_t base = 0; base < 2 * n; base += RETIRE * BOOT_THREADS) {
+    uint32_t blk[RETIRE];
+#pragma unroll
+    for (int k = 0; k < RETIRE; k++) {
+      const uint32_t i = base + k * BOOT_THREADS + threadIdx.x;
+      blk[k] = i < n ? atomicExch(s->spares + i, NOBLK) : i < 2 * n ? atomicExch(s->slots + (i - n), NOBLK) : NOBLK;
+    }
+    retire_tile(s, blk, sm);
   }
 }
 
-// one fresh segment of class t, its first `taken` blocks given to the slots
-// from `slot` on: what setup_segment and `taken` get_block calls leave (full warp)
-static __device__ void boot_segment(const state *s, uint32_t seg, uint32_t t, uint32_t slot, uint32_t taken) {
+// A fresh segment of class t, its first `taken` blocks given to the slots from
+// `slot` on: what setup_segment and `taken` get_block calls leave, in two steps
+// with a fence between them (full warp; false: listed free, yet owned).
+static __device__ bool boot_segment(const state *s, uint32_t seg, uint32_t t, uint32_t slot, uint32_t taken) {
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t nb = blocks_in_segment(s, t);
-  if (ld_rlx(&s->tree_ids[seg]) != FREE_TREE) {  // listed free, yet owned
+  if (ld_rlx(&s->tree_ids[seg]) != FREE_TREE) {
     if (lane == 0) {
       set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
       if (taken) set_error(s, GAL_DEV_ERR_BOOT);
     }
-    return;
+    return false;
   }
   const uint32_t blk0 = seg << s->bps_shift;
   for (uint32_t i = lane; i < nb; i += 32) st_rlx(s->queues + blk0 + i, NOBLK);
@@ -151,18 +195,17 @@ static __device__ void boot_segment(const state *s, uint32_t seg, uint32_t t, ui
     st_rlx(mword_ptr(s, blk0 + i), (unsigned long long)t << 32);
     st_rlx(s->slots + s->slot_base[t] + slot + i, blk0 + i);
   }
-  __syncwarp();
   if (lane == 0) {
-    const uint32_t high = (uint32_t)(ld_rlx(&s->act[seg]) >> 32);
-    const uint32_t next = (((high >> 8) + 1u) << 8) | t;
-    s->tree_ids[seg] = (uint16_t)t;
+    st_rlx(&s->tree_ids[seg], (uint16_t)t);
     st_rlx(&s->qc[seg], taken);
     st_rlx(&s->qfc[seg], 0u);
     st_rlx(&s->fqfc[seg], 0u);
-    fence_acq_rel();
-    atomicAdd(&s->act[seg], ((unsigned long long)(next - high) << 32) + nb - taken);
-    if (taken < nb) veb_insert(sub_tree(s, t), seg);
   }
+  return true;
+}
+static __device__ void boot_open(const state *s, uint32_t seg, uint32_t t, uint32_t taken) {
+  atomicAdd(&s->act[seg], ((unsigned long long)(t + 1u) << 32) + blocks_in_segment(s, t) - taken);  // see setup_open
+  if (taken < blocks_in_segment(s, t)) veb_insert(sub_tree(s, t), seg);
 }
 
 // Boots every slot (all empty) in the one-thread order.  One CTA of
@@ -172,23 +215,32 @@ static __device__ void boot_all(const state *s, boot_smem &sm) {
   const veb_ref segs = seg_tree(s);
   const uint32_t nwords = s->veb.nwords[s->veb.layers - 1];  // at most 1,024: 65,532 segments
   uint64_t *bottom = veb_bottom(segs);
+  if (threadIdx.x >= 32 && threadIdx.x < 32 + T) {
+    const uint32_t t = threadIdx.x - 32;
+    sm.lone[t] = blocks_in_segment(s, t) > 1 && !finds_lone_zero(s, t);
+  }
   if (threadIdx.x < T)
     sm.fast[threadIdx.x] = ld_rlx(sub_tree(s, threadIdx.x).w) == 0 && ld_rlx(s->locks + threadIdx.x * LOCK_STRIDE) == 0;
   __syncthreads();
   for (uint32_t t0 = 0; t0 < T;) {
     uint32_t t1 = t0;  // classes [t0, t1) are booted together
     while (t1 < T && sm.fast[t1]) t1++;
-    if (threadIdx.x == 0) {
-      uint32_t at = 0;
-      sm.lone0 = (ld_rlx(bottom) & 1ull) && blocks_in_segment(s, t0) > 1 && !finds_lone_zero(s, t0);
-      for (uint32_t t = t0; t < t1; t++) {
-        sm.first[t] = at;
-        at += boot_segments(s, t, s->slot_count[t], t == t0 ? sm.lone0 : 0u);
-      }
-      sm.first[t1] = at;
-    }
     // free segments below this thread's word
     const uint64_t word = t1 > t0 && threadIdx.x < nwords ? ld_rlx(bottom + threadIdx.x) : 0ull;
+    if (warp == 0) {  // the classes' first gathered segments: lane t's class, summed in order
+      const bool mine = lane >= t0 && lane < t1;
+      const uint32_t lone0 = (uint32_t)(__shfl_sync(0xFFFFFFFFu, word, 0) & 1ull) && t1 > t0 ? sm.lone[t0] : 0u;
+      const uint32_t n = mine ? boot_segments(s, lane, s->slot_count[lane], lane == t0 ? lone0 : 0u) : 0u;
+      uint32_t upto = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+        if ((int)lane >= o) upto += v;
+      }
+      if (mine) sm.first[lane] = upto - n;
+      if (mine && lane == t1 - 1) sm.first[t1] = upto;
+      if (lane == 0) sm.lone[t0] = lone0;
+    }
     uint32_t below = (uint32_t)__popcll(word);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -215,10 +267,15 @@ static __device__ void boot_all(const state *s, boot_smem &sm) {
       continue;
     }
     uint64_t taken = word;  // the bits of `word` among the first `total` free segments
-    if (below >= total) taken = 0;
-    else
-      for (uint32_t n = below + (uint32_t)__popcll(word); n > total; n--)
-        taken &= ~(1ull << (63 - __clzll((long long)taken)));
+    if (below >= total) {
+      taken = 0;
+    } else if (below + (uint32_t)__popcll(word) > total) {  // its lowest total - below
+      uint32_t end = 0;  // the most bits [0, end) that hold no more
+#pragma unroll
+      for (uint32_t step = 32; step; step >>= 1)
+        if ((uint32_t)__popcll(word & bitmask((int)(end + step))) <= total - below) end += step;
+      taken = word & bitmask((int)end);
+    }
     if (taken) {
       amo_and(bottom + threadIdx.x, ~taken);
       if (taken == word) {  // emptied: off the summaries, as veb_remove does
@@ -236,15 +293,30 @@ static __device__ void boot_all(const state *s, boot_smem &sm) {
         if (r >= base && r - base < (uint32_t)BOOT_THREADS)
           sm.list[r - base] = (uint16_t)(threadIdx.x * 64u + (uint32_t)__ffsll((long long)b) - 1u);
       __syncthreads();
-      for (uint32_t e = warp; e < (uint32_t)BOOT_THREADS && base + e < total; e += BOOT_WARPS) {
-        uint32_t t = t0;
+      // entry e of the tile: its class, its blocks, the first of its slots
+      auto entry = [&](uint32_t e, uint32_t &t, uint32_t &slot) {
+        t = t0;
         while (base + e >= sm.first[t + 1]) t++;
         const uint32_t n = s->slot_count[t], j = base + e - sm.first[t];
-        const uint32_t lone = t == t0 ? sm.lone0 : 0u;
+        const uint32_t lone = t == t0 ? sm.lone[t0] : 0u;
         // blocks of the class's segments before this one, and of this one
-        const uint32_t slot = lone && j ? ((j - 1u) << (s->bps_shift - t)) + 1u : j << (s->bps_shift - t);
+        slot = lone && j ? ((j - 1u) << (s->bps_shift - t)) + 1u : j << (s->bps_shift - t);
         const uint32_t most = lone && !j ? 1u : blocks_in_segment(s, t);
-        boot_segment(s, sm.list[e], t, slot, min(most, n - min(n, slot)));
+        return min(most, n - min(n, slot));
+      };
+      uint32_t mine = 0;  // the warp's entries that were set up
+      for (uint32_t e = warp, k = 0; e < (uint32_t)BOOT_THREADS && base + e < total; e += BOOT_WARPS, k++) {
+        uint32_t t, slot;
+        const uint32_t taken = entry(e, t, slot);
+        if (boot_segment(s, sm.list[e], t, slot, taken)) mine |= 1u << k;
+      }
+      fence_acq_rel();
+      __syncwarp();
+      if ((mine >> lane) & 1u) {  // lane k opens the warp's k-th
+        const uint32_t e = warp + lane * BOOT_WARPS;
+        uint32_t t, slot;
+        const uint32_t taken = entry(e, t, slot);
+        boot_open(s, sm.list[e], t, taken);
       }
       __syncthreads();
     }

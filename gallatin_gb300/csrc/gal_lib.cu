@@ -87,8 +87,7 @@ __global__ void __launch_bounds__(gal::BOOT_THREADS) k_boot(const gal::state *s)
 // again in the one-thread order.
 __global__ void __launch_bounds__(gal::BOOT_THREADS) k_trim(const gal::state *s) {
   __shared__ gal::boot_smem sm;
-  gal::retire_all(s, s->spares, s->total_slots, sm);
-  gal::retire_all(s, s->slots, s->total_slots, sm);
+  gal::retire_all(s, sm);
   // segments of a class none of whose blocks is out (those gathered ahead when
   // a class took the last block of its previous segment) go back too
   for (uint64_t seg = threadIdx.x; seg < s->num_segments; seg += blockDim.x) {
@@ -125,12 +124,10 @@ __global__ void k_stats(const gal::state *s, gal_stats *out) {
   __syncthreads();
   const uint32_t bottom = s->veb.layers - 1;
   const uint64_t nw = s->veb.nwords[bottom];
-  for (uint64_t w = threadIdx.x; w < nw; w += blockDim.x) {
-    atomicAdd(&acc[0], (unsigned long long)__popcll(s->seg_tree[s->veb.off[bottom] + w]));
-    for (uint32_t t = 0; t < T; t++)
-      atomicAdd(&acc[3 + GAL_MAX_TREES + t],
-                (unsigned long long)__popcll(
-                    s->sub_trees[(uint64_t)t * s->veb.words + s->veb.off[bottom] + w]));
+  for (uint64_t i = threadIdx.x; i < nw * (T + 1); i += blockDim.x) {  // the segment tree, then the classes'
+    const uint64_t t = i / nw, w = s->veb.off[bottom] + i % nw;
+    const uint64_t *tree = t ? s->sub_trees + (t - 1) * s->veb.words : s->seg_tree;
+    atomicAdd(&acc[t ? 2 + GAL_MAX_TREES + t : 0], (unsigned long long)__popcll(tree[w]));
   }
   for (uint64_t g = threadIdx.x; g < s->num_segments; g += blockDim.x) {
     uint16_t id = s->tree_ids[g];
