@@ -245,9 +245,11 @@ __global__ void __launch_bounds__(MALLOC_THREADS, 4)
 // 253; 4 Mi mixed, one slot per SM: 67 against 98).  K is the smallest that fits
 // the list in one wave of two CTAs per SM: larger chunks claim less often,
 // smaller ones start more SMs (262,144 mixed: 17, 11, 11, 21 us at K = 1, 2, 4, 8).
+// Lists of several waves gain from a third CTA per SM (40 registers; 4 Mi mixed:
+// 70 -> 64 us), one wave does not.
 constexpr uint64_t BULK_FROM = 1u << 15;
 template <int K>
-__global__ void __launch_bounds__(gal::BULK_THREADS, 2)
+__global__ void __launch_bounds__(gal::BULK_THREADS, K == 8 ? 3 : 2)
     k_malloc_bulk(const gal::state *s, const uint64_t *sizes, uint64_t n, void **out) {
   __shared__ gal::bulk_smem sm;
   gal::bulk_malloc<K>(s, sizes, n, (uint64_t)blockIdx.x * (K * gal::BULK_THREADS), out, sm);
