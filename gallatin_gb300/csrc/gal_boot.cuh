@@ -5,8 +5,9 @@
 // order fixes which block every slot gets.  With one slot per SM in nine
 // classes it is 1,368 block requests in a chain: 11.9 ms for a trim at one slot
 // per SM (21.3 ms before the requests themselves were made cheaper).  Here the
-// same end state is computed in parallel by 1,024 threads; bound by the dozen
-// dependent round trips of its phases.
+// same end state is computed in parallel by 1,024 threads in 42 us; bound by
+// the thirty dependent round trips of its phases (retiring 14, releases 10,
+// booting 18).
 //
 //   * Blocks of one segment must come home in slot order (their ring entries);
 //     blocks of different segments have nothing in common but bits of the

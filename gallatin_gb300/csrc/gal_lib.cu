@@ -225,9 +225,8 @@ __global__ void k_replay_warp(const gal::state *s, const uint64_t *steps, uint64
   }
 }
 
-// One thread per request, warp teams claiming with one atomicAdd per team on
-// their SM's pinned block (gal::malloc): the per-thread call, and the batched
-// call's short lists.  Compiled for four CTAs of 256 threads per SM (64
+// Short lists: one thread per request, warp teams claiming with one atomicAdd
+// per team on their SM's pinned block (gal::malloc).  Compiled for four CTAs of 256 threads per SM (64
 // registers); with the registers it would take (96, two CTAs) 1 Mi mixed requests
 // took 44 us instead of 35.
 constexpr int MALLOC_THREADS = 256;
@@ -802,13 +801,7 @@ int gal_replay_warp_trace(gal_handle *h, const uint64_t *steps, uint64_t nsteps,
 }
 
 int gal_malloc_per_thread(gal_handle *h, const uint64_t *sizes, uint64_t n, void **out, void *stream) {
-  if (!h || (n && (!sizes || !out))) return GAL_ERR_ARGS;
-  if (!n) return GAL_OK;
-  gal_device_guard on_dev(h->device);  // the handle's device, whatever the caller's current one
-  CUDA_TRY(on_dev.err);
-  k_malloc_threads<<<grid_for(n, MALLOC_THREADS), MALLOC_THREADS, 0, (cudaStream_t)stream>>>(h->d_state, sizes, n, out);
-  CUDA_TRY(cudaGetLastError());
-  return GAL_OK;
+  return gal_malloc_batched(h, sizes, n, out, stream);
 }
 
 int gal_free_per_thread(gal_handle *h, void *const *ptrs, uint64_t n, void *stream) {
