@@ -16,7 +16,8 @@
 //   reinsert the deleted keys; look up every key (all present, right value);
 //   count the live pairs of every table; free every node and bucket array.
 // Node allocation inside an insert: per thread under the bucket lock (plain
-// form), or CTA-aggregated (batched form: every thread holds a node ready, and
+// form; the CTA keeps a copy of its pinned block, which spares the claim a round
+// trip), or CTA-aggregated (batched form: every thread holds a node ready, and
 // the threads that used theirs ask for the next together through
 // gal::cta_malloc; a node left over at the end is freed).
 //
@@ -28,8 +29,11 @@
 // time.  Now a lane tries its lock once per turn; the lanes that got theirs
 // search, allocate, change and release together and fetch their next op, the
 // others (one in twenty, so most warps have one) keep theirs for the next turn.
+// What bounds an insert now is its three or four scattered 32-byte sectors, which
+// it writes to L2: keeping the lock to the next turn, so that one fence serves
+// the release and the next acquire, gave nothing (0.46 and 0.47 ms).
 // 8.6 M pairs in 128 tables, one slot per SM, in ms, before and now: insert 2.22,
-// 0.68; delete 1.47, 0.33; lookups 0.43 + 0.71, 0.16 + 0.20; reinsert 1.70, 0.49;
+// 0.46; delete 1.47, 0.34; lookups 0.43 + 0.71, 0.16 + 0.18; reinsert 1.70, 0.37;
 // teardown 0.81, 0.11.
 //
 // Keys: a bijective 64-bit mix of (table << 32 | index) so the keys of a table
@@ -81,7 +85,7 @@ struct node {
 };
 static_assert(sizeof(node) == 128, "one 128 B slice per node");
 
-struct table_desc {
+struct alignas(16) table_desc {
   unsigned long long *heads;
   uint64_t nbuckets;  // a power of two
 };
@@ -193,62 +197,81 @@ __device__ __forceinline__ probe find(unsigned long long head, uint64_t key, uin
   return r;
 }
 
+// A thread's op between its turns and across a turn's malloc, and its counts,
+// in shared memory and read back where they are wanted: held in registers they
+// were spilled, and a spill is written through to L2 (some 20 M of the 47 M write
+// requests of 8.6 M inserts; 260 bytes of spills a thread, now 42).  With the
+// descriptors read as constants and the CTA's copy of its pinned block: insert
+// 0.71 -> 0.46 ms, reinsert 0.48 -> 0.37, aggregated form 0.70 -> 0.54.
+struct pending {
+  volatile uint64_t i[TBT];  // the next op
+  volatile uint64_t key[TBT], hp[TBT], head[TBT];
+  volatile uint32_t tag[TBT], waited[TBT];
+  volatile uint32_t pairs[TBT], nodes[TBT];  // inserted and allocated, or deleted and freed
+};
+
 // One turn of an insert, by a whole warp together: true when the op is done.
 // A bucket without room takes `spare`, when there is one (null afterwards);
 // MALLOC: else a node from the allocator under the lock.  The warp meets before
 // the malloc, whose teams are the lanes that call together: lanes that left the
-// search one by one claimed one by one.
+// search one by one claimed one by one.  The others have written their pairs by
+// then, and the release at the end finds those writes done.
 template <bool MALLOC>
-__device__ __forceinline__ bool insert_turn(const gal::state *s, unsigned long long *hp, bool go, uint64_t key,
-                                            uint32_t tag, node *&spare, counters &lc) {
-  unsigned long long head = 0;
-  const bool mine = go && try_lock_bucket(hp, head);
-  probe p{};
-  if (mine) p = find(head, key, tag);
-  const bool full = mine && !p.n;
-  __syncwarp();
-  if (MALLOC) {
-    if (full) {
-      spare = (node *)gal::malloc(s, sizeof(node));
-      if (spare) count(lc, S_NODES);
+__device__ __forceinline__ bool insert_turn(const gal::state *s, pending &op, bool go, node *&spare,
+                                            gal::slot_cache &cache, unsigned long long *stats) {
+  const uint32_t me = threadIdx.x;
+  bool mine = false, full = false;
+  if (go) {
+    unsigned long long head;
+    mine = try_lock_bucket((unsigned long long *)op.hp[me], head);
+    if (mine) {
+      op.head[me] = head;
+      const uint64_t key = op.key[me];
+      const uint32_t tag = op.tag[me];
+      const probe p = find(head, key, tag);
+      full = !p.n;
+      if (p.n) {
+        p.n->pair[p.slot] = make_ulonglong2(key, table_val(key));
+        if (!p.found) {
+          p.n->meta = with_place(p.meta, p.slot, tag);
+          op.pairs[me] += 1u;
+        }
+      }
     }
-    __syncwarp();
   }
-  if (!mine) return false;
-  node *n = p.n;
+  __syncwarp();
   if (full) {
-    n = spare;
+    node *n = spare;
+    if (MALLOC) n = (node *)gal::malloc_cached(s, sizeof(node), cache);
     spare = nullptr;
     if (n) {
-      n->next = head;
-      head = (unsigned long long)n;
+      const uint64_t key = op.key[me];
+      *(ulonglong2 *)n = make_ulonglong2(op.head[me], with_place(0, 0, op.tag[me]));
+      n->pair[0] = make_ulonglong2(key, table_val(key));
+      op.head[me] = (uint64_t)n;
+      op.pairs[me] += 1u;
+      if (MALLOC) op.nodes[me] += 1u;
     } else {
-      count(lc, S_MFAIL);
+      count_global(stats, S_MFAIL);
     }
   }
-  if (n) {
-    n->pair[p.slot] = make_ulonglong2(key, table_val(key));
-    if (!p.found) {
-      n->meta = with_place(p.meta, p.slot, tag);
-      count(lc, S_INSERTED);
-    }
-  }
-  unlock_bucket(hp, head);
-  return true;
+  __syncwarp();
+  if (mine) unlock_bucket((unsigned long long *)op.hp[me], op.head[me]);
+  return mine;
 }
 
-__device__ __forceinline__ bool delete_turn(const gal::state *s, unsigned long long *hp, bool go, uint64_t key,
-                                            uint32_t tag, counters &lc) {
+__device__ __forceinline__ bool delete_turn(const gal::state *s, pending &op, bool go) {
+  const uint32_t me = threadIdx.x;
   unsigned long long head = 0;
-  const bool mine = go && try_lock_bucket(hp, head);
+  const bool mine = go && try_lock_bucket((unsigned long long *)op.hp[me], head);
   probe p{};
-  if (mine) p = find(head, key, tag);
+  if (mine) p = find(head, op.key[me], op.tag[me]);
   __syncwarp();
   node *dead = nullptr;
   if (mine) {
     if (p.found) {
       const unsigned long long meta = p.meta & ~(1ull << p.slot);
-      count(lc, S_DELETED);
+      op.pairs[me] += 1u;
       if ((uint32_t)meta & FULL) {
         p.n->meta = meta;
       } else {  // unlink and free the empty node
@@ -257,12 +280,12 @@ __device__ __forceinline__ bool delete_turn(const gal::state *s, unsigned long l
         dead = p.n;
       }
     }
-    unlock_bucket(hp, head);
+    unlock_bucket((unsigned long long *)op.hp[me], head);
   }
   __syncwarp();
   if (dead) {
     gal::free_sized(s, dead, sizeof(node));
-    count(lc, S_NODES_FREED);
+    op.nodes[me] += 1u;
   }
   return mine;
 }
@@ -280,8 +303,9 @@ enum : int { PH_INSERT = 0, PH_DELETE = 1, PH_CHECK_DELETED = 2, PH_REINSERT = 3
 
 // One phase; BATCHED: nodes of an insert phase come from gal::cta_malloc.
 // Registers for five CTAs per SM where the phase allocates, although the
-// allocator's rare paths then spill (insert 0.88, 0.84, 0.81 ms at 3, 4 and 5
-// CTAs), and for six where it only frees or reads.
+// allocator's rare paths then spill (insert at 4, 5 and 6 CTAs: 0.49, 0.46 and
+// 0.45 ms with a slot per SM, 0.17, 0.17 and 0.20 for 1.7 M pairs with shared
+// slots), and for six where it only frees or reads.
 template <int PHASE, bool BATCHED>
 __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSERT ? 5 : 6)
     k_tables_phase(const gal::state *s, uint32_t ntab, const uint64_t *offsets, const table_desc *desc, uint64_t seed,
@@ -290,65 +314,83 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
   constexpr bool LOCKS = INSERTS || PHASE == PH_DELETE;
   extern __shared__ uint64_t off[];  // [ntab + 1]
   __shared__ gal::cta_claim_smem cm;
+  __shared__ gal::slot_cache cache;
+  __shared__ pending op;
   for (uint32_t i = threadIdx.x; i <= ntab; i += blockDim.x) off[i] = offsets[i];
   if (INSERTS && BATCHED) gal::cta_claim_init(cm);
+  if (INSERTS && !BATCHED) gal::slot_cache_init(cache);
   __syncthreads();
   counters lc = {};
   const uint64_t total = off[ntab];
   const uint64_t stride = (uint64_t)gridDim.x * TBT;
-  uint64_t i = (uint64_t)blockIdx.x * TBT + threadIdx.x;  // this thread's next op
-  unsigned long long *hp = nullptr;
-  uint64_t key = 0;
-  uint32_t tag = 0, waited = 0;
-  bool go = false, coin = false;
-  // the op at i, if it is one of the phase's (half are not where the coin selects)
-  auto fetch = [&]() {
+  const uint32_t me = threadIdx.x;
+  // op i of the phase, if it is one of its own (half are not where the coin selects)
+  auto fetch = [&](uint64_t i, uint64_t &key, uint32_t &tag, unsigned long long *&hp, bool &coin) {
     const uint32_t t = table_of(off, ntab, i);
-    const table_desc d = desc[t];
+    const ulonglong2 w = __ldg((const ulonglong2 *)desc + t);  // (in lines that an acquire leaves in L1)
+    const table_desc d{(unsigned long long *)w.x, w.y};
     key = table_key(t, i - off[t], seed);
     coin = table_coin(key);
     const uint64_t hash = table_hash(key);
     tag = tag_of(hash);
     hp = d.heads + bucket_of(hash, d.nbuckets);
-    go = d.heads && (PHASE == PH_INSERT || !LOCKS || coin);
-    waited = 0;
-    i += stride;
+    return d.heads && (PHASE == PH_INSERT || !LOCKS || coin);
   };
+  uint64_t key;
+  uint32_t tag;
+  unsigned long long *hp;
+  bool coin;
   if (LOCKS) {
     constexpr int FETCHES = PHASE == PH_INSERT ? 1 : 3;  // seven lanes in eight have an op then
+    op.i[me] = (uint64_t)blockIdx.x * TBT + me;
+    op.pairs[me] = 0;
+    op.nodes[me] = 0;
+    bool go = false;
     node *spare = nullptr;
     for (;;) {
+      bool more = go || op.i[me] < total;
 #pragma unroll 1
-      for (int f = 0; f < FETCHES && __any_sync(0xFFFFFFFFu, !go && i < total); f++)
-        if (!go && i < total) fetch();
-      const bool more = go || i < total;
+      for (int f = 0; f < FETCHES && __any_sync(0xFFFFFFFFu, !go && more); f++)
+        if (!go && more) {
+          const uint64_t i = op.i[me];
+          go = fetch(i, key, tag, hp, coin);
+          op.key[me] = key;
+          op.tag[me] = tag;
+          op.hp[me] = (uint64_t)hp;
+          op.waited[me] = 0;
+          op.i[me] = i + stride;
+          more = go || i + stride < total;
+        }
       if (INSERTS && BATCHED) {
         if (!__syncthreads_or(more)) break;
         node *n = (node *)gal::cta_malloc(s, sizeof(node), go && !spare, cm);
         if (n) {
           spare = n;
-          count(lc, S_NODES);
+          op.nodes[me] += 1u;
         }
       } else if (!__any_sync(0xFFFFFFFFu, more)) {
         break;
       }
-      const bool done = INSERTS ? insert_turn<!BATCHED>(s, hp, go, key, tag, spare, lc)
-                                : delete_turn(s, hp, go, key, tag, lc);
+      const bool done = INSERTS ? insert_turn<!BATCHED>(s, op, go, spare, cache, stats) : delete_turn(s, op, go);
       if (done) go = false;
-      if (go && ++waited > s->spin_limit) {
-        count(lc, S_LOCK);
-        go = false;
+      if (go) {
+        const uint32_t w = op.waited[me] + 1u;
+        op.waited[me] = w;
+        if (w > gal::cfield(s->spin_limit)) {
+          count_global(stats, S_LOCK);
+          go = false;
+        }
       }
     }
     if (spare) {  // held ready to the end
       gal::free_sized(s, spare, sizeof(node));
       count(lc, S_SPARE);
     }
+    count(lc, INSERTS ? S_INSERTED : S_DELETED, op.pairs[me]);
+    count(lc, INSERTS ? S_NODES : S_NODES_FREED, op.nodes[me]);
   } else {
-    while (i < total) {
-      fetch();
-      if (go) lookup_op(hp, key, tag, PHASE == PH_CHECK_ALL || !coin, lc);
-    }
+    for (uint64_t i = (uint64_t)blockIdx.x * TBT + me; i < total; i += stride)
+      if (fetch(i, key, tag, hp, coin)) lookup_op(hp, key, tag, PHASE == PH_CHECK_ALL || !coin, lc);
     __syncwarp();
   }
   flush(stats, lc);  // whole warps
