@@ -33,7 +33,7 @@
 // it writes to L2: keeping the lock to the next turn, so that one fence serves
 // the release and the next acquire, gave nothing (0.46 and 0.47 ms).
 // 8.6 M pairs in 128 tables, one slot per SM, in ms, before and now: insert 2.22,
-// 0.46; delete 1.47, 0.34; lookups 0.43 + 0.71, 0.16 + 0.18; reinsert 1.70, 0.37;
+// 0.46; delete 1.47, 0.22; lookups 0.43 + 0.71, 0.15 + 0.16; reinsert 1.70, 0.27;
 // teardown 0.81, 0.11.
 //
 // Keys: a bijective 64-bit mix of (table << 32 | index) so the keys of a table
@@ -176,11 +176,18 @@ struct probe {
   unsigned long long next;
   unsigned long long val;
 };
+// A node's link and meta; its whole line comes to L2 with them, as one of its
+// pairs is read or written next (4 % of a delete, 6 % of a reinsert).
+__device__ __forceinline__ ulonglong2 ld_node(const node *n) {
+  ulonglong2 v;
+  asm volatile("ld.global.cg.L2::128B.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(n) : "memory");
+  return v;
+}
 __device__ __forceinline__ probe find(unsigned long long head, uint64_t key, uint32_t tag) {
   probe r{};
   node *prev = nullptr;
   for (node *n = (node *)(head & ~1ull); n;) {
-    const ulonglong2 w = __ldcg((const ulonglong2 *)n);  // link, meta
+    const ulonglong2 w = ld_node(n);
     for (uint32_t m = tagged(w.y, tag); m; m &= m - 1u) {
       const uint32_t k = (uint32_t)__ffs(m) - 1u;
       const ulonglong2 kv = __ldcg(&n->pair[k]);
@@ -203,21 +210,29 @@ __device__ __forceinline__ probe find(unsigned long long head, uint64_t key, uin
 // requests of 8.6 M inserts; 260 bytes of spills a thread, now 42).  With the
 // descriptors read as constants and the CTA's copy of its pinned block: insert
 // 0.71 -> 0.46 ms, reinsert 0.48 -> 0.37, aggregated form 0.70 -> 0.54.
+// Where the coin selects half of the ops a warp looks through 32 at a time and
+// keeps those of the phase in a ring from which its free lanes serve themselves:
+// each lane looking for itself (up to three ops a turn, for the few lanes that
+// were free) was 8,400 of a delete's 20,600 cycles a turn.  Delete 0.34 -> 0.22,
+// reinsert 0.37 -> 0.27.  Where every op is the phase's a lane takes its own
+// (insert 0.46 ms, 0.50 through a ring).
+template <bool RING>
 struct pending {
-  volatile uint64_t i[TBT];  // the next op
   volatile uint64_t key[TBT], hp[TBT], head[TBT];
   volatile uint32_t tag[TBT], waited[TBT];
   volatile uint32_t pairs[TBT], nodes[TBT];  // inserted and allocated, or deleted and freed
+  volatile uint64_t i[RING ? 1 : TBT];               // the lane's next op, or
+  volatile uint32_t ready[RING ? 2 * TBT : 1], ready_table[RING ? 2 * TBT : 1];  // the ops that no lane has
+  // taken yet, a ring of 64 for each warp: index in the table, table
 };
-
 // One turn of an insert, by a whole warp together: true when the op is done.
 // A bucket without room takes `spare`, when there is one (null afterwards);
 // MALLOC: else a node from the allocator under the lock.  The warp meets before
 // the malloc, whose teams are the lanes that call together: lanes that left the
 // search one by one claimed one by one.  The others have written their pairs by
 // then, and the release at the end finds those writes done.
-template <bool MALLOC>
-__device__ __forceinline__ bool insert_turn(const gal::state *s, pending &op, bool go, node *&spare,
+template <bool MALLOC, bool RING>
+__device__ __forceinline__ bool insert_turn(const gal::state *s, pending<RING> &op, bool go, node *&spare,
                                             gal::slot_cache &cache, unsigned long long *stats) {
   const uint32_t me = threadIdx.x;
   bool mine = false, full = false;
@@ -260,7 +275,8 @@ __device__ __forceinline__ bool insert_turn(const gal::state *s, pending &op, bo
   return mine;
 }
 
-__device__ __forceinline__ bool delete_turn(const gal::state *s, pending &op, bool go) {
+template <bool RING>
+__device__ __forceinline__ bool delete_turn(const gal::state *s, pending<RING> &op, bool go) {
   const uint32_t me = threadIdx.x;
   unsigned long long head = 0;
   const bool mine = go && try_lock_bucket((unsigned long long *)op.hp[me], head);
@@ -315,52 +331,83 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
   extern __shared__ uint64_t off[];  // [ntab + 1]
   __shared__ gal::cta_claim_smem cm;
   __shared__ gal::slot_cache cache;
-  __shared__ pending op;
+  constexpr bool RING = PHASE == PH_DELETE || PHASE == PH_REINSERT;
+  __shared__ pending<RING> op;
   for (uint32_t i = threadIdx.x; i <= ntab; i += blockDim.x) off[i] = offsets[i];
   if (INSERTS && BATCHED) gal::cta_claim_init(cm);
   if (INSERTS && !BATCHED) gal::slot_cache_init(cache);
   __syncthreads();
   counters lc = {};
   const uint64_t total = off[ntab];
-  const uint64_t stride = (uint64_t)gridDim.x * TBT;
   const uint32_t me = threadIdx.x;
-  // op i of the phase, if it is one of its own (half are not where the coin selects)
-  auto fetch = [&](uint64_t i, uint64_t &key, uint32_t &tag, unsigned long long *&hp, bool &coin) {
-    const uint32_t t = table_of(off, ntab, i);
+  auto place = [&](uint32_t t, uint64_t key, uint32_t &tag) {
     const ulonglong2 w = __ldg((const ulonglong2 *)desc + t);  // (in lines that an acquire leaves in L1)
-    const table_desc d{(unsigned long long *)w.x, w.y};
-    key = table_key(t, i - off[t], seed);
-    coin = table_coin(key);
     const uint64_t hash = table_hash(key);
     tag = tag_of(hash);
-    hp = d.heads + bucket_of(hash, d.nbuckets);
-    return d.heads && (PHASE == PH_INSERT || !LOCKS || coin);
+    return (unsigned long long *)w.x + bucket_of(hash, w.y);
   };
-  uint64_t key;
-  uint32_t tag;
-  unsigned long long *hp;
-  bool coin;
   if (LOCKS) {
-    constexpr int FETCHES = PHASE == PH_INSERT ? 1 : 3;  // seven lanes in eight have an op then
-    op.i[me] = (uint64_t)blockIdx.x * TBT + me;
+    const uint32_t lane = me & 31u, warp = me / 32u, lt = gal::lanemask_lt();
+    // RING: 32 ops at a time for the warp, the next at `at`.  Else one for the lane.
+    uint64_t at = ((uint64_t)blockIdx.x * TBT + me) - (RING ? lane : 0u);
+    if (!RING) op.i[me] = at;
+    uint32_t first = 0, have = 0;  // of the warp's ring
     op.pairs[me] = 0;
     op.nodes[me] = 0;
     bool go = false;
     node *spare = nullptr;
     for (;;) {
-      bool more = go || op.i[me] < total;
-#pragma unroll 1
-      for (int f = 0; f < FETCHES && __any_sync(0xFFFFFFFFu, !go && more); f++)
-        if (!go && more) {
-          const uint64_t i = op.i[me];
-          go = fetch(i, key, tag, hp, coin);
-          op.key[me] = key;
-          op.tag[me] = tag;
-          op.hp[me] = (uint64_t)hp;
-          op.waited[me] = 0;
-          op.i[me] = i + stride;
-          more = go || i + stride < total;
+      uint32_t t = 0, index = 0;
+      bool mine = false, more = go;  // takes op `index` of table t up; is not through yet
+      if (RING) {
+        const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !go), want = (uint32_t)__popc(idle);
+        while (have < want && at < total) {
+          const uint64_t i = at + lane;
+          bool sel = i < total;
+          if (sel) {
+            t = table_of(off, ntab, i);
+            index = (uint32_t)(i - off[t]);
+            sel = table_coin(table_key(t, index, seed)) && __ldg((const uint64_t *)(desc + t));
+          }
+          const uint32_t selected = __ballot_sync(0xFFFFFFFFu, sel);
+          if (sel) {
+            const uint32_t k = warp * 64u + ((first + have + (uint32_t)__popc(selected & lt)) & 63u);
+            op.ready[k] = index;
+            op.ready_table[k] = t;
+          }
+          have += (uint32_t)__popc(selected);
+          at += (uint64_t)gridDim.x * TBT;
         }
+        __syncwarp();
+        const uint32_t r = (uint32_t)__popc(idle & lt);
+        mine = !go && r < have;
+        if (mine) {
+          const uint32_t k = warp * 64u + ((first + r) & 63u);
+          index = op.ready[k];
+          t = op.ready_table[k];
+        }
+        const uint32_t taken = min(want, have);
+        first += taken;
+        have -= taken;
+      } else {
+        const uint64_t i = op.i[me];
+        if (!go && i < total) {
+          t = table_of(off, ntab, i);
+          index = (uint32_t)(i - off[t]);
+          mine = __ldg((const uint64_t *)(desc + t));  // (a table without buckets has no ops)
+          op.i[me] = i + (uint64_t)gridDim.x * TBT;
+          more = true;
+        }
+      }
+      if (mine) {
+        const uint64_t key = table_key(t, index, seed);
+        uint32_t tag;
+        op.hp[me] = (uint64_t)place(t, key, tag);
+        op.key[me] = key;
+        op.tag[me] = tag;
+        op.waited[me] = 0;
+        go = more = true;
+      }
       if (INSERTS && BATCHED) {
         if (!__syncthreads_or(more)) break;
         node *n = (node *)gal::cta_malloc(s, sizeof(node), go && !spare, cm);
@@ -381,6 +428,7 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
           go = false;
         }
       }
+      __syncwarp();
     }
     if (spare) {  // held ready to the end
       gal::free_sized(s, spare, sizeof(node));
@@ -388,9 +436,15 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
     }
     count(lc, INSERTS ? S_INSERTED : S_DELETED, op.pairs[me]);
     count(lc, INSERTS ? S_NODES : S_NODES_FREED, op.nodes[me]);
+    __syncwarp();
   } else {
-    for (uint64_t i = (uint64_t)blockIdx.x * TBT + me; i < total; i += stride)
-      if (fetch(i, key, tag, hp, coin)) lookup_op(hp, key, tag, PHASE == PH_CHECK_ALL || !coin, lc);
+    for (uint64_t i = (uint64_t)blockIdx.x * TBT + me; i < total; i += (uint64_t)gridDim.x * TBT) {
+      const uint32_t t = table_of(off, ntab, i);
+      const uint64_t key = table_key(t, i - off[t], seed);
+      uint32_t tag;
+      const unsigned long long *hp = place(t, key, tag);
+      if (__ldg((const uint64_t *)(desc + t))) lookup_op(hp, key, tag, PHASE == PH_CHECK_ALL || !table_coin(key), lc);
+    }
     __syncwarp();
   }
   flush(stats, lc);  // whole warps

@@ -37,3 +37,22 @@ def test_tables_of_every_shape(sizes, dump, batched):
                                               "free_counters"]) == []
     finally:
         g.close()
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_table_without_buckets(batched):
+    """A table whose bucket array the arena cannot hold has no ops; the tables
+    on both sides of it are served whole."""
+    import gallatin_gb300 as G
+    from gallatin_gb300 import tables as T
+    sizes = np.array([500, 1 << 29, 300], dtype=np.uint64)  # 2**27 heads: as large as the arena
+    g = G.Gallatin.generate_on_device(1 << 30, 42, zero_arena=0)
+    try:
+        d = T.run(g, sizes, seed=5, batched=batched)
+        n_del = sum(int(T.table_coins(T.table_keys(t, int(sizes[t]), 5)).sum()) for t in (0, 2))
+        assert d["setup_failed"] == 1
+        for k in ("missing", "unexpected", "wrong_value", "count_mismatch", "malloc_failed", "lock_timeouts"):
+            assert d[k] == 0, k
+        assert d["deleted"] == n_del and d["inserted"] == 800 + n_del
+    finally:
+        g.close()
