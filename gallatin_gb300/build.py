@@ -60,19 +60,26 @@ def build(force=False, verbose=False):
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed:\n{' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
 
-    dropin_src = os.path.join(ROOT, "tests", "dropin", "dropin_test.cu")
-    dropin_lib = os.path.join(ROOT, "tests", "dropin", "libdropin_test.so")
+    # user code compiled against the headers and linked to the library: a
+    # source-compatibility check written against the reference's headers, and
+    # kernels of the tests
+    tests = os.path.join(ROOT, "tests")
     dropin_headers = HEADERS + [os.path.join(ROOT, "include", "gallatin", "allocators", h)
                                 for h in ("gallatin.cuh", "global_allocator.cuh")]
+    users = [(os.path.join(tests, "dropin", "dropin_test.cu"), os.path.join(tests, "dropin", "libdropin_test.so")),
+             (os.path.join(tests, "device", "device_test.cu"), os.path.join(tests, "device", "libdevice_test.so"))]
     with ThreadPoolExecutor(max_workers=(len(jobs) or 1) + 1) as ex:
         list(ex.map(run, jobs))
     if force or jobs or _stale(LIB, objs):
         run([nvcc(), "-shared", "-cudart", "shared"] + ARCH + objs + ["-o", LIB])
-    # drop-in source-compatibility check: user code written against the
-    # reference's headers, compiled against ours and linked to the library
-    if os.path.exists(dropin_src) and (force or _stale(dropin_lib, [dropin_src, LIB] + dropin_headers)):
-        run([nvcc()] + NVCC_FLAGS + ARCH + ["-shared", "-cudart", "shared", dropin_src, "-o", dropin_lib,
-             "-L" + HERE, "-lgallatin_gb300", "-Xlinker", "-rpath," + HERE])
+    def run_user(src_lib):
+        src, target = src_lib
+        if os.path.exists(src) and (force or _stale(target, [src, LIB] + dropin_headers)):
+            run([nvcc()] + NVCC_FLAGS + ARCH + ["-shared", "-cudart", "shared", src, "-o", target,
+                 "-L" + HERE, "-lgallatin_gb300", "-Xlinker", "-rpath," + HERE])
+
+    with ThreadPoolExecutor(max_workers=len(users)) as ex:
+        list(ex.map(run_user, users))
     return LIB
 
 

@@ -854,14 +854,53 @@ GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool t
   return ok ? (int64_t)seg : -1;
 }
 
+// A class's tree lists the segments that have a block to give, as far as its
+// atomics let it: whoever raises a count lists the segment after that, and who
+// finds a listed segment without one takes it off again.  A segment counts as
+// serving while its word has the class and a count that is not negative.
+GAL_DEVICE_INLINE bool serves(const state *s, uint32_t tree, uint64_t seg) {
+  const unsigned long long w = ld_rlx(&cfield(s->act)[seg]);
+  return act_class(w) == tree && act_count(w) >= 0;
+}
+
+// Takes a segment that has no block to give (or is another class's by now) off
+// its class's tree: by the thread that took its last block, or by any that
+// finds it listed meanwhile, so that nobody waits for the former.  Blocks may
+// have come home since, so the segment is listed again if it has one to give
+// (the fence: who raised the count and listed the segment before this removal
+// is seen here, who lists it after it undoes the removal).
+// The release of a segment closes its count word before it unlists it, so a
+// listing made here and still valid when the word is read again is either right
+// or taken off by the release.  One thread alone never finds such a segment.
+GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
+  while (veb_remove(sub_tree(s, tree), seg)) {
+    fence_acq_rel();
+    if (!serves(s, tree, seg)) return;
+    veb_insert(sub_tree(s, tree), seg);
+    fence_acq_rel();
+    if (serves(s, tree, seg)) return;
+  }
+}
+
+// Lists a segment whose count this thread has raised (after a fence).  Raised
+// first: a search that found the segment listed and its count still negative
+// would take it off, and the next listing is a lap of the ring away.  The
+// segment may have been emptied, or released and set up for another class, in
+// between: then it does not stay listed.
+GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint64_t seg) {
+  veb_insert(sub_tree(s, tree), seg);
+  fence_acq_rel();
+  if (!serves(s, tree, seg)) unlist_refusing(s, tree, seg);
+}
+
 // Releases segment `seg` of class `tree` when its count word still reads
 // `gen` with every block home (nb - 1): removes it from the class's tree,
 // frees its class and lists it in the segment tree (the release steps of
 // Gallatin::return_block, gallatin.cuh:1663-1722, finish_freeing_block,
 // memory_table.cuh:1226-1241).
-GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
+GAL_DEVICE_COLD bool release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
   const unsigned long long home = act_word(gen, tree, (int32_t)nb - 1);
-  if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return;
+  if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return false;
   fence_acq_rel();
   veb_remove(sub_tree(s, tree), seg);
   fence_acq_rel();
@@ -870,22 +909,26 @@ GAL_DEVICE_COLD void release_segment(const state *s, uint64_t seg, uint32_t tree
   st_rlx(&cfield(s->tree_ids)[seg], FREE_TREE);
   fence_acq_rel();
   veb_insert(seg_tree(s), seg);
+  return true;
 }
 
 // Gives back a reservation taken from segment `seg` that no block came of.
 // While it was held the count stayed below every-block-home, so no release
 // could run; if giving it back brings the count there and blocks were handed
 // out in this generation (every one of them has come home, the last return
-// having found the count one short), the segment is released here.  With no
-// hand-out yet the segment is a fresh one whose gatherer takes its first
-// block next, so it stays.
+// having found the count one short), the segment is released here.  While it
+// was held the count may also have read negative with a block there to give,
+// and a search that met the segment then has taken it off its tree: it is
+// listed again.
 GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
   const unsigned long long old = add_acquire(&cfield(s->act)[seg], 1ull);
   const uint32_t tree = act_class(old);
-  if (tree >= cfield(s->num_trees)) return;
+  if (tree >= cfield(s->num_trees) || act_count(old) + 1 < 0) return;
   const uint32_t nb = blocks_in_segment(s, tree);
-  if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&cfield(s->qc)[seg]) != 0)
-    release_segment(s, seg, tree, act_gen(old), nb);
+  if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&cfield(s->qc)[seg]) != 0 &&
+      release_segment(s, seg, tree, act_gen(old), nb))
+    return;
+  list_serving(s, tree, seg);
 }
 
 // alloc_table::get_block (memory_table.cuh:915-993)
@@ -948,24 +991,6 @@ GAL_DEVICE_INLINE uint32_t *waiters_of(const state *s, uint32_t tree) {
 }
 GAL_DEVICE_INLINE uint32_t more_segments(const state *s, uint32_t tree, uint32_t waiting) {
   return min(MORE_SEGMENTS, waiting / blocks_in_segment(s, tree));
-}
-
-// Takes a segment that has no block to give (or is another class's by now) off
-// its class's tree: by the thread that took its last block, or by any that
-// finds it listed meanwhile, so that nobody waits for the former.  Blocks may
-// have come home since, so the segment is listed again if it has one to give.
-// The release of a segment closes its count word before it unlists it, so a
-// listing made here and still valid when the word is read again is either right
-// or taken off by the release.  One thread alone never finds such a segment.
-GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
-  while (veb_remove(sub_tree(s, tree), seg)) {
-    unsigned long long w = ld_rlx(&cfield(s->act)[seg]);
-    if (act_class(w) != tree || act_count(w) < 0) return;
-    veb_insert(sub_tree(s, tree), seg);
-    fence_acq_rel();
-    w = ld_rlx(&cfield(s->act)[seg]);
-    if (act_class(w) == tree && act_count(w) >= 0) return;
-  }
 }
 
 // The rest of a block request that took the last block of a segment
