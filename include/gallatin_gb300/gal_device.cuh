@@ -1117,11 +1117,13 @@ GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
   // re-register at the 10% crossing (gallatin.cuh:1646): live/nb >= 0.1 and
   // (live-1)/nb < 0.1 in doubles; for the power-of-two nb used here that is
   // 10*live > nb >= 10*(live-1) with live-1 taken as unsigned (live 0 never).
-  if (live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb) veb_insert(sub_tree(s, tree), seg);
+  const bool crossing = live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb;
   fence_acq_rel();  // the ring entry before the count that lets it be handed out
   const unsigned long long old = add_acquire(&cfield(s->act)[seg], 1ull);
-  if ((uint32_t)(act_count(old) + 2) == nb)  // all_blocks_free: the count was nb - 2
-    release_segment(s, seg, tree, act_gen(old), nb);
+  if ((uint32_t)(act_count(old) + 2) == nb &&  // all_blocks_free: the count was nb - 2
+      release_segment(s, seg, tree, act_gen(old), nb))
+    return;
+  if (crossing) list_serving(s, tree, seg);
 }
 
 // Block::block_free_multiple + reset_free + free_block (block.cuh:87-98,200-212,

@@ -8,6 +8,38 @@
 
 namespace {
 
+__device__ __forceinline__ uint64_t mix(uint64_t z) {
+  z ^= z >> 30;
+  z *= 0xBF58476D1CE4E5B9ull;
+  z ^= z >> 27;
+  z *= 0x94D049BB133111EBull;
+  return z ^ (z >> 31);
+}
+
+// whole blocks of `size` bytes asked for and freed by every thread, at most `keep`
+// (up to 4) held at a time; kept[4 * thread ..] is what it holds (null: nothing)
+__global__ void k_blocks(const gal::state *s, uint64_t size, uint32_t turns, uint32_t keep, uint64_t seed,
+                         void **kept, unsigned long long *failed) {
+  const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  void *held[4];
+  uint32_t n = 0;
+  for (uint32_t j = 0; j < 4; j++)
+    if (kept[4 * me + j]) held[n++] = kept[4 * me + j];
+  for (uint32_t k = 0; k < turns; k++) {
+    const uint64_t r = mix(seed + me * turns + k);
+    if (n < keep && (n == 0 || (r & 1u))) {
+      void *p = gal::malloc(s, size);
+      if (!p) atomicAdd(failed, 1ull);
+      else held[n++] = p;
+    } else {
+      const uint32_t j = (uint32_t)(r >> 8) % n;
+      gal::free(s, held[j]);
+      held[j] = held[--n];
+    }
+  }
+  for (uint32_t j = 0; j < 4; j++) kept[4 * me + j] = j < n ? held[j] : nullptr;
+}
+
 // One thread: a segment of class `tree` with one block left to give, whose count
 // a reservation meant for an earlier owner takes below zero; a request that
 // meets it then; the reservation given back.  `fresh`: a segment gathered ahead,
@@ -42,6 +74,11 @@ __global__ void k_give_back(const gal::state *s, uint32_t tree, int fresh, unsig
   return cudaDeviceSynchronize() == cudaSuccess ? 0 : 2
 
 extern "C" {
+
+int dev_blocks(const gal::state *s, uint64_t size, uint32_t ctas, uint32_t threads, uint32_t turns, uint32_t keep,
+               uint64_t seed, void **kept, unsigned long long *failed) {
+  RUN(k_blocks<<<ctas, threads>>>(s, size, turns, keep, seed, kept, failed));
+}
 
 int dev_give_back(const gal::state *s, uint32_t tree, int fresh, unsigned long long *out) {
   RUN(k_give_back<<<1, 1>>>(s, tree, fresh, out));

@@ -18,6 +18,7 @@ def D():
     gallatin_gb300.lib()
     L = C.CDLL(LIB)
     u32, u64, vp = C.c_uint32, C.c_uint64, C.c_void_p
+    L.dev_blocks.argtypes = [vp, u64, u32, u32, u32, u32, u64, vp, vp]
     L.dev_give_back.argtypes = [vp, u32, C.c_int, vp]
     return L
 
@@ -43,5 +44,52 @@ def test_reservation_given_back_lists_the_segment_again(D, cls, fresh):
         g.trim()
         assert (_bottom(g.export(), g.dims()) == fresh_trees).all()
         assert g.error_word() == 0, g.error_info()
+    finally:
+        g.close()
+
+
+def _unlisted_past_crossing(g):
+    """(segment, class) of every owned segment that has blocks to give and is in
+    no tree although one of them came home at the ring position that lists a
+    segment (the first of which ten times is more than the segment's blocks).
+    The first to come home since the segment was last empty is left out: it may
+    have taken its position before, and been counted after, the last block went."""
+    e, d = g.export(), g.dims()
+    listed = _bottom(e, d)
+    bad = []
+    for seg in range(d.num_segments):
+        t, home = int(e.tree_ids[seg]), int(e.active_counts[seg]) + 1
+        if t >= d.num_trees or home <= 0 or (int(listed[t, seg // 64]) >> (seg % 64)) & 1:
+            continue
+        nb, back = d.blocks_per_segment >> t, int(e.queue_free_counters[seg])
+        if any(p % nb == nb // 10 + 1 for p in range(max(back - home, 0) + 1, back)):
+            bad.append((seg, t))
+    return bad
+
+
+@pytest.mark.parametrize("cls", [3, 4, 5])
+def test_returned_blocks_stay_listed(D, cls):
+    """Whole blocks of one class (32, 16 and 8 to a segment) asked for and returned
+    by many threads at once, its segments emptying and filling all the time: a
+    segment that a returned block put back into its class's tree stays there."""
+    import torch
+    import gallatin_gb300 as G
+    size = (16 << cls) * 4096
+    failed = torch.zeros(1, dtype=torch.int64, device="cuda")
+    g = G.Gallatin.generate_on_device(8 * GIB, 42, zero_arena=0)
+    try:
+        fresh = g.export()
+        kept = torch.zeros(4 * 1024, dtype=torch.int64, device="cuda")
+        for seed in range(30):
+            assert D.dev_blocks(g.device_state, size, 32, 32, 41, 2, seed, kept.data_ptr(), failed.data_ptr()) == 0
+            assert _unlisted_past_crossing(g) == []
+        assert int(failed) == 0 and g.error_word() == 0, g.error_info()
+        g.free_per_thread(kept)
+        torch.cuda.synchronize()
+        g.trim()
+        assert g.error_word() == 0, g.error_info()
+        now = g.export()
+        assert now.diff(fresh, fields=["seg_tree_words", "tree_ids", "slots", "free_counters"]) == []
+        assert (_bottom(now, g.dims()) == _bottom(fresh, g.dims())).all()
     finally:
         g.close()
