@@ -230,6 +230,16 @@ GAL_DEVICE_INLINE void st_rlx(uint32_t *p, uint32_t v) {
 GAL_DEVICE_INLINE void st_rlx(uint16_t *p, uint16_t v) {
   asm volatile("st.relaxed.gpu.global.u16 [%0], %1;" ::"l"(p), "h"(v) : "memory");
 }
+// a store after everything this thread has done and seen so far ...
+GAL_DEVICE_INLINE void st_release(uint32_t *p, uint32_t v) {
+  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// ... and an exchange that takes all of that over with the value it finds
+GAL_DEVICE_INLINE uint32_t exch_acquire(uint32_t *p, uint32_t v) {
+  uint32_t r;
+  asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], %2;" : "=r"(r) : "l"(p), "r"(v) : "memory");
+  return r;
+}
 GAL_DEVICE_INLINE uint16_t cas16(uint16_t *p, uint16_t cmp, uint16_t val) {
   return (uint16_t)atomicCAS((unsigned short *)p, (unsigned short)cmp, (unsigned short)val);
 }
@@ -961,10 +971,10 @@ GAL_DEVICE_COLD uint32_t get_block(const state *s, uint64_t seg, uint32_t tree, 
     blk = (uint32_t)(seg << cfield(s->bps_shift)) + pos;
   } else {
     uint32_t *e = cfield(s->queues) + (seg << cfield(s->bps_shift)) + (pos & (nb - 1u));
-    blk = atomicExch(e, NOBLK);
+    blk = exch_acquire(e, NOBLK);
     for (uint32_t i = 0; blk == NOBLK && i < cfield(s->spin_limit); i++) {  // a return still in flight
       backoff(i);
-      blk = atomicExch(e, NOBLK);
+      blk = exch_acquire(e, NOBLK);
     }
     if (blk == NOBLK) {
       set_error(s, GAL_DEV_ERR_NULL_QUEUE);
@@ -1108,7 +1118,9 @@ GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
   uint32_t nb = blocks_in_segment(s, tree);
   uint32_t pos = atomicAdd(&cfield(s->qfc)[seg], 1u);
   uint32_t live = pos & (nb - 1u);
-  st_rlx(cfield(s->queues) + (seg << cfield(s->bps_shift)) + live, blk);
+  // with the block's free counter at 0: counts are interchangeable, so whoever
+  // takes the entry may have been let in by another block's return
+  st_release(cfield(s->queues) + (seg << cfield(s->bps_shift)) + live, blk);
   // The reference finalises returns in position order with a CAS spin
   // (memory_table.cuh:906-910) so a hand-out never meets an empty ring entry;
   // get_block here waits (bounded) for an entry still in flight instead, so a
@@ -1135,7 +1147,7 @@ GAL_DEVICE_INLINE void credit_frees(const state *s, uint32_t blk, uint32_t n) {
 // the block's free counter was `old` before this thread added n
 GAL_DEVICE_INLINE void credit_done(const state *s, uint32_t blk, uint32_t old, uint32_t n) {
   if (old + n == SLICES_PER_BLOCK) {
-    st_rlx(fctr_ptr(s, blk), 0u);  // published by return_block's fence
+    st_rlx(fctr_ptr(s, blk), 0u);  // published with the block's ring entry
     return_block(s, blk);
   } else if (old + n > SLICES_PER_BLOCK) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OVERFLOW, blk,

@@ -40,6 +40,55 @@ __global__ void k_blocks(const gal::state *s, uint64_t size, uint32_t turns, uin
   for (uint32_t j = 0; j < 4; j++) kept[4 * me + j] = j < n ? held[j] : nullptr;
 }
 
+// Every thread asks for `turns` sizes, log-uniform over [16, hi], stamps each
+// allocation at both ends and frees it `keep` (at most 4) of its own requests
+// later, its stamps checked.  form 0: malloc and free; 1: malloc and free_sized;
+// 2: malloc_cached and free_sized.  out: failed, wrong stamps.
+__global__ void k_churn(const gal::state *s, uint32_t turns, uint32_t hi_bits, uint32_t keep, int form, uint64_t seed,
+                        unsigned long long *out) {
+  __shared__ gal::slot_cache cache;
+  gal::slot_cache_init(cache);
+  __syncthreads();
+  const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint64_t *held[5], len[5], id[5];
+  uint32_t n = 0, bad = 0, failed = 0;
+  auto drop = [&]() {  // the oldest
+    bad += held[0][0] != id[0] || held[0][len[0] / 8 - 1] != id[0];
+    if (form == 0) gal::free(s, held[0]);
+    else gal::free_sized(s, held[0], len[0]);
+    n--;
+    for (uint32_t j = 0; j < n; j++) {
+      held[j] = held[j + 1];
+      len[j] = len[j + 1];
+      id[j] = id[j + 1];
+    }
+  };
+  for (uint32_t k = 0; k < turns; k++) {
+    const uint64_t r = mix(seed + me * turns + k), bits = 4 + r % (hi_bits - 3);
+    const uint64_t size = min((1ull << bits) + ((r >> 16) & ((1ull << bits) - 1)), 1ull << hi_bits);
+    uint64_t *p = (uint64_t *)(form == 2 ? gal::malloc_cached(s, size, cache) : gal::malloc(s, size));
+    if (!p) {
+      failed++;
+    } else {
+      held[n] = p;
+      len[n] = size;
+      id[n] = me << 32 | k;
+      p[0] = p[size / 8 - 1] = id[n];
+      n++;
+    }
+    if (n > keep) drop();
+  }
+  while (n) drop();
+  if (failed) atomicAdd(&out[0], (unsigned long long)failed);
+  if (bad) atomicAdd(&out[1], (unsigned long long)bad);
+}
+
+// out[i] = malloc(size) from every thread, one per thread
+__global__ void k_fill(const gal::state *s, uint64_t size, uint64_t n, void **out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = gal::malloc(s, size);
+}
+
 // One thread: a segment of class `tree` with one block left to give, whose count
 // a reservation meant for an earlier owner takes below zero; a request that
 // meets it then; the reservation given back.  `fresh`: a segment gathered ahead,
@@ -78,6 +127,15 @@ extern "C" {
 int dev_blocks(const gal::state *s, uint64_t size, uint32_t ctas, uint32_t threads, uint32_t turns, uint32_t keep,
                uint64_t seed, void **kept, unsigned long long *failed) {
   RUN(k_blocks<<<ctas, threads>>>(s, size, turns, keep, seed, kept, failed));
+}
+
+int dev_churn(const gal::state *s, uint32_t ctas, uint32_t threads, uint32_t turns, uint32_t hi_bits, uint32_t keep,
+              int form, uint64_t seed, unsigned long long *out) {
+  RUN(k_churn<<<ctas, threads>>>(s, turns, hi_bits, keep, form, seed, out));
+}
+
+int dev_fill(const gal::state *s, uint64_t size, uint64_t n, void **out) {
+  RUN(k_fill<<<(unsigned)((n + 255) / 256), 256>>>(s, size, n, out));
 }
 
 int dev_give_back(const gal::state *s, uint32_t tree, int fresh, unsigned long long *out) {

@@ -19,6 +19,8 @@ def D():
     L = C.CDLL(LIB)
     u32, u64, vp = C.c_uint32, C.c_uint64, C.c_void_p
     L.dev_blocks.argtypes = [vp, u64, u32, u32, u32, u32, u64, vp, vp]
+    L.dev_churn.argtypes = [vp, u32, u32, u32, u32, u32, C.c_int, u64, vp]
+    L.dev_fill.argtypes = [vp, u64, u64, vp]
     L.dev_give_back.argtypes = [vp, u32, C.c_int, vp]
     return L
 
@@ -27,6 +29,72 @@ def _bottom(e, d):
     """The lowest words of every class's tree: the segments it lists."""
     per_tree = e.sub_tree_words.reshape(d.num_trees, -1)
     return per_tree[:, per_tree.shape[1] - (d.num_segments + 63) // 64:]
+
+
+def _as_fresh(g, fresh):
+    """After a trim the allocator is as it was when it was made (but for bits of
+    the trees' upper layers, which may outlast the items below them)."""
+    g.trim()
+    assert g.error_word() == 0, g.error_info()
+    now = g.export()
+    assert now.diff(fresh, fields=["seg_tree_words", "tree_ids", "slots", "free_counters"]) == []
+    assert (_bottom(now, g.dims()) == _bottom(fresh, g.dims())).all()
+
+
+TUNED = dict(pinned_slots_first=0, pinned_slots_min=0, gather_unlocked_below=16, bytes_per_segment=64 << 20,
+             spare_blocks=1)
+
+
+@pytest.mark.parametrize("form", [0, 1, 2], ids=["free", "free_sized", "cached"])
+@pytest.mark.parametrize("cfg,hi_bits", [(dict(), 9), (dict(), 17), (dict(team_width=8), 15), (TUNED, 15),
+                                         (dict(min_size=128, max_size=16384, bytes_per_segment=64 << 20), 20)],
+                         ids=["small", "blocks", "narrow-teams", "tuned", "large-classes"])
+def test_mallocs_and_frees_inside_a_kernel(D, cfg, hi_bits, form):
+    """A grid that fills the chip, every thread allocating and freeing mixed sizes
+    by itself (single slices, runs of slices and whole blocks): each allocation
+    is its owner's alone, and once all are free every block is home with its
+    free counter at 0."""
+    import torch
+    import gallatin_gb300 as G
+    out = torch.zeros(2, dtype=torch.int64, device="cuda")
+    g = G.Gallatin.generate_on_device(48 * GIB, 42, zero_arena=0, **cfg)
+    try:
+        fresh = g.export()
+        ctas = 608 if hi_bits <= 15 else 76
+        for seed in range(3):
+            assert D.dev_churn(g.device_state, ctas, 256, 24, hi_bits, 3, form, seed << 40, out.data_ptr()) == 0
+            assert out.tolist() == [0, 0]
+        _as_fresh(g, fresh)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("size", [64, 1000, 4096, 9000, 4 << 20])
+def test_one_request_per_thread_until_nothing_is_left(D, size):
+    """One malloc per thread of a user's kernel, a few thousand more than the arena
+    can serve: what is handed out is disjoint and no less than the segments that
+    were free at first hold; freed, all of it is home."""
+    import torch
+    import gallatin_gb300 as G
+    held = 1 << (size - 1).bit_length()
+    g = G.Gallatin.generate_on_device(1 * GIB, 42, zero_arena=0)
+    try:
+        fresh = g.export()
+        free = int(g.stats().free_segments) * (16 << 20)
+        n = int(1.1 * free) // held + 4000
+        ptrs = torch.zeros(n, dtype=torch.int64, device="cuda")
+        assert D.dev_fill(g.device_state, size, n, ptrs.data_ptr()) == 0
+        off = np.sort(ptrs.cpu().numpy())
+        off = off[off != 0] - g.arena_base
+        assert off[0] >= 0 and off[-1] + held <= g.arena_bytes
+        assert (np.diff(off) >= held).all()
+        assert free <= len(off) * held and len(off) < n
+        assert g.error_word() == 0, g.error_info()
+        g.free_per_thread(ptrs)
+        torch.cuda.synchronize()
+        _as_fresh(g, fresh)
+    finally:
+        g.close()
 
 
 @pytest.mark.parametrize("cls,fresh", [(0, 0), (4, 0), (7, 0), (8, 1)])
@@ -86,10 +154,6 @@ def test_returned_blocks_stay_listed(D, cls):
         assert int(failed) == 0 and g.error_word() == 0, g.error_info()
         g.free_per_thread(kept)
         torch.cuda.synchronize()
-        g.trim()
-        assert g.error_word() == 0, g.error_info()
-        now = g.export()
-        assert now.diff(fresh, fields=["seg_tree_words", "tree_ids", "slots", "free_counters"]) == []
-        assert (_bottom(now, g.dims()) == _bottom(fresh, g.dims())).all()
+        _as_fresh(g, fresh)
     finally:
         g.close()
