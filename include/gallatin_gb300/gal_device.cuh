@@ -23,7 +23,8 @@
 //     and it never has to give back into a later owner's count;
 //   * every class lock sits in a 32-byte sector of its own;
 //   * every spin-wait is bounded by state::spin_limit and reports through the
-//     error word instead of trapping (the reference traps, gallatin.cuh:87);
+//     error word instead of trapping (the reference traps, gallatin.cuh:87), and
+//     so is every loop that other threads' changes can send round again;
 //   * a vEB remove re-checks the emptied child word after clearing its
 //     summary bit, with acquire-release fences ordering each thread's word
 //     and summary accesses, closing the race that hides a non-empty word;
@@ -55,6 +56,7 @@ static constexpr uint32_t SLICES_PER_BLOCK = 4096;
 // retry caps of the reference (gallatin.cuh:108-112, veb.cuh:59)
 static constexpr int SLICE_ATTEMPTS = 500 * 10;
 static constexpr int VEB_ATTEMPTS = 15;
+static constexpr uint32_t VEB_LOSSES = 1024;  // items of one word lost to other threads before a search goes on
 static constexpr int GATHER_RETRIES = 8;
 static constexpr int BLOCK_ATTEMPTS = 8;
 static constexpr int SEGMENT_ATTEMPTS = 8;
@@ -266,6 +268,7 @@ enum : uint64_t {
   SITE_REQUEST_LOCK = 6,   // request_block: the class lock stayed taken (a: class, b: spins)
   SITE_REQUEST_RETRY = 7,  // request_block: listed segments kept refusing a block (a: class, b: last segment)
   SITE_RUN_LOCK = 8,       // malloc_segment_run: the run lock stayed taken (a: segments wanted)
+  SITE_UNLIST = 9,         // unlist_refusing: the segment kept changing (a: class, b: segment)
 };
 GAL_DEVICE_INLINE void backoff(uint32_t i) { __nanosleep(i < 8 ? 32u << i : 4096u); }
 
@@ -473,7 +476,7 @@ GAL_DEVICE_INLINE uint64_t veb_malloc_first(const veb_ref &v, veb_low l) {
     for (uint64_t top = l.top; top; top &= top - 1ull) {
       const uint64_t high = (uint64_t)(__ffsll((long long)top) - 1);
       uint64_t word = veb_low_word(l, bottom, high);
-      for (uint32_t turn = 0; word; turn = spread) {
+      for (uint32_t turn = 0, lost = 0; word && lost < VEB_LOSSES; turn = spread, lost++) {
         const uint64_t turned = (word >> turn) | (turn ? word << (64u - turn) : 0ull);
         const uint64_t low = ((uint64_t)(__ffsll((long long)turned) - 1) + turn) & 63u;
         if (veb_remove(v, (high << 6) + low, word)) return (high << 6) + low;
@@ -695,7 +698,8 @@ GAL_DEVICE_COLD uint64_t veb_gather_in_word(const veb_ref &v, uint64_t n) {
   for (int tries = 0; tries < choices; tries++) {
     uint64_t *word = words + pick[at];
     uint64_t seen = ld_rlx(word);
-    for (int c; (uint64_t)(c = cfc64(seen)) >= n;) {
+    uint32_t lost = 0;
+    for (int c; (uint64_t)(c = cfc64(seen)) >= n && lost < VEB_LOSSES; lost++) {
       const uint64_t acq = bitmask((int)n) << (c - (int)n);
       const uint64_t got = atomicCAS((unsigned long long *)word, (unsigned long long)seen,
                                      (unsigned long long)(seen & ~acq));
@@ -883,12 +887,16 @@ GAL_DEVICE_INLINE bool serves(const state *s, uint32_t tree, uint64_t seg) {
 // listing made here and still valid when the word is read again is either right
 // or taken off by the release.  One thread alone never finds such a segment.
 GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
-  while (veb_remove(sub_tree(s, tree), seg)) {
+  for (uint32_t tries = 0; veb_remove(sub_tree(s, tree), seg); tries++) {
     fence_acq_rel();
     if (!serves(s, tree, seg)) return;
     veb_insert(sub_tree(s, tree), seg);
     fence_acq_rel();
     if (serves(s, tree, seg)) return;
+    if (tries >= cfield(s->spin_limit)) {  // left listed: the next search meets it again
+      set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_UNLIST, tree, seg);
+      return;
+    }
   }
 }
 
