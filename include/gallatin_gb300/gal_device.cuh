@@ -1523,7 +1523,8 @@ GAL_DEVICE_INLINE void *handed_out(const state *s, void *p, uint64_t size) {
 // the block and segment tiers of Gallatin::malloc (gallatin.cuh:1203-1258)
 GAL_DEVICE_COLD void *malloc_large(const state *s, uint64_t size, int block_tree) {
   if (block_tree < (int)cfield(s->num_trees)) return malloc_whole_block(s, (uint32_t)block_tree);
-  return malloc_segment_run(s, (uint32_t)((size - 1) >> cfield(s->seg_shift)) + 1);
+  const uint64_t count = ((size - 1) >> cfield(s->seg_shift)) + 1;  // (may not fit 32 bits)
+  return count <= cfield(s->num_segments) ? malloc_segment_run(s, (uint32_t)count) : nullptr;
 }
 
 // Gallatin::malloc (gallatin.cuh:1186-1276) called by the lanes in `callers`

@@ -869,7 +869,9 @@ uint64_t orc_malloc(orc_alloc *a, uint64_t size, uint32_t smid, uint64_t tid) {
       if (off == ORC_FAIL) return ORC_FAIL;
       return offset_to_bytes(a, off, block_tree);
     } else {
-      uint32_t count = (uint32_t)((size - 1) / a->seg_bytes + 1);
+      uint64_t needed = (size - 1) / a->seg_bytes + 1;
+      if ((a->fix & ORC_FIX_HUGE_RUN) && needed > a->S) return ORC_FAIL;
+      uint32_t count = (uint32_t)needed;
       uint64_t off = malloc_segments(a, count);
       if (off == ORC_FAIL) return ORC_FAIL;
       return offset_to_bytes(a, off, 0);

@@ -39,6 +39,10 @@ extern "C" {
  * word, which climbs only from an empty word).  With the fix every word the
  * run leaves non-empty is listed. */
 #define ORC_FIX_RUN_RETURN_SUMMARY 0x8u
+/* A request of more segments than there are is served by the low 32 bits of
+ * their number (one segment for 2^56 + 1 bytes, none for 2^64 - 1).  With the
+ * fix it fails. */
+#define ORC_FIX_HUGE_RUN 0x10u
 
 typedef struct orc_alloc orc_alloc;
 

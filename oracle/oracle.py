@@ -18,9 +18,10 @@ FIX_GATHER_EXIT_ROLLBACK = 0x1
 FIX_LEFTOVER_COMPLETES = 0x2
 FIX_RUN_BELOW_ARENA = 0x4
 FIX_RUN_RETURN_SUMMARY = 0x8
+FIX_HUGE_RUN = 0x10
 # the product fixes these reference defects; parity runs against the product use them
 PRODUCT_FIXES = (FIX_GATHER_EXIT_ROLLBACK | FIX_LEFTOVER_COMPLETES | FIX_RUN_BELOW_ARENA
-                 | FIX_RUN_RETURN_SUMMARY)
+                 | FIX_RUN_RETURN_SUMMARY | FIX_HUGE_RUN)
 
 _lib = None
 
