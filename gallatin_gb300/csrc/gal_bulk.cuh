@@ -105,8 +105,9 @@ GAL_DEVICE_COLD uint32_t bulk_claim(const state *s, uint32_t tree, uint32_t want
 GAL_DEVICE_COLD void *bulk_fallback(const state *s, uint64_t size) { return gal::malloc(s, size); }
 
 // out[i] = malloc(sizes[i]) for the CTA's K x BULK_THREADS requests from
-// `base` on (fewer at the end of the list).
-template <int K>
+// `base` on (fewer at the end of the list).  ZERO: calloc mode.  `out` may be
+// `sizes`: a size is read again only before its pointer is written.
+template <int K, bool ZERO>
 __device__ __forceinline__ void bulk_malloc(const state *s, const uint64_t *sizes, uint64_t n, uint64_t base,
                                             void **out, bulk_smem &sm) {
   const int T = (int)cfield(s->num_trees), min_shift = (int)cfield(s->min_shift);
@@ -185,17 +186,16 @@ __device__ __forceinline__ void bulk_malloc(const state *s, const uint64_t *size
         }
       }
     }
-    out[i0 + (uint64_t)k * BULK_THREADS] = p;
-    if (!p) unserved |= 1u << k;
+    if (!p) {
+      unserved |= 1u << k;
+      continue;
+    }
+    const uint64_t i = i0 + (uint64_t)k * BULK_THREADS;
+    if (ZERO) zero_fill(p, sizes[i]);
+    out[i] = p;
   }
   // before the fallback, whose waits must not hold up what others wait for
   if (refill != NOBLK) refill_spare(s, warp, refill, (uint32_t)thread_linear_id());
-  // out of the loop above, which then keeps its registers to itself
-  if (s->zero_fill)
-    for (int k = 0; k < K; k++) {
-      const uint64_t i = i0 + (uint64_t)k * BULK_THREADS;
-      if (i < n && !((unserved >> k) & 1u)) zero_fill(out[i], sizes[i]);
-    }
   for (; unserved; unserved &= unserved - 1u) {
     const uint64_t i = i0 + (uint64_t)(__ffs(unserved) - 1) * BULK_THREADS;
     out[i] = bulk_fallback(s, sizes[i]);  // clears its own bytes in calloc mode

@@ -247,11 +247,11 @@ __global__ void __launch_bounds__(MALLOC_THREADS, 4)
 // Lists of several waves gain from a third CTA per SM (40 registers; 4 Mi mixed:
 // 70 -> 64 us), one wave does not.
 constexpr uint64_t BULK_FROM = 1u << 15;
-template <int K>
+template <int K, bool ZERO>
 __global__ void __launch_bounds__(gal::BULK_THREADS, K == 8 ? 3 : 2)
     k_malloc_bulk(const gal::state *s, const uint64_t *sizes, uint64_t n, void **out) {
   __shared__ gal::bulk_smem sm;
-  gal::bulk_malloc<K>(s, sizes, n, (uint64_t)blockIdx.x * (K * gal::BULK_THREADS), out, sm);
+  gal::bulk_malloc<K, ZERO>(s, sizes, n, (uint64_t)blockIdx.x * (K * gal::BULK_THREADS), out, sm);
 }
 
 // Batched free: a persistent grid, a CTA taking chunks of 256 K entries and
@@ -826,14 +826,16 @@ int gal_malloc_batched(gal_handle *h, const uint64_t *sizes, uint64_t n, void **
   if (n < BULK_FROM) {
     k_malloc_threads<<<grid_for(n, MALLOC_THREADS), MALLOC_THREADS, 0, st>>>(h->d_state, sizes, n, out);
   } else {
-    auto bulk = [&](auto kern, int k) {
-      kern<<<grid_for(n, gal::BULK_THREADS * k), gal::BULK_THREADS, 0, st>>>(h->d_state, sizes, n, out);
+    auto bulk = [&](auto kern, auto calloc_kern, int k) {
+      const unsigned grid = grid_for(n, gal::BULK_THREADS * k);
+      if (h->st.zero_fill) calloc_kern<<<grid, gal::BULK_THREADS, 0, st>>>(h->d_state, sizes, n, out);
+      else kern<<<grid, gal::BULK_THREADS, 0, st>>>(h->d_state, sizes, n, out);
     };
     const uint64_t wave = 2ull * (uint64_t)h->sms * gal::BULK_THREADS;  // requests one wave serves, one per thread
-    if (n <= wave) bulk(k_malloc_bulk<1>, 1);
-    else if (n <= 2 * wave) bulk(k_malloc_bulk<2>, 2);
-    else if (n <= 4 * wave) bulk(k_malloc_bulk<4>, 4);
-    else bulk(k_malloc_bulk<8>, 8);
+    if (n <= wave) bulk(k_malloc_bulk<1, false>, k_malloc_bulk<1, true>, 1);
+    else if (n <= 2 * wave) bulk(k_malloc_bulk<2, false>, k_malloc_bulk<2, true>, 2);
+    else if (n <= 4 * wave) bulk(k_malloc_bulk<4, false>, k_malloc_bulk<4, true>, 4);
+    else bulk(k_malloc_bulk<8, false>, k_malloc_bulk<8, true>, 8);
   }
   CUDA_TRY(cudaGetLastError());
   return GAL_OK;

@@ -308,7 +308,9 @@ int gal_replay_warp_trace(gal_handle *h, const uint64_t *steps, uint64_t nsteps,
                           uint64_t *out_offsets, uint32_t *out_smid, void *stream);
 
 /* out_ptrs[i] = malloc(sizes[i]) for every i, as one global_malloc per thread
- * (global_allocator.cuh:72-76); the same kernels as gal_malloc_batched. */
+ * (global_allocator.cuh:72-76); the same kernels as gal_malloc_batched.
+ * sizes and out_ptrs may be one buffer, here and there (each pointer then takes
+ * its size's place); they must not overlap in any other way. */
 int gal_malloc_per_thread(gal_handle *h, const uint64_t *sizes, uint64_t n,
                           void **out_ptrs, void *stream);
 /* free(ptrs[i]) for every i unless NULL (global_free,
