@@ -43,6 +43,7 @@ GAL_DEVICE_COLD uint32_t bulk_claim(const state *s, uint32_t tree, uint32_t want
   // takes up to `need` slices of a block, installed or not; false: none of them
   // are this class's to use.  A block read in an earlier life may be claimed
   // from by a slow team at any time, so every take is an atomic on its count.
+  // crossed: nothing is left of the block and this thread is to replace it.
   uint32_t crossed = 0, rest = want;
   auto take = [&](uint32_t blk, uint32_t need) {
     const unsigned long long old = atomicAdd(mword_ptr(s, blk), (unsigned long long)need);
@@ -62,37 +63,59 @@ GAL_DEVICE_COLD uint32_t bulk_claim(const state *s, uint32_t tree, uint32_t want
     rest -= got;
     return true;
   };
-  while (rest >= SLICES_PER_BLOCK && n < (uint32_t)BULK_RUNS) {
+  for (int attempt = 0; attempt < BULK_ATTEMPTS && rest >= SLICES_PER_BLOCK && n < (uint32_t)BULK_RUNS; attempt++) {
     const uint32_t blk = request_block(s, tree, tid);
     if (blk == NOBLK) break;
     take(blk, SLICES_PER_BLOCK);  // all that is left of it: it never enters a slot
   }
+  uint32_t refused = NOBLK, refusals = 0;  // the exhausted block last met, and how often in a row
   for (int attempt = 0; attempt < BULK_ATTEMPTS && rest && rest < SLICES_PER_BLOCK && n < (uint32_t)BULK_RUNS;
        attempt++) {
     uint32_t blk;
     const uint32_t slot = pick_slot(s, tree, blk);
-    if (blk == NOBLK || !take(blk, rest)) {  // empty or exhausted: its crosser is installing the next block
-      __nanosleep(blk == NOBLK ? 200u : 100u);
-      continue;
+    if (blk == NOBLK || blk == refused || !take(blk, rest)) {
+      // empty or exhausted: its crosser is installing the next block.  (A block
+      // met again is only looked at, as every take adds to its count.)
+      refusals = blk != NOBLK && blk == refused ? refusals + 1u : 0u;
+      refused = blk;
+      if (refusals < (uint32_t)STUCK_ATTEMPTS || (uint32_t)ld_rlx(mword_ptr(s, blk)) < SLICES_PER_BLOCK) {
+        if (refusals >= (uint32_t)STUCK_ATTEMPTS) refused = NOBLK;  // it is a block to claim from again
+        __nanosleep(blk == NOBLK ? 200u : 100u);
+        continue;
+      }
+      refused = NOBLK;  // nobody replaces it (see STUCK_ATTEMPTS): done here
+    } else {
+      refused = NOBLK;
+      if (!crossed) continue;
     }
-    if (!crossed) continue;
-    uint32_t *const sp = s->slots + s->slot_base[tree] + slot;
-    uint32_t next = s->use_spares ? atomicExch(s->spares + s->slot_base[tree] + slot, NOBLK) : NOBLK;
-    const bool spare = next != NOBLK;
-    if (s->use_spares) refill = slot;
+    const uint32_t at = s->slot_base[tree] + slot;
+    uint32_t next = s->use_spares ? atomicExch(s->spares + at, NOBLK) : NOBLK;
+    if (s->use_spares) {
+      if (refill != NOBLK && refill != slot) refill_spare(s, tree, refill, tid);  // of a slot crossed before
+      refill = slot;
+    }
+    const uint32_t found = next != NOBLK ? blk : NOBLK;  // what the slot holds until the next block is in
+    if (next == NOBLK && atomicCAS(s->slots + at, blk, NOBLK) != blk) continue;
     uint64_t asked = ~0ull;  // nothing to finish
-    if (!spare) {
-      if (atomicCAS(sp, blk, NOBLK) != blk) continue;
-      asked = request_block_begin(s, tree, tid);
-      next = requested_block(asked);
-      if (next == NOBLK) break;
+    for (int tries = 0; tries < BLOCK_ATTEMPTS; tries++) {
+      if (next == NOBLK) {
+        asked = request_block_begin(s, tree, tid);
+        next = requested_block(asked);
+        if (next == NOBLK) break;
+      }
+      if (!rest || n >= (uint32_t)BULK_RUNS || (take(next, rest) && !crossed)) break;
+      // slow teams and this claim have used it up: not a block for the slot
+      request_done(s, tree, asked);
+      asked = ~0ull;
+      next = NOBLK;
     }
-    if (rest && n < (uint32_t)BULK_RUNS) take(next, rest);
+    if (next == NOBLK) {  // no block to be had: the slot is left empty
+      if (found != NOBLK) atomicCAS(s->slots + at, found, NOBLK);
+      break;
+    }
     fence_acq_rel();
-    if (spare) {
-      if (atomicCAS(sp, blk, next) != blk) retire_block(s, next);  // the slot moved on
-    } else if (atomicCAS(sp, NOBLK, next) != NOBLK) {
-      set_error(s, GAL_DEV_ERR_SLOT_SWAP);
+    if (atomicCAS(s->slots + at, found, next) != found) {  // the slot moved on
+      if (found == NOBLK) set_error(s, GAL_DEV_ERR_SLOT_SWAP);
       retire_block(s, next);
     }
     request_done(s, tree, asked);

@@ -6,6 +6,8 @@
 
 #include <gallatin_gb300/gal_device.cuh>
 
+#include "../../gallatin_gb300/csrc/gal_bulk.cuh"
+
 namespace {
 
 __device__ __forceinline__ uint64_t mix(uint64_t z) {
@@ -89,6 +91,53 @@ __global__ void k_fill(const gal::state *s, uint64_t size, uint64_t n, void **ou
   if (i < n) out[i] = gal::malloc(s, size);
 }
 
+// Of block `blk` all slices but `left` handed out; the number that were not yet.
+__device__ uint32_t use_up(const gal::state *s, uint32_t blk, uint32_t left) {
+  const uint32_t count = (uint32_t)gal::ld_rlx(gal::mword_ptr(s, blk)), to = gal::SLICES_PER_BLOCK - left;
+  if (count >= to) return 0;
+  atomicAdd(gal::mword_ptr(s, blk), (unsigned long long)(to - count));
+  return to - count;
+}
+
+// One thread's chunk claim of `want` slices of class `tree` when every pinned
+// block has `slot_left` slices left and every spare `spare_left`, as after claims
+// of slow teams.  out: slices claimed, runs, slices left in the slot's block,
+// blocks that could not be read.  Everything is given back.
+__global__ void k_chunk_claim(const gal::state *s, uint32_t tree, uint32_t want, uint32_t slot_left,
+                              uint32_t spare_left, unsigned long long *out) {
+  __shared__ gal::bulk_smem sm;
+  constexpr uint32_t MOST = 64;
+  uint32_t blks[2 * MOST], used[2 * MOST], n = 0;
+  const uint32_t slots = s->slot_count[tree], base = s->slot_base[tree];
+  if (slots > MOST) return;
+  for (uint32_t i = 0; i < slots; i++) {
+    if (s->use_spares) gal::refill_spare(s, tree, i, 0);
+    for (uint32_t *at = s->slots + base + i; at; at = at == s->slots + base + i && s->use_spares ? s->spares + base + i : nullptr) {
+      const uint32_t blk = gal::ld_rlx(at);
+      if (blk == gal::NOBLK) {
+        out[3]++;
+        continue;
+      }
+      used[n] = use_up(s, blk, at == s->slots + base + i ? slot_left : spare_left);
+      blks[n++] = blk;
+    }
+  }
+  const uint32_t refill = gal::bulk_claim(s, tree, want, sm);
+  for (uint32_t j = 0; j < sm.nruns[tree]; j++) out[0] += sm.len[tree][j];
+  out[1] = sm.nruns[tree];
+  uint32_t blk;
+  gal::pick_slot(s, tree, blk);
+  const uint32_t count = blk == gal::NOBLK ? gal::SLICES_PER_BLOCK : (uint32_t)gal::ld_rlx(gal::mword_ptr(s, blk));
+  out[2] = count < gal::SLICES_PER_BLOCK ? gal::SLICES_PER_BLOCK - count : 0;
+  if (refill != gal::NOBLK) gal::refill_spare(s, tree, refill, 0);
+  for (uint32_t j = 0; j < sm.nruns[tree]; j++) {
+    uint16_t t;
+    gal::credit_frees(s, gal::block_of(s, sm.at[tree][j], t), sm.len[tree][j]);
+  }
+  for (uint32_t k = 0; k < n; k++)
+    if (used[k]) gal::credit_frees(s, blks[k], used[k]);
+}
+
 // One thread: a segment of class `tree` with one block left to give, whose count
 // a reservation meant for an earlier owner takes below zero; a request that
 // meets it then; the reservation given back.  `fresh`: a segment gathered ahead,
@@ -136,6 +185,11 @@ int dev_churn(const gal::state *s, uint32_t ctas, uint32_t threads, uint32_t tur
 
 int dev_fill(const gal::state *s, uint64_t size, uint64_t n, void **out) {
   RUN(k_fill<<<(unsigned)((n + 255) / 256), 256>>>(s, size, n, out));
+}
+
+int dev_chunk_claim(const gal::state *s, uint32_t tree, uint32_t want, uint32_t slot_left, uint32_t spare_left,
+                    unsigned long long *out) {
+  RUN(k_chunk_claim<<<1, 1>>>(s, tree, want, slot_left, spare_left, out));
 }
 
 int dev_give_back(const gal::state *s, uint32_t tree, int fresh, unsigned long long *out) {

@@ -21,6 +21,7 @@ def D():
     L.dev_blocks.argtypes = [vp, u64, u32, u32, u32, u32, u64, vp, vp]
     L.dev_churn.argtypes = [vp, u32, u32, u32, u32, u32, C.c_int, u64, vp]
     L.dev_fill.argtypes = [vp, u64, u64, vp]
+    L.dev_chunk_claim.argtypes = [vp, u32, u32, u32, u32, vp]
     L.dev_give_back.argtypes = [vp, u32, C.c_int, vp]
     return L
 
@@ -92,6 +93,32 @@ def test_one_request_per_thread_until_nothing_is_left(D, size):
         assert g.error_word() == 0, g.error_info()
         g.free_per_thread(ptrs)
         torch.cuda.synchronize()
+        _as_fresh(g, fresh)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("spares", [0, 1])
+@pytest.mark.parametrize("slot_left,spare_left,want,left", [
+    (0, 4096, 100, 3996),      # a block that nobody replaces
+    (6, 96, 200, 3998),        # the next one used up by this claim
+    (6, 0, 200, 3902),         # ... or already by others
+    (200, 70, 200, 70),        # nothing more wanted
+    (50, 4096, 4095, 51),
+])
+def test_chunk_claim_of_blocks_used_up_by_slow_teams(D, slot_left, spare_left, want, left, spares):
+    """A chunk's claim gets all its slices and leaves a block to claim from in the
+    slot, whatever slow teams took of the pinned block and of its successor."""
+    import torch
+    import gallatin_gb300 as G
+    out = torch.zeros(4, dtype=torch.int64, device="cuda")
+    g = G.Gallatin.generate_on_device(2 * GIB, 42, zero_arena=0, spare_blocks=spares)
+    try:
+        fresh = g.export()
+        assert D.dev_chunk_claim(g.device_state, 2, want, slot_left, spare_left, out.data_ptr()) == 0
+        claimed, runs, there, unread = out.tolist()
+        assert claimed == want and unread == 0
+        assert there == (left if spares else 4096 - (want - slot_left))
         _as_fresh(g, fresh)
     finally:
         g.close()
