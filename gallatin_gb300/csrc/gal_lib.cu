@@ -456,6 +456,7 @@ int build(uint64_t num_bytes, uint64_t seed, const gal_config *cfg_in, bool boot
   st.error = (uint32_t *)(m + o_err);
   h->d_state = (gal::state *)(m + o_state);
   h->d_stats = (gal_stats *)(m + o_stats);
+  st.resident = h->d_state;
 
   int rc = GAL_OK;
   do {

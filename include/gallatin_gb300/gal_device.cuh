@@ -71,7 +71,9 @@ struct veb_shape {
 };
 
 // Everything a kernel needs; lives in device memory (the object a
-// Gallatin<>* points to) and may also be passed by value as a kernel param.
+// Gallatin<>* points to).  A copy of it, passed by value as a kernel parameter
+// or kept in shared, local or constant memory, stands for that object: the
+// device calls take either (see resident).
 struct state {
   char *memory;
   uint64_t num_segments;
@@ -109,6 +111,7 @@ struct state {
                                  // (gal_config.spare_blocks; NOBLK: none)
   uint32_t *locks;               // lock word of tree t at t * LOCK_STRIDE; runs at num_trees
   uint32_t *error;               // GAL_DEV_ERR_* bits
+  const state *resident;         // the state in device memory that this is (a copy of)
 };
 
 // A field of the state (or of its tree shape), which lives in global memory, on
@@ -128,6 +131,11 @@ GAL_DEVICE_INLINE __host__ T cfield(const T &f) {
 #else
   return f;
 #endif
+}
+// cfield reads global memory; a copy of the state elsewhere names the one there.
+// (A kernel's parameters lie in a window of the global address space.)
+GAL_DEVICE_INLINE const state *resident(const state *s) {
+  return __isGlobal(s) && !__isGridConstant(s) ? s : s->resident;
 }
 
 // ------------------------------------------------------------------ layout
@@ -1554,7 +1562,7 @@ GAL_DEVICE_INLINE void *malloc_from(const state *s, uint64_t size, uint32_t call
 // Gallatin::malloc as the reference calls it: each attempt's team is the lanes
 // executing it together (its coalesced_threads(), gallatin.cuh:883).
 GAL_DEVICE_INLINE void *malloc(const state *s, uint64_t size) {
-  return malloc_from<false>(s, size, active_lanes());
+  return malloc_from<false>(resident(s), size, active_lanes());
 }
 
 // malloc for kernels whose CTAs serve many requests (persistent loops): the
@@ -1563,7 +1571,7 @@ GAL_DEVICE_INLINE void *malloc(const state *s, uint64_t size) {
 // a team's claim costs one L2 round trip instead of two.  Same results
 // contract as malloc.
 GAL_DEVICE_INLINE void *malloc_cached(const state *s, uint64_t size, slot_cache &cache) {
-  return malloc_from<false>(s, size, active_lanes(), &cache);
+  return malloc_from<false>(resident(s), size, active_lanes(), &cache);
 }
 
 // malloc with the calling lanes named: every lane of `callers` calls with the
@@ -1571,7 +1579,7 @@ GAL_DEVICE_INLINE void *malloc_cached(const state *s, uint64_t size, slot_cache 
 // for slices of one class form one team whatever grouping of diverged lanes
 // the scheduler chose.
 GAL_DEVICE_INLINE void *malloc_team(const state *s, uint64_t size, uint32_t callers) {
-  return malloc_from<true>(s, size, callers);
+  return malloc_from<true>(resident(s), size, callers);
 }
 
 // multi-segment free (gallatin.cuh:1394-1417, 1283-1302), id reset first
@@ -1587,6 +1595,7 @@ GAL_DEVICE_COLD void free_segment_run(const state *s, uint64_t seg, uint16_t tre
 
 // Gallatin::free (gallatin.cuh:1378-1461)
 GAL_DEVICE_INLINE void free(const state *s, void *ptr) {
+  s = resident(s);
   uint64_t off = (uint64_t)((char *)ptr - cfield(s->memory));
   uint64_t seg = off >> cfield(s->seg_shift);
   if (seg >= cfield(s->num_segments)) {
@@ -1611,6 +1620,7 @@ GAL_DEVICE_INLINE void free(const state *s, void *ptr) {
 // follows from the size, so the pointer's segment need not be looked up (the
 // first of free's two dependent round trips).
 GAL_DEVICE_INLINE void free_sized(const state *s, void *ptr, uint64_t size) {
+  s = resident(s);
   const int T = (int)cfield(s->num_trees), min_shift = (int)cfield(s->min_shift);
   const int bits = size > 1 ? 64 - __clzll((long long)(size - 1)) : 0;
   const int t = max(bits - min_shift, 0);
@@ -1626,6 +1636,7 @@ GAL_DEVICE_INLINE void free_sized(const state *s, void *ptr, uint64_t size) {
 
 // block id of a live pointer (slice or whole block), NOBLK for a segment run
 GAL_DEVICE_INLINE uint32_t block_of(const state *s, const void *ptr, uint16_t &tree_out) {
+  s = resident(s);
   uint64_t off = (uint64_t)((const char *)ptr - cfield(s->memory));
   uint64_t seg = off >> cfield(s->seg_shift);
   uint16_t tree = seg < cfield(s->num_segments) ? ld_rlx(&cfield(s->tree_ids)[seg]) : FREE_TREE;
@@ -1644,6 +1655,7 @@ GAL_DEVICE_INLINE uint32_t block_of(const state *s, const void *ptr, uint16_t &t
 template <int N>
 GAL_DEVICE_INLINE void free_n(const state *s, void *const (&p)[N], const bool (&go)[N],
                               const uint16_t *classes = nullptr) {
+  s = resident(s);
   uint16_t tree[N];
   uint64_t off[N];
 #pragma unroll
@@ -1687,6 +1699,7 @@ GAL_DEVICE_INLINE void free_n(const state *s, void *const (&p)[N], const bool (&
 // __syncthreads().  Returns false (nothing staged) for larger arenas.
 static constexpr uint32_t CLASS_STAGE_BYTES = 32768;
 GAL_DEVICE_INLINE bool stage_classes(const state *s, uint16_t *smem) {
+  s = resident(s);
   if (cfield(s->num_segments) * 2 > CLASS_STAGE_BYTES) return false;
   for (uint64_t g = threadIdx.x; g < cfield(s->num_segments); g += blockDim.x) smem[g] = ld_rlx(&cfield(s->tree_ids)[g]);
   return true;
@@ -1700,6 +1713,7 @@ GAL_DEVICE_INLINE uint32_t export_mword(const state *s, uint32_t blk) {
 
 // bytes a request of `size` occupies (Gallatin::get_allocated_size, gallatin.cuh:1152-1183)
 GAL_DEVICE_INLINE uint64_t allocated_size(const state *s, uint64_t size) {
+  s = resident(s);
   if (size < 16) size = 16;
   int bits = ceil_log2(size);
   int tree = bits - (int)cfield(s->min_shift);
@@ -1711,6 +1725,7 @@ GAL_DEVICE_INLINE uint64_t allocated_size(const state *s, uint64_t size) {
 }
 
 GAL_DEVICE_INLINE bool owns(const state *s, const void *p) {
+  s = resident(s);
   return (uint64_t)((const char *)p - cfield(s->memory)) < (cfield(s->num_segments) << cfield(s->seg_shift));
 }
 

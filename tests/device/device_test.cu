@@ -91,6 +91,63 @@ __global__ void k_fill(const gal::state *s, uint64_t size, uint64_t n, void **ou
   if (i < n) out[i] = gal::malloc(s, size);
 }
 
+// Every device call once through `s`, wherever that state is kept.  out: failed,
+// wrong answers, in the way of k_churn's stamps.
+__device__ void every_call(const gal::state *s, uint64_t seed, gal::slot_cache &cache, unsigned long long *out) {
+  const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int k = 0; k < 6; k++) {
+    const uint64_t size = 16 + mix(seed + 8 * me + k) % 9000;
+    uint64_t *p = (uint64_t *)(k % 3 == 0 ? gal::malloc(s, size)
+                               : k % 3 == 1 ? gal::malloc_cached(s, size, cache)
+                                            : gal::malloc_team(s, size, 0xFFFFFFFFu));
+    bool ok = p != nullptr;
+    if (ok) {
+      p[0] = p[size / 8 - 1] = me;
+      uint16_t tree;
+      const uint64_t held = gal::allocated_size(s, size);
+      ok = gal::owns(s, p) && held >= size && held < 2 * size && gal::block_of(s, p, tree) != gal::NOBLK;
+    }
+    __syncwarp();
+    ok = ok && p[0] == me && p[size / 8 - 1] == me;
+    if (!ok) atomicAdd(&out[p ? 1 : 0], 1ull);
+    if (p && k == 0) {
+      gal::free(s, p);
+    } else if (p && k == 1) {
+      gal::free_sized(s, p, size);
+    } else if (p) {
+      void *const list[1] = {p};
+      const bool go[1] = {true};
+      gal::free_n<1>(s, list, go);
+    }
+    __syncwarp();
+  }
+}
+__constant__ gal::state constant_state;
+__global__ void k_state_pointer(const gal::state *s, int form, uint64_t seed, unsigned long long *out) {
+  __shared__ gal::slot_cache cache;
+  __shared__ gal::state copy;
+  gal::slot_cache_init(cache);
+  if (threadIdx.x == 0) copy = *s;
+  __syncthreads();
+  gal::state local = *s;
+  if (form == 0) every_call(s, seed, cache, out);
+  if (form == 1) every_call(&copy, seed, cache, out);
+  if (form == 2) every_call(&local, seed, cache, out);
+  if (form == 3) every_call(&constant_state, seed, cache, out);
+}
+__global__ void k_state_value(const gal::state s, uint64_t seed, unsigned long long *out) {
+  __shared__ gal::slot_cache cache;
+  gal::slot_cache_init(cache);
+  __syncthreads();
+  every_call(&s, seed, cache, out);
+}
+__global__ void k_state_grid_constant(const __grid_constant__ gal::state s, uint64_t seed, unsigned long long *out) {
+  __shared__ gal::slot_cache cache;
+  gal::slot_cache_init(cache);
+  __syncthreads();
+  every_call(&s, seed, cache, out);
+}
+
 // Of block `blk` all slices but `left` handed out; the number that were not yet.
 __device__ uint32_t use_up(const gal::state *s, uint32_t blk, uint32_t left) {
   const uint32_t count = (uint32_t)gal::ld_rlx(gal::mword_ptr(s, blk)), to = gal::SLICES_PER_BLOCK - left;
@@ -185,6 +242,21 @@ int dev_churn(const gal::state *s, uint32_t ctas, uint32_t threads, uint32_t tur
 
 int dev_fill(const gal::state *s, uint64_t size, uint64_t n, void **out) {
   RUN(k_fill<<<(unsigned)((n + 255) / 256), 256>>>(s, size, n, out));
+}
+
+// form: the state in global (0), shared (1), local (2) or constant memory (3), a
+// kernel's parameter (4) or one whose address is taken (5)
+int dev_state_copy(const gal::state *s, int form, uint64_t seed, unsigned long long *out) {
+  gal::state value;
+  if (cudaMemcpy(&value, s, sizeof(value), cudaMemcpyDeviceToHost) != cudaSuccess) return 3;
+  if (cudaMemcpyToSymbol(constant_state, &value, sizeof(value)) != cudaSuccess) return 4;
+  if (form < 4) {
+    RUN(k_state_pointer<<<32, 128>>>(s, form, seed, out));
+  } else if (form == 4) {
+    RUN(k_state_value<<<32, 128>>>(value, seed, out));
+  } else {
+    RUN(k_state_grid_constant<<<32, 128>>>(value, seed, out));
+  }
 }
 
 int dev_chunk_claim(const gal::state *s, uint32_t tree, uint32_t want, uint32_t slot_left, uint32_t spare_left,

@@ -21,6 +21,7 @@ def D():
     L.dev_blocks.argtypes = [vp, u64, u32, u32, u32, u32, u64, vp, vp]
     L.dev_churn.argtypes = [vp, u32, u32, u32, u32, u32, C.c_int, u64, vp]
     L.dev_fill.argtypes = [vp, u64, u64, vp]
+    L.dev_state_copy.argtypes = [vp, C.c_int, u64, vp]
     L.dev_chunk_claim.argtypes = [vp, u32, u32, u32, u32, vp]
     L.dev_give_back.argtypes = [vp, u32, C.c_int, vp]
     return L
@@ -93,6 +94,23 @@ def test_one_request_per_thread_until_nothing_is_left(D, size):
         assert g.error_word() == 0, g.error_info()
         g.free_per_thread(ptrs)
         torch.cuda.synchronize()
+        _as_fresh(g, fresh)
+    finally:
+        g.close()
+
+
+@pytest.mark.parametrize("form", range(6), ids=["global", "shared", "local", "constant", "parameter", "grid-constant"])
+def test_state_by_value(D, form):
+    """Every device call through the state itself and through copies of it."""
+    import torch
+    import gallatin_gb300 as G
+    out = torch.zeros(2, dtype=torch.int64, device="cuda")
+    g = G.Gallatin.generate_on_device(4 * GIB, 42, zero_arena=0, spare_blocks=1)
+    try:
+        fresh = g.export()
+        for seed in range(3):
+            assert D.dev_state_copy(g.device_state, form, seed << 32, out.data_ptr()) == 0
+            assert out.tolist() == [0, 0]
         _as_fresh(g, fresh)
     finally:
         g.close()
