@@ -225,6 +225,18 @@ GAL_DEVICE_INLINE uint64_t amo_or(uint64_t *p, uint64_t v) {
 GAL_DEVICE_INLINE uint64_t amo_and(uint64_t *p, uint64_t v) {
   return atomicAnd((unsigned long long *)p, (unsigned long long)v);
 }
+// ... whose later accesses by this thread stay after them; a set that also stays
+// after its earlier ones
+GAL_DEVICE_INLINE uint64_t and_acquire(uint64_t *p, uint64_t v) {
+  uint64_t r;
+  asm volatile("atom.acquire.gpu.global.and.b64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(v) : "memory");
+  return r;
+}
+GAL_DEVICE_INLINE uint64_t or_acq_rel(uint64_t *p, uint64_t v) {
+  uint64_t r;
+  asm volatile("atom.acq_rel.gpu.global.or.b64 %0, [%1], %2;" : "=l"(r) : "l"(p), "l"(v) : "memory");
+  return r;
+}
 // atomicAdd whose later accesses by this thread stay after it
 GAL_DEVICE_INLINE unsigned long long add_acquire(unsigned long long *p, unsigned long long v) {
   unsigned long long r;
@@ -360,20 +372,24 @@ GAL_DEVICE_COLD void veb_unlist(uint64_t *w, const veb_shape *sh, uint32_t word)
 // while the re-read still saw the empty word, leaving a non-empty word behind
 // a clear summary bit, where top-down searches never find its items.
 // `left` receives the other items the bottom word held.
+// ACQUIRE: with all that the item's insert came after (see veb_insert).
+template <bool ACQUIRE = false>
 GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x, uint64_t &left) {
   const int layer = (int)cfield(v.sh->layers) - 1;
   const uint64_t high = x >> 6;
   const int low = (int)(x & 63);
-  const uint64_t old = amo_and(v.word(layer, high), ~(1ULL << low));
+  const uint64_t keep = ~(1ULL << low);
+  const uint64_t old = ACQUIRE ? and_acquire(v.word(layer, high), keep) : amo_and(v.word(layer, high), keep);
   left = old & ~(1ULL << low);
   if (!(old & (1ULL << low))) return false;
   if (left == 0) veb_unlist(v.w, v.sh, (uint32_t)high);
   return true;
 }
 
+template <bool ACQUIRE = false>
 GAL_DEVICE_INLINE bool veb_remove(const veb_ref &v, uint64_t x) {
   uint64_t left;
-  return veb_remove(v, x, left);
+  return veb_remove<ACQUIRE>(v, x, left);
 }
 
 // Lists a bottom word this thread found empty in the summaries above it.
@@ -388,11 +404,14 @@ GAL_DEVICE_COLD void veb_list_above(uint64_t *w, const veb_shape *sh, uint32_t w
 }
 
 // veb_tree::insert_force_update (veb.cuh:775-798); the fence orders each
-// word's set before its summary's (see veb_remove)
+// word's set before its summary's (see veb_remove).  ORDERED: the item is there after
+// all that this thread has done and seen, and before all that it does next.
+template <bool ORDERED = false>
 GAL_DEVICE_INLINE bool veb_insert(const veb_ref &v, uint64_t x) {
   const int layer = (int)cfield(v.sh->layers) - 1;
   const uint64_t high = x >> 6;
-  const uint64_t old = amo_or(v.word(layer, high), 1ULL << (x & 63));
+  const uint64_t bit = 1ULL << (x & 63);
+  const uint64_t old = ORDERED ? or_acq_rel(v.word(layer, high), bit) : amo_or(v.word(layer, high), bit);
   if (old == 0) veb_list_above(v.w, v.sh, (uint32_t)high);
   return !((old >> (x & 63)) & 1ULL);
 }
@@ -889,17 +908,15 @@ GAL_DEVICE_INLINE bool serves(const state *s, uint32_t tree, uint64_t seg) {
 // its class's tree: by the thread that took its last block, or by any that
 // finds it listed meanwhile, so that nobody waits for the former.  Blocks may
 // have come home since, so the segment is listed again if it has one to give
-// (the fence: who raised the count and listed the segment before this removal
-// is seen here, who lists it after it undoes the removal).
+// (who raised the count and listed the segment before this removal is seen
+// here, who lists it after it undoes the removal).
 // The release of a segment closes its count word before it unlists it, so a
 // listing made here and still valid when the word is read again is either right
 // or taken off by the release.  One thread alone never finds such a segment.
 GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
-  for (uint32_t tries = 0; veb_remove(sub_tree(s, tree), seg); tries++) {
-    fence_acq_rel();
+  for (uint32_t tries = 0; veb_remove<true>(sub_tree(s, tree), seg); tries++) {
     if (!serves(s, tree, seg)) return;
-    veb_insert(sub_tree(s, tree), seg);
-    fence_acq_rel();
+    veb_insert<true>(sub_tree(s, tree), seg);
     if (serves(s, tree, seg)) return;
     if (tries >= cfield(s->spin_limit)) {  // left listed: the next search meets it again
       set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_UNLIST, tree, seg);
@@ -908,14 +925,12 @@ GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg
   }
 }
 
-// Lists a segment whose count this thread has raised (after a fence).  Raised
-// first: a search that found the segment listed and its count still negative
+// Lists a segment whose count this thread has raised.  Raised first: a search that found the segment listed and its count still negative
 // would take it off, and the next listing is a lap of the ring away.  The
 // segment may have been emptied, or released and set up for another class, in
 // between: then it does not stay listed.
 GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint64_t seg) {
-  veb_insert(sub_tree(s, tree), seg);
-  fence_acq_rel();
+  veb_insert<true>(sub_tree(s, tree), seg);
   if (!serves(s, tree, seg)) unlist_refusing(s, tree, seg);
 }
 
@@ -927,14 +942,12 @@ GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint64_t seg) {
 GAL_DEVICE_COLD bool release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
   const unsigned long long home = act_word(gen, tree, (int32_t)nb - 1);
   if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return false;
-  fence_acq_rel();
+  fence_acq_rel();  // closed before it is taken off (see unlist_refusing)
   veb_remove(sub_tree(s, tree), seg);
-  fence_acq_rel();
   // closed and unlisted, the segment is this thread's alone
   if (ld_rlx(&cfield(s->tree_ids)[seg]) != (uint16_t)tree) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
   st_rlx(&cfield(s->tree_ids)[seg], FREE_TREE);
-  fence_acq_rel();
-  veb_insert(seg_tree(s), seg);
+  veb_insert<true>(seg_tree(s), seg);
   return true;
 }
 
