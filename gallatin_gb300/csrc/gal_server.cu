@@ -74,7 +74,10 @@ __device__ __forceinline__ bool stamps_ok(const void *p, uint64_t size, uint64_t
   return q[0] == id && *(const uint64_t *)((const char *)p + ((size - 8) & ~7ull)) == id;
 }
 
-__global__ void __launch_bounds__(SRV_BT)
+// Registers for three CTAs per SM: left to itself the compiler takes 64, 80 or 128
+// from one build to the next.  Direct producers of 16-4,096 B: 0.70 ms a step at
+// 80, 0.76 at 64; the three bench streams 1.05-1.12 ms at either.
+__global__ void __launch_bounds__(SRV_BT, 3)
     k_server_step(const gal::state *s, gal::server_rings r, streams_param sp, uint32_t server_ctas, int direct,
                   unsigned long long *stats) {
   __shared__ gal::server_smem sm;

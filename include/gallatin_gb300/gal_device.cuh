@@ -913,25 +913,30 @@ GAL_DEVICE_INLINE bool serves(const state *s, uint32_t tree, uint64_t seg) {
 // The release of a segment closes its count word before it unlists it, so a
 // listing made here and still valid when the word is read again is either right
 // or taken off by the release.  One thread alone never finds such a segment.
-GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
-  for (uint32_t tries = 0; veb_remove<true>(sub_tree(s, tree), seg); tries++) {
-    if (!serves(s, tree, seg)) return;
-    veb_insert<true>(sub_tree(s, tree), seg);
-    if (serves(s, tree, seg)) return;
+// (Its two steps are functions of their own, so that little is kept across the
+// calls they make: a kernel that frees needs 48 registers, 54 with them inlined.)
+GAL_DEVICE_COLD bool listing_off(const state *s, uint32_t tree, uint32_t seg) {
+  return !veb_remove<true>(sub_tree(s, tree), seg) || !serves(s, tree, seg);
+}
+GAL_DEVICE_COLD bool listing_on(const state *s, uint32_t tree, uint32_t seg) {
+  veb_insert<true>(sub_tree(s, tree), seg);
+  return serves(s, tree, seg);
+}
+GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint32_t seg) {
+  for (uint32_t tries = 0; !listing_off(s, tree, seg) && !listing_on(s, tree, seg); tries++)
     if (tries >= cfield(s->spin_limit)) {  // left listed: the next search meets it again
       set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_UNLIST, tree, seg);
       return;
     }
-  }
 }
 
-// Lists a segment whose count this thread has raised.  Raised first: a search that found the segment listed and its count still negative
-// would take it off, and the next listing is a lap of the ring away.  The
-// segment may have been emptied, or released and set up for another class, in
-// between: then it does not stay listed.
-GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint64_t seg) {
-  veb_insert<true>(sub_tree(s, tree), seg);
-  if (!serves(s, tree, seg)) unlist_refusing(s, tree, seg);
+// Lists a segment whose count this thread has raised.  Raised first: a search
+// that found the segment listed and its count still negative would take it off,
+// and the next listing is a lap of the ring away.  The segment may have been
+// emptied, or released and set up for another class, in between: then it does
+// not stay listed.
+GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint32_t seg) {
+  if (!listing_on(s, tree, seg)) unlist_refusing(s, tree, seg);
 }
 
 // Releases segment `seg` of class `tree` when its count word still reads
