@@ -158,7 +158,7 @@ static __device__ void retire_tile(const state *s, const uint32_t (&blk)[RETIRE]
     atomicAdd(&s->qfc[g], n);
     atomicAdd(&s->fqfc[g], n);
     const unsigned long long old = atomicAdd(&s->act[g], (unsigned long long)n);
-    if (act_count(old) + (int32_t)n == (int32_t)nb - 1) release_segment(s, g, t, act_gen(old), nb);
+    if (act_count(old) + (int32_t)n == (int32_t)nb - 1) release_segment(s, g, t, act_gen(old), nb, NOSEG);
   }
   __syncthreads();
 }

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(gal::BOOT_THREADS) k_trim(const gal::state *s)
     const uint32_t nb = gal::blocks_in_segment(s, tree);
     const unsigned long long w = gal::ld_rlx(&s->act[seg]);
     if (gal::act_count(w) != (int32_t)nb - 1) continue;
-    gal::release_segment(s, seg, tree, gal::act_gen(w), nb);
+    gal::release_segment(s, seg, tree, gal::act_gen(w), nb, gal::NOSEG);
   }
   gal::fence_acq_rel();
   __syncthreads();

@@ -153,6 +153,7 @@ GAL_DEVICE_INLINE __host__ uint32_t *fctr_ptr(const state *s, uint32_t blk) {
 // which holds the class that owns the segment (ACT_FREE: none) in its low byte
 // and the set-up generation in the rest.  The atomic that reserves a block
 // thus also says whose segment it was taken from, with no second word to read.
+static constexpr uint32_t NOSEG = 0xFFFFFFFFu;  // no segment
 static constexpr uint32_t ACT_BIAS = 0x80000000u;
 static constexpr uint32_t ACT_FREE = 0xFFu;
 GAL_DEVICE_INLINE __host__ int32_t act_unbias(uint32_t low) { return (int32_t)(low - ACT_BIAS); }
@@ -288,7 +289,7 @@ enum : uint64_t {
   SITE_REQUEST_LOCK = 6,   // request_block: the class lock stayed taken (a: class, b: spins)
   SITE_REQUEST_RETRY = 7,  // request_block: listed segments kept refusing a block (a: class, b: last segment)
   SITE_RUN_LOCK = 8,       // malloc_segment_run: the run lock stayed taken (a: segments wanted)
-  SITE_UNLIST = 9,         // unlist_refusing: the segment kept changing (a: class, b: segment)
+  SITE_LISTING = 9,        // settle_listing: the segment kept changing (a: class, b: segment)
 };
 GAL_DEVICE_INLINE void backoff(uint32_t i) { __nanosleep(i < 8 ? 32u << i : 4096u); }
 
@@ -904,56 +905,64 @@ GAL_DEVICE_INLINE bool serves(const state *s, uint32_t tree, uint64_t seg) {
   return act_class(w) == tree && act_count(w) >= 0;
 }
 
-// Takes a segment that has no block to give (or is another class's by now) off
-// its class's tree: by the thread that took its last block, or by any that
-// finds it listed meanwhile, so that nobody waits for the former.  Blocks may
-// have come home since, so the segment is listed again if it has one to give
-// (who raised the count and listed the segment before this removal is seen
-// here, who lists it after it undoes the removal).
-// The release of a segment closes its count word before it unlists it, so a
-// listing made here and still valid when the word is read again is either right
-// or taken off by the release.  One thread alone never finds such a segment.
-// (Its two steps are functions of their own, so that little is kept across the
-// calls they make: a kernel that frees needs 48 registers, 54 with them inlined.)
-GAL_DEVICE_COLD bool listing_off(const state *s, uint32_t tree, uint32_t seg) {
-  return !veb_remove<true>(sub_tree(s, tree), seg) || !serves(s, tree, seg);
-}
+// The two steps of a listing; true: it agrees with the count.
 GAL_DEVICE_COLD bool listing_on(const state *s, uint32_t tree, uint32_t seg) {
   veb_insert<true>(sub_tree(s, tree), seg);
   return serves(s, tree, seg);
 }
-GAL_DEVICE_COLD void unlist_refusing(const state *s, uint32_t tree, uint32_t seg) {
-  for (uint32_t tries = 0; !listing_off(s, tree, seg) && !listing_on(s, tree, seg); tries++)
-    if (tries >= cfield(s->spin_limit)) {  // left listed: the next search meets it again
-      set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_UNLIST, tree, seg);
-      return;
-    }
+GAL_DEVICE_COLD bool listing_off(const state *s, uint32_t tree, uint32_t seg) {
+  return !veb_remove<true>(sub_tree(s, tree), seg) || !serves(s, tree, seg);
 }
-
-// Lists a segment whose count this thread has raised.  Raised first: a search
-// that found the segment listed and its count still negative would take it off,
-// and the next listing is a lap of the ring away.  The segment may have been
-// emptied, or released and set up for another class, in between: then it does
-// not stay listed.
-GAL_DEVICE_COLD void list_serving(const state *s, uint32_t tree, uint32_t seg) {
-  if (!listing_on(s, tree, seg)) unlist_refusing(s, tree, seg);
+// Makes the listing of a segment in the tree of class `tree` agree with its count.
+//   listed: it is, but has no block to give (or is another class's by now).  It is
+//     taken off by the thread that took its last block, or by any that finds it
+//     meanwhile, so that nobody waits for the former.  Blocks may have come home
+//     since, and then it is listed again (who raised the count and listed the
+//     segment before this removal is seen here, who lists it after it undoes
+//     the removal).
+//   not listed: this thread has raised its count.  Raised first: a search that
+//     found the segment listed and its count still negative would take it off,
+//     and the next listing is a lap of the ring away.  The segment may have been
+//     emptied, or released and set up for another class, in between: then it
+//     does not stay listed.
+// The release of a segment closes its count word before it unlists it, so a
+// listing made here and still valid when the word is read again is either right
+// or taken off by the release.  One thread alone never has to undo a step.
+// (The steps are functions of their own, and whoever returns blocks calls this
+// after return_block, not inside it: the registers of a chain of calls add up in
+// every kernel that frees.)
+GAL_DEVICE_COLD void settle_listing(const state *s, uint32_t tree, uint32_t seg, bool listed) {
+  for (uint32_t tries = 0; tries < cfield(s->spin_limit); tries++) {
+    if (!listed && listing_on(s, tree, seg)) return;
+    if (listing_off(s, tree, seg)) return;
+    listed = false;
+  }
+  if (!listing_on(s, tree, seg))  // left listed: the next search meets it again
+    set_error_info(s, GAL_DEV_ERR_TIMEOUT, SITE_LISTING, tree, seg);
+}
+GAL_DEVICE_INLINE void unlist_refusing(const state *s, uint32_t tree, uint64_t seg) {
+  settle_listing(s, tree, (uint32_t)seg, true);
+}
+GAL_DEVICE_INLINE void list_serving(const state *s, uint32_t tree, uint64_t seg) {
+  settle_listing(s, tree, (uint32_t)seg, false);
 }
 
 // Releases segment `seg` of class `tree` when its count word still reads
 // `gen` with every block home (nb - 1): removes it from the class's tree,
 // frees its class and lists it in the segment tree (the release steps of
 // Gallatin::return_block, gallatin.cuh:1663-1722, finish_freeing_block,
-// memory_table.cuh:1226-1241).
-GAL_DEVICE_COLD bool release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb) {
+// memory_table.cuh:1226-1241).  NOSEG, or `list` when the segment has moved on.
+GAL_DEVICE_COLD uint32_t release_segment(const state *s, uint64_t seg, uint32_t tree, uint32_t gen, uint32_t nb,
+                                         uint32_t list) {
   const unsigned long long home = act_word(gen, tree, (int32_t)nb - 1);
-  if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return false;
-  fence_acq_rel();  // closed before it is taken off (see unlist_refusing)
+  if (atomicCAS(&cfield(s->act)[seg], home, act_word(gen, ACT_FREE, -1)) != home) return list;
+  fence_acq_rel();  // closed before it is taken off (see settle_listing)
   veb_remove(sub_tree(s, tree), seg);
   // closed and unlisted, the segment is this thread's alone
   if (ld_rlx(&cfield(s->tree_ids)[seg]) != (uint16_t)tree) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
   st_rlx(&cfield(s->tree_ids)[seg], FREE_TREE);
   veb_insert<true>(seg_tree(s), seg);
-  return true;
+  return NOSEG;
 }
 
 // Gives back a reservation taken from segment `seg` that no block came of.
@@ -970,7 +979,7 @@ GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
   if (tree >= cfield(s->num_trees) || act_count(old) + 1 < 0) return;
   const uint32_t nb = blocks_in_segment(s, tree);
   if (act_count(old) + 1 == (int32_t)nb - 1 && ld_rlx(&cfield(s->qc)[seg]) != 0 &&
-      release_segment(s, seg, tree, act_gen(old), nb))
+      release_segment(s, seg, tree, act_gen(old), nb, 0) == NOSEG)
     return;
   list_serving(s, tree, seg);
 }
@@ -1049,7 +1058,6 @@ GAL_DEVICE_INLINE uint32_t more_segments(const state *s, uint32_t tree, uint32_t
 // (alone, a thread always finds the lock free): each would add a segment to a
 // class that needs one, and threads that take a class's last blocks together
 // would leave it holding hundreds.
-static constexpr uint32_t NOSEG = 0xFFFFFFFFu;
 static constexpr uint32_t SEG_UNLISTED = 0x80000000u;  // with a segment: it was never listed
 GAL_DEVICE_COLD void finish_emptied(const state *s, uint32_t tree, uint32_t emptied) {
   if (cfield(s->gather_ahead)) {
@@ -1142,12 +1150,13 @@ GAL_DEVICE_INLINE uint32_t request_block(const state *s, uint32_t tree, uint32_t
 
 // Gallatin::return_block (gallatin.cuh:1637-1726) with reserve_segment_slot,
 // finalize_free_queue and finish_freeing_block (memory_table.cuh:906-910,1158-1241)
-GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
+// Returns what is to be listed after it (see block_returned; NOSEG: nothing).
+GAL_DEVICE_COLD uint32_t return_block(const state *s, uint32_t blk) {
   uint64_t seg = blk >> cfield(s->bps_shift);
   uint16_t tree = ld_rlx(&cfield(s->tree_ids)[seg]);
   if (tree >= cfield(s->num_trees)) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_RETURN_BAD_TREE, blk, tree);
-    return;
+    return NOSEG;
   }
   uint32_t nb = blocks_in_segment(s, tree);
   uint32_t pos = atomicAdd(&cfield(s->qfc)[seg], 1u);
@@ -1164,12 +1173,15 @@ GAL_DEVICE_COLD void return_block(const state *s, uint32_t blk) {
   // (live-1)/nb < 0.1 in doubles; for the power-of-two nb used here that is
   // 10*live > nb >= 10*(live-1) with live-1 taken as unsigned (live 0 never).
   const bool crossing = live != 0 && 10ull * live > nb && 10ull * (live - 1) < nb;
+  const uint32_t list = crossing ? (uint32_t)seg << 8 | tree : NOSEG;
   fence_acq_rel();  // the ring entry before the count that lets it be handed out
   const unsigned long long old = add_acquire(&cfield(s->act)[seg], 1ull);
-  if ((uint32_t)(act_count(old) + 2) == nb &&  // all_blocks_free: the count was nb - 2
-      release_segment(s, seg, tree, act_gen(old), nb))
-    return;
-  if (crossing) list_serving(s, tree, seg);
+  if ((uint32_t)(act_count(old) + 2) == nb)  // all_blocks_free: the count was nb - 2
+    return release_segment(s, seg, tree, act_gen(old), nb, list);
+  return list;
+}
+GAL_DEVICE_INLINE void block_returned(const state *s, uint32_t list) {
+  if (list != NOSEG) list_serving(s, list & 0xFFu, list >> 8);
 }
 
 // Block::block_free_multiple + reset_free + free_block (block.cuh:87-98,200-212,
@@ -1182,7 +1194,7 @@ GAL_DEVICE_INLINE void credit_frees(const state *s, uint32_t blk, uint32_t n) {
 GAL_DEVICE_INLINE void credit_done(const state *s, uint32_t blk, uint32_t old, uint32_t n) {
   if (old + n == SLICES_PER_BLOCK) {
     st_rlx(fctr_ptr(s, blk), 0u);  // published with the block's ring entry
-    return_block(s, blk);
+    block_returned(s, return_block(s, blk));
   } else if (old + n > SLICES_PER_BLOCK) {
     set_error_info(s, GAL_DEV_ERR_BAD_FREE, SITE_FREE_OVERFLOW, blk,
                    ((uint64_t)old << 32) | n);

@@ -23,7 +23,7 @@ __device__ __forceinline__ uint64_t mix(uint64_t z) {
 __global__ void k_blocks(const gal::state *s, uint64_t size, uint32_t turns, uint32_t keep, uint64_t seed,
                          void **kept, unsigned long long *failed) {
   const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  void *held[4];
+  void *held[4] = {};
   uint32_t n = 0;
   for (uint32_t j = 0; j < 4; j++)
     if (kept[4 * me + j]) held[n++] = kept[4 * me + j];
@@ -52,7 +52,7 @@ __global__ void k_churn(const gal::state *s, uint32_t turns, uint32_t hi_bits, u
   gal::slot_cache_init(cache);
   __syncthreads();
   const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  uint64_t *held[5], len[5], id[5];
+  uint64_t *held[5] = {}, len[5] = {}, id[5] = {};
   uint32_t n = 0, bad = 0, failed = 0;
   auto drop = [&]() {  // the oldest
     bad += held[0][0] != id[0] || held[0][len[0] / 8 - 1] != id[0];
