@@ -226,12 +226,13 @@ __global__ void k_replay_warp(const gal::state *s, const uint64_t *steps, uint64
 }
 
 // Short lists: one thread per request, warp teams claiming with one atomicAdd
-// per team on their SM's pinned block (gal::malloc).  Compiled for four CTAs of 256 threads per SM (64
-// registers); with the registers it would take (96, two CTAs) 1 Mi mixed requests
-// took 44 us instead of 35.
+// per team on their SM's pinned block (gal::malloc).  Fewer CTAs than SMs, so the
+// kernel may have the registers it takes (96); bounded to 64 its spills cost up
+// to 2 % (malloc and free of 30,000 runs, one slot per SM: 36.1 us, now 35.5;
+// 4,096 of them 25.3, now 24.8; mixed single slices the same at either).
 constexpr int MALLOC_THREADS = 256;
 
-__global__ void __launch_bounds__(MALLOC_THREADS, 4)
+__global__ void __launch_bounds__(MALLOC_THREADS, 2)
     k_malloc_threads(const gal::state *s, const uint64_t *sizes, uint64_t n, void **out) {
   const uint64_t i = (uint64_t)blockIdx.x * MALLOC_THREADS + threadIdx.x;
   if (i < n) out[i] = gal::malloc(s, sizes[i]);
@@ -241,7 +242,10 @@ __global__ void __launch_bounds__(MALLOC_THREADS, 4)
 // (gal_bulk.cuh).  Below BULK_FROM requests the barriers of a chunk cost as much
 // as the claims they save (4,096 mixed: 2 us more than one request per thread;
 // 30,000: 19 against 17 us; 100,003: 25 against 27; 1 Mi x 256 B: 62 against
-// 253; 4 Mi mixed, one slot per SM: 67 against 98).  K is the smallest that fits
+// 253; 4 Mi mixed, one slot per SM: 67 against 98).  Runs of 2-8 slices claim as
+// much as a longer list but change sides no earlier (malloc and free of 4,096,
+// 16,384 and 30,000: 33.9, 70.7, 109 us chunked against 34.7, 71, 111 at the
+// reference's slots, 25.5, 34.6, 38.5 against 25.3, 33.0, 36.1 at one per SM).  K is the smallest that fits
 // the list in one wave of two CTAs per SM: larger chunks claim less often,
 // smaller ones start more SMs (262,144 mixed: 17, 11, 11, 21 us at K = 1, 2, 4, 8).
 // Lists of several waves gain from a third CTA per SM (40 registers; 4 Mi mixed:
