@@ -4,7 +4,7 @@ Jobs arrive as a Poisson process (default mean 2,000 jobs/s, seed 5).  A job is
 either a device vector of uint32 grown by push_back to n elements (n
 log-uniform over 1K-16M, capacity doubling through the allocator) or a queue
 of 32 B nodes with n enqueue/dequeue operations (n log-uniform over 1K-4M);
-each runs as a grid of up to 8 CTAs (gal_job_launch, gal_job_ctas) on a stream
+each runs as one kernel of up to 8,192 threads (gal_job_launch) on a stream
 slot.  The loop keeps every
 slot busy: a job that has arrived is admitted as soon as a slot is free and the
 arena bytes reserved by running jobs plus its own estimated footprint fit in
@@ -33,8 +33,8 @@ SEG = 16 << 20
 
 
 def job_ctas(kind, n):
-    """CTAs of a job (gal_job_ctas): one per 2^20 vector elements or 2^18
-    queue operations, 1 to 8."""
+    """Units of 1,024 threads of a job (gal_job_ctas): one per 2^20 vector elements
+    or 2^18 queue operations, 1 to 8.  A vector's is one CTA, a queue's sixteen."""
     g = n >> 20 if kind == JOB_VECTOR else n >> 18
     return int(min(8, max(1, g)))
 

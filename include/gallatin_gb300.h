@@ -75,7 +75,10 @@ typedef struct gal_config {
                                    frees: lanes that share one atomic come from
                                    aligned groups of this many (1..32, a power
                                    of two; 32 or 0 = the whole warp, as the
-                                   reference's coalesced teams)                  */
+                                   reference's coalesced teams).  It holds for
+                                   the device calls and for malloc lists of less
+                                   than 32 Ki requests; longer ones and every
+                                   list of frees aggregate per CTA               */
   uint32_t arena_kind;          /* GAL_ARENA_*: where the arena lives; metadata
                                    is always device memory                       */
   uint32_t spare_blocks;        /* 1: every pinned slot keeps its next block
@@ -345,12 +348,12 @@ int gal_free_batched_n(gal_handle *h, void *const *ptrs, const unsigned long lon
                        uint64_t max_n, void *stream);
 
 /* ---- served jobs (request loop, gallatin_gb300/serve.py) -------------------
- * One job = a grid of gal_job_ctas(kind, n) CTAs launched on `stream` that
- * allocate through the device allocator: GAL_JOB_VECTOR grows device vectors
- * of uint32 by capacity doubling (the reference's
- * data_structs/single_vector.cuh:86-143 growth), CTA b of G over elements
- * [b n / G, (b + 1) n / G); GAL_JOB_QUEUE runs n enqueue/dequeue operations
- * on queues of 32 B nodes.  result (device u64[3], zeroed by the caller):
+ * One job = a kernel launched on `stream` whose threads allocate through the
+ * device allocator; with G = gal_job_ctas(kind, n): GAL_JOB_VECTOR, G CTAs, grows
+ * device vectors of uint32 by capacity doubling (the reference's
+ * data_structs/single_vector.cuh:86-143 growth), CTA b over elements
+ * [b n / G, (b + 1) n / G); GAL_JOB_QUEUE, 1,024 G threads in CTAs of 64, runs n
+ * enqueue/dequeue operations on a queue of 32 B nodes per thread.  result (device u64[3], zeroed by the caller):
  * checksum, mallocs+frees, failed mallocs.  hist (device
  * u64[2 * GAL_JOB_LAT_BINS] or NULL): the job adds the latency of each of its
  * mallocs (bins 0..GAL_JOB_LAT_BINS-1) and frees (the next GAL_JOB_LAT_BINS),
