@@ -178,7 +178,7 @@ static __device__ void retire_all(const state *s, boot_smem &sm) {
 }
 
 // A fresh segment of class t, its first `taken` blocks given to the slots from
-// `slot` on: what setup_segment and `taken` get_block calls leave, in two steps
+// `slot` on: what setup_begin, setup_open and `taken` get_block calls leave, in two steps
 // with a fence between them (full warp; false: listed free, yet owned).
 static __device__ bool boot_segment(const state *s, uint32_t seg, uint32_t t, uint32_t slot, uint32_t taken) {
   const uint32_t lane = threadIdx.x & 31u;

@@ -992,7 +992,7 @@ GAL_DEVICE_COLD void give_back_reservation(const state *s, uint64_t seg) {
 // raises the new owner's count above its blocks, and one that lands after the
 // segment's last return leaves it unreleased.  Here the count word carries the
 // class: a word of another class or a count already negative is not touched,
-// and the subtraction carries into a new set-up (see setup_segment), so the
+// and the subtraction carries into a new set-up (see setup_open), so the
 // only give-backs left are the rare ones of a race between the load and the
 // subtraction, which give_back_reservation settles.  The new block's malloc
 // word is stored, not yet published: whoever installs the block fences first.
