@@ -127,6 +127,10 @@ __device__ __forceinline__ void flush(unsigned long long *stats, const counters 
   }
 }
 
+// Turns that a lane tries a lock without a pause.  A lock is held for a few turns;
+// one that is held longer waits for a malloc that finds nothing, in an arena that
+// is full, and the limit on the turns is to be a limit of time (some 0.4 s).
+constexpr uint32_t WAITS_BRIEFLY = 64;
 // Bucket lock: bit 0 of the head word.  One try (a round trip whether or not
 // somebody holds it); true: `head` is the list, this thread's until it unlocks.
 __device__ __forceinline__ bool try_lock_bucket(unsigned long long *hp, unsigned long long &head) {
@@ -426,6 +430,8 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
         if (w > gal::cfield(s->spin_limit)) {
           count_global(stats, S_LOCK);
           go = false;
+        } else if (w >= WAITS_BRIEFLY) {
+          gal::backoff(w);
         }
       }
       __syncwarp();
