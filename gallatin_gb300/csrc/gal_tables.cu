@@ -19,7 +19,12 @@
 // form; the CTA keeps a copy of its pinned block, which spares the claim a round
 // trip), or CTA-aggregated (batched form: every thread holds a node ready, and
 // the threads that used theirs ask for the next together through
-// gal::cta_malloc; a node left over at the end is freed).
+// gal::cta_malloc).  The nodes held ready must not be what the arena is short of:
+// a thread takes its own along from one insert phase to the next, and once one
+// lacks a node the others put theirs into a queue for those that lack one, and
+// only a thread whose bucket is full asks.  (Freed, they would leave gaps in
+// blocks that come back only when all of their slices are free.)  What is left
+// is freed with the tables.
 //
 // Bound by latency: an op is a chain of scattered round trips (lock 800 cycles,
 // a node 700-1,000 from L2, more from DRAM, a release 800-1,600).  What kept the
@@ -229,15 +234,68 @@ struct pending {
   volatile uint32_t ready[RING ? 2 * TBT : 1], ready_table[RING ? 2 * TBT : 1];  // the ops that no lane has
   // taken yet, a ring of 64 for each warp: index in the table, table
 };
+// Whether an insert phase is short of nodes: a word for all CTAs, which each looks
+// at once in LOOK_TURNS turns (the look holds the CTA up for a round trip).
+enum : uint32_t { NODES_ENOUGH = 0, NODES_SHORT = 1, NODES_GONE = 2 };
+constexpr uint32_t LOOK_TURNS = 8;
+// Turns in which a lacked node may come from another CTA: that one may be in a
+// request that the allocator is about to refuse, which takes up to 100 ms, so
+// after the first the turns are slow.
+constexpr uint32_t LACK_TURNS = 240, LACK_SLOWLY = 4 * LOOK_TURNS;
+// The nodes that threads held ready: between the insert phases (one place for
+// each thread of a grid), and those for threads that lack one.
+struct node_pool {
+  unsigned long long *kept, *queue;  // [cap] each, 0: none
+  unsigned long long *ends;          // taken, put
+  uint32_t cap;
+};
+__device__ __forceinline__ bool put_node(const node_pool &p, node *n) {
+  const unsigned long long at = atomicAdd(&p.ends[1], 1ull);
+  if (at >= p.cap) return false;
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p.queue + at), "l"(n) : "memory");
+  return true;
+}
+__device__ __noinline__ node *take_node(const gal::state *s, const node_pool &p) {
+  for (int tries = 0; tries < 16; tries++) {
+    const unsigned long long at = gal::ld_rlx(&p.ends[0]);
+    if (at >= min(gal::ld_rlx(&p.ends[1]), (unsigned long long)p.cap)) break;
+    if (atomicCAS(&p.ends[0], at, at + 1) != at) continue;
+    for (uint32_t i = 0; i < gal::cfield(s->spin_limit); i++) {  // its place is taken, it follows at once
+      unsigned long long n;
+      asm volatile("atom.acquire.gpu.global.exch.b64 %0, [%1], 0;" : "=l"(n) : "l"(p.queue + at) : "memory");
+      if (n) return (node *)n;
+      gal::backoff(i);
+    }
+    break;
+  }
+  return nullptr;
+}
+struct node_state {
+  unsigned long long *left;  // the word for all
+  volatile uint32_t seen;    // ... as last seen
+  volatile uint32_t turns;
+  volatile uint8_t lacked[TBT];  // turns that the thread's op has stayed for want of a node
+};
+// A thread found its bucket full and has no node for it: true while its op stays.
+__device__ __forceinline__ bool lacks_node(node_state &nodes, uint32_t me) {
+  const uint32_t turns = nodes.lacked[me];
+  const bool stays = nodes.seen != NODES_GONE && turns < LACK_TURNS;
+  const uint32_t now = stays ? NODES_SHORT : NODES_GONE;
+  atomicMax(nodes.left, (unsigned long long)now);
+  nodes.seen = now;
+  nodes.lacked[me] = turns + 1u;
+  return stays;
+}
 // One turn of an insert, by a whole warp together: true when the op is done.
 // A bucket without room takes `spare`, when there is one (null afterwards);
-// MALLOC: else a node from the allocator under the lock.  The warp meets before
+// MALLOC: else a node from the allocator under the lock.  Without either the op
+// stays for LACK_TURNS more turns, then it fails.  The warp meets before
 // the malloc, whose teams are the lanes that call together: lanes that left the
 // search one by one claimed one by one.  The others have written their pairs by
 // then, and the release at the end finds those writes done.
 template <bool MALLOC, bool RING>
 __device__ __forceinline__ bool insert_turn(const gal::state *s, pending<RING> &op, bool go, node *&spare,
-                                            gal::slot_cache &cache, unsigned long long *stats) {
+                                            gal::slot_cache &cache, unsigned long long *stats, node_state &nodes) {
   const uint32_t me = threadIdx.x;
   bool mine = false, full = false;
   if (go) {
@@ -271,12 +329,19 @@ __device__ __forceinline__ bool insert_turn(const gal::state *s, pending<RING> &
       op.pairs[me] += 1u;
       if (MALLOC) op.nodes[me] += 1u;
     } else {
-      count_global(stats, S_MFAIL);
+      if constexpr (!MALLOC) full = lacks_node(nodes, me);
+      if (MALLOC || !full) count_global(stats, S_MFAIL);
     }
+    if constexpr (!MALLOC) full = full && !n;
   }
   __syncwarp();
   if (mine) unlock_bucket((unsigned long long *)op.hp[me], op.head[me]);
-  return mine;
+  if constexpr (MALLOC) {
+    return mine;
+  } else {
+    if (mine && !full) nodes.lacked[me] = 0;
+    return mine && !full;
+  }
 }
 
 template <bool RING>
@@ -329,7 +394,7 @@ enum : int { PH_INSERT = 0, PH_DELETE = 1, PH_CHECK_DELETED = 2, PH_REINSERT = 3
 template <int PHASE, bool BATCHED>
 __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSERT ? 5 : 6)
     k_tables_phase(const gal::state *s, uint32_t ntab, const uint64_t *offsets, const table_desc *desc, uint64_t seed,
-                   unsigned long long *stats) {
+                   unsigned long long *stats, const __grid_constant__ node_pool pool) {
   constexpr bool INSERTS = PHASE == PH_INSERT || PHASE == PH_REINSERT;
   constexpr bool LOCKS = INSERTS || PHASE == PH_DELETE;
   extern __shared__ uint64_t off[];  // [ntab + 1]
@@ -337,6 +402,15 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
   __shared__ gal::slot_cache cache;
   constexpr bool RING = PHASE == PH_DELETE || PHASE == PH_REINSERT;
   __shared__ pending<RING> op;
+  __shared__ node_state nodes;
+  if constexpr (INSERTS && BATCHED) {
+    nodes.lacked[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+      nodes.left = stats + S_N + 1 + (PHASE == PH_REINSERT);
+      nodes.seen = NODES_ENOUGH;
+      nodes.turns = 0;
+    }
+  }
   for (uint32_t i = threadIdx.x; i <= ntab; i += blockDim.x) off[i] = offsets[i];
   if (INSERTS && BATCHED) gal::cta_claim_init(cm);
   if (INSERTS && !BATCHED) gal::slot_cache_init(cache);
@@ -360,6 +434,7 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
     op.nodes[me] = 0;
     bool go = false;
     node *spare = nullptr;
+    if constexpr (PHASE == PH_REINSERT && BATCHED) spare = (node *)pool.kept[(uint64_t)blockIdx.x * TBT + me];
     for (;;) {
       uint32_t t = 0, index = 0;
       bool mine = false, more = go;  // takes op `index` of table t up; is not through yet
@@ -413,8 +488,23 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
         go = more = true;
       }
       if (INSERTS && BATCHED) {
+        if (me == 0) {
+          const uint32_t turn = nodes.turns + 1u;
+          nodes.turns = turn;
+          if (turn % LOOK_TURNS == 0) nodes.seen = (uint32_t)gal::ld_rlx(nodes.left);
+        }
         if (!__syncthreads_or(more)) break;
-        node *n = (node *)gal::cta_malloc(s, sizeof(node), go && !spare, cm);
+        bool asks = !spare;
+        if (nodes.seen != NODES_ENOUGH && !nodes.lacked[me]) {
+          asks = false;
+          if (spare && put_node(pool, spare)) spare = nullptr;
+        } else if (asks && go && nodes.seen != NODES_ENOUGH) {
+          spare = take_node(s, pool);
+          const uint32_t turn = nodes.lacked[me];
+          asks = !spare && turn == 1;  // (nothing else is freed meanwhile)
+          if (!spare && turn > LACK_SLOWLY) __nanosleep(1000000);
+        }
+        node *n = (node *)gal::cta_malloc(s, sizeof(node), go && asks, cm);
         if (n) {
           spare = n;
           op.nodes[me] += 1u;
@@ -422,7 +512,8 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
       } else if (!__any_sync(0xFFFFFFFFu, more)) {
         break;
       }
-      const bool done = INSERTS ? insert_turn<!BATCHED>(s, op, go, spare, cache, stats) : delete_turn(s, op, go);
+      const bool done = INSERTS ? insert_turn<!BATCHED>(s, op, go, spare, cache, stats, nodes)
+                                : delete_turn(s, op, go);
       if (done) go = false;
       if (go) {
         const uint32_t w = op.waited[me] + 1u;
@@ -436,9 +527,9 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
       }
       __syncwarp();
     }
-    if (spare) {  // held ready to the end
-      gal::free_sized(s, spare, sizeof(node));
-      count(lc, S_SPARE);
+    if constexpr (INSERTS && BATCHED) {  // held ready to the end
+      if (spare && nodes.seen != NODES_ENOUGH && put_node(pool, spare)) spare = nullptr;
+      pool.kept[(uint64_t)blockIdx.x * TBT + me] = (unsigned long long)spare;
     }
     count(lc, INSERTS ? S_INSERTED : S_DELETED, op.pairs[me]);
     count(lc, INSERTS ? S_NODES : S_NODES_FREED, op.nodes[me]);
@@ -564,6 +655,20 @@ __global__ void __launch_bounds__(TBT)
   freed = __reduce_add_sync(0xFFFFFFFFu, freed);
   if ((threadIdx.x & 31) == 0) count_global(stats, S_NODES_FREED, freed);
 }
+// the nodes that were held ready and not needed
+__global__ void __launch_bounds__(TBT) k_tables_spares(const gal::state *s, node_pool pool, unsigned long long *stats) {
+  const uint32_t i = blockIdx.x * TBT + threadIdx.x;
+  uint32_t freed = 0;
+  if (i < 2u * pool.cap) {  // (the queue follows the places)
+    const unsigned long long n = pool.kept[i];
+    if (n) {
+      gal::free_sized(s, (void *)n, sizeof(node));
+      freed = 1;
+    }
+  }
+  freed = __reduce_add_sync(0xFFFFFFFFu, freed);
+  if ((threadIdx.x & 31) == 0) count_global(stats, S_SPARE, freed);
+}
 __global__ void __launch_bounds__(TBT) k_tables_drop(const gal::state *s, uint32_t ntab, const table_desc *desc) {
   const uint32_t t = blockIdx.x * TBT + threadIdx.x;
   if (t < ntab && desc[t].heads) gal::free(s, desc[t].heads);
@@ -592,8 +697,11 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
   // the dumped pairs with their number
   const bool dump = dump_keys && dump_vals && dump_n && dump_table < n_tables && dump_cap;
   // (the pairs on 256-byte boundaries: a copy from an odd word ran at 4 GB/s)
-  const size_t head_words = ((size_t)n_tables * 4 + 1 + S_N + 1 + 31) / 32 * 32;
+  // (after the pairs' number, per insert phase whether it is short of nodes)
+  const size_t head_words = ((size_t)n_tables * 4 + 1 + S_N + 3 + 31) / 32 * 32;
   const size_t pair_words = dump ? ((size_t)dump_cap + 31) / 32 * 32 : 0;
+  size_t pool_words = 0;
+  node_pool pool = {};
   static_assert(sizeof(table_desc) == 16, "two words per table");
   uint64_t *buf = nullptr;
   cudaEvent_t ev[8] = {};  // phase boundaries 0-5, teardown 6-7
@@ -612,14 +720,28 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
       goto done;                     \
     }                                \
   } while (0)
-  TK(cudaMalloc(&buf, (head_words + 2 * pair_words) * sizeof(uint64_t)));
+  if (batched) {
+    int most = 0, per_sm = 0;  // the larger of the two insert grids
+    TK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most, k_tables_phase<PH_INSERT, true>, TBT, smem));
+    TK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_tables_phase<PH_REINSERT, true>, TBT, smem));
+    const uint64_t fit = (uint64_t)sms * std::max(std::max(most, per_sm), 1);
+    pool.cap = (uint32_t)std::min<uint64_t>(need_ctas ? need_ctas : 1, fit) * TBT;
+    pool_words = 2 * (size_t)pool.cap + 2;
+  }
+  TK(cudaMalloc(&buf, (head_words + 2 * pair_words + pool_words) * sizeof(uint64_t)));
   {
   table_desc *d_desc = (table_desc *)buf;
   uint64_t *d_off = buf + 2 * (size_t)n_tables;
   unsigned long long *live = (unsigned long long *)(d_off + n_tables + 1), *stats = live + n_tables;
   unsigned long long *d_n = stats + S_N, *d_keys = (unsigned long long *)buf + head_words, *d_vals = d_keys + pair_words;
   TK(cudaMemcpy(d_off, offsets, (n_tables + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice));
-  TK(cudaMemset(live, 0, (n_tables + S_N + 1) * sizeof(uint64_t)));
+  TK(cudaMemset(live, 0, (n_tables + S_N + 3) * sizeof(uint64_t)));
+  if (batched) {
+    pool.kept = (unsigned long long *)d_vals + pair_words;
+    pool.queue = pool.kept + pool.cap;
+    pool.ends = pool.queue + pool.cap;
+    TK(cudaMemset(pool.kept, 0, pool_words * sizeof(uint64_t)));
+  }
   for (auto &e : ev) TK(cudaEventCreate(&e));
   k_tables_setup<<<n_tables, TBT>>>(d, d_off, d_desc, stats);
   TK(cudaGetLastError());
@@ -630,7 +752,7 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TBT, smem);
       const uint64_t fit = (uint64_t)sms * (per_sm > 0 ? per_sm : 1);
       kern<<<(unsigned)std::min<uint64_t>(need_ctas ? need_ctas : 1, fit), TBT, smem>>>(d, n_tables, d_off, d_desc,
-                                                                                        seed, stats);
+                                                                                        seed, stats, pool);
       return cudaGetLastError();
     };
     TK(batched ? phase(k_tables_phase<PH_INSERT, true>) : phase(k_tables_phase<PH_INSERT, false>));
@@ -661,6 +783,10 @@ int gal_bench_tables(gal_handle *h, uint32_t n_tables, const uint64_t *offsets, 
   TK(cudaGetLastError());
   k_tables_drop<<<(n_tables + TBT - 1) / TBT, TBT>>>(d, n_tables, d_desc);
   TK(cudaGetLastError());
+  if (batched) {
+    k_tables_spares<<<(2 * pool.cap + TBT - 1) / TBT, TBT>>>(d, pool, stats);
+    TK(cudaGetLastError());
+  }
   TK(cudaEventRecord(ev[7]));
   TK(cudaEventSynchronize(ev[7]));
   TK(cudaEventElapsedTime(&res->ms[5], ev[6], ev[7]));

@@ -1,11 +1,28 @@
-"""Hash tables (gallatin_gb300/csrc/gal_tables.cu) in an arena that does not
-hold all of their nodes."""
+"""Hash tables (gallatin_gb300/csrc/gal_tables.cu) in an arena that holds their
+nodes and hardly more: nodes that threads hold ready must not be the ones that
+others lack."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
 SEG = 16 << 20
+
+
+@pytest.mark.parametrize("batched", [False, True])
+@pytest.mark.parametrize("pairs,segments", [(200000, 17), (1000000, 20)])
+def test_tables_that_just_fit(pairs, segments, batched):
+    import gallatin_gb300 as G
+    from gallatin_gb300 import tables as T
+    g = G.Gallatin.generate_on_device(segments * SEG, 42, zero_arena=0)
+    try:
+        for seed in range(4):
+            d = T.run(g, np.full(16, pairs // 16, dtype=np.uint64), seed=seed, batched=batched)
+            assert d["violations"] == 0, d
+            assert d["nodes_allocated"] == d["nodes_freed"] + d["spare_nodes_freed"]
+            g.trim()
+    finally:
+        g.close()
 
 
 @pytest.mark.parametrize("batched", [False, True])
