@@ -485,6 +485,7 @@ __global__ void __launch_bounds__(TBT, PHASE == PH_INSERT || PHASE == PH_REINSER
         op.key[me] = key;
         op.tag[me] = tag;
         op.waited[me] = 0;
+        if constexpr (INSERTS && BATCHED) nodes.lacked[me] = 0;
         go = more = true;
       }
       if (INSERTS && BATCHED) {
