@@ -889,6 +889,7 @@ GAL_DEVICE_COLD int64_t gather_new_segment(const state *s, uint32_t tree, bool t
   if (ok) closed &= setup_open(s, seg, tree, take ? 1u : 0u);
   for (uint64_t b = extra; b; b &= b - 1ull)
     closed &= setup_open(s, base + (uint64_t)__ffsll((long long)b) - 1u, tree, 0);
+  // (the counts are open before the listings below: their atomics have answered)
   if (act_class(closed) != ACT_FREE) set_error(s, GAL_DEV_ERR_SEGMENT_SETUP);
   const veb_ref sub = sub_tree(s, tree);
   if (ok && (!take || blocks_in_segment(s, tree) > 1)) veb_insert(sub, seg);

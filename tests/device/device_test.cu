@@ -169,13 +169,13 @@ __global__ void k_chunk_claim(const gal::state *s, uint32_t tree, uint32_t want,
   if (slots > MOST) return;
   for (uint32_t i = 0; i < slots; i++) {
     if (s->use_spares) gal::refill_spare(s, tree, i, 0);
-    for (uint32_t *at = s->slots + base + i; at; at = at == s->slots + base + i && s->use_spares ? s->spares + base + i : nullptr) {
-      const uint32_t blk = gal::ld_rlx(at);
+    for (uint32_t spare = 0; spare <= (s->use_spares ? 1u : 0u); spare++) {
+      const uint32_t blk = gal::ld_rlx((spare ? s->spares : s->slots) + base + i);
       if (blk == gal::NOBLK) {
         out[3]++;
         continue;
       }
-      used[n] = use_up(s, blk, at == s->slots + base + i ? slot_left : spare_left);
+      used[n] = use_up(s, blk, spare ? spare_left : slot_left);
       blks[n++] = blk;
     }
   }
